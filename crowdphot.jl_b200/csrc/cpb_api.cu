@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <set>
 #include <string>
 #include <vector>
@@ -320,38 +321,58 @@ int cpb_psf_upload(cpb_ctx* ctx, const cpb_psf_desc* d, cpb_psf** out) {
                             (kk / nd.isx) * nd.LPY] = h64[nd.off + si + sk * nd.ny];
                     }
             }
-            check(cudaMalloc(&ps->d_lpp64, sizeof(double) * std::max<size_t>(lpp.size(), 1)), "cudaMalloc");
-            check(cudaMemcpy(ps->d_lpp64, lpp.data(), sizeof(double) * lpp.size(), cudaMemcpyHostToDevice), "h2d");
-            std::vector<float> pp32(pp.size());
+            // row-phase copies (DevNode), each node on a 16-byte boundary
+            std::vector<double> rpp;
+            std::vector<float> rpp32, pp32(pp.size());
+            for (int k = 0; k < nn; ++k) {
+                DevNode& nd = nodes[k];
+                nd.RPX = (nd.nx + 3) | 1;
+                auto fill = [&](auto& v, int c, int gh) {
+                    const int ph = gh * nd.isy;
+                    nd.RPY[c] = (nd.ny + 3 + ph - 1) / ph;
+                    nd.rpoff[c] = (int64_t)v.size();
+                    v.resize(v.size() + ((size_t)ph * nd.RPY[c] * nd.RPX + 3) / 4 * 4);
+                    for (int64_t pi = 0; pi < nd.ny + 3; ++pi)
+                        for (int64_t qi = 0; qi < nd.nx + 3; ++qi) {
+                            const int64_t si = std::min<int64_t>(std::max<int64_t>(pi - 1, 0), nd.ny - 1);
+                            const int64_t sk = std::min<int64_t>(std::max<int64_t>(qi - 1, 0), nd.nx - 1);
+                            v[nd.rpoff[c] + ((pi % ph) * nd.RPY[c] + pi / ph) * nd.RPX + qi] =
+                                (std::decay_t<decltype(v[0])>)h64[nd.off + si + sk * nd.ny];
+                        }
+                };
+                fill(rpp, 0, 2);
+                fill(rpp32, 1, 4);
+            }
             for (size_t q = 0; q < pp.size(); ++q) pp32[q] = (float)pp[q];
-            check(cudaMalloc(&ps->d_pp64, sizeof(double) * std::max<size_t>(pp.size(), 1)), "cudaMalloc");
-            check(cudaMalloc(&ps->d_pp32, sizeof(float) * std::max<size_t>(pp.size(), 1)), "cudaMalloc");
-            check(cudaMemcpy(ps->d_pp64, pp.data(), sizeof(double) * pp.size(), cudaMemcpyHostToDevice), "h2d");
-            check(cudaMemcpy(ps->d_pp32, pp32.data(), sizeof(float) * pp32.size(), cudaMemcpyHostToDevice), "h2d");
-            check(cudaMalloc(&ps->d_data64, sizeof(double) * h64.size()), "cudaMalloc");
-            check(cudaMalloc(&ps->d_data32, sizeof(float) * h32.size()), "cudaMalloc");
-            check(cudaMalloc(&ps->d_nodes, sizeof(DevNode) * nn), "cudaMalloc");
-            check(cudaMalloc(&ps->d_ygrid, sizeof(double) * yg.size()), "cudaMalloc");
-            check(cudaMalloc(&ps->d_xgrid, sizeof(double) * xg.size()), "cudaMalloc");
-            check(cudaMalloc(&ps->d_index_grid, sizeof(int32_t) * ig.size()), "cudaMalloc");
-            check(cudaMemcpy(ps->d_data64, h64.data(), sizeof(double) * h64.size(), cudaMemcpyHostToDevice), "h2d");
-            check(cudaMemcpy(ps->d_data32, h32.data(), sizeof(float) * h32.size(), cudaMemcpyHostToDevice), "h2d");
-            check(cudaMemcpy(ps->d_nodes, nodes.data(), sizeof(DevNode) * nn, cudaMemcpyHostToDevice), "h2d");
-            check(cudaMemcpy(ps->d_ygrid, yg.data(), sizeof(double) * yg.size(), cudaMemcpyHostToDevice), "h2d");
-            check(cudaMemcpy(ps->d_xgrid, xg.data(), sizeof(double) * xg.size(), cudaMemcpyHostToDevice), "h2d");
-            check(cudaMemcpy(ps->d_index_grid, ig.data(), sizeof(int32_t) * ig.size(), cudaMemcpyHostToDevice), "h2d");
+            // one device block and one copy for every table (256-byte aligned pieces)
+            std::vector<char> blob;
+            auto add = [&](const void* src, size_t bytes) {
+                const size_t at = (blob.size() + 255) & ~size_t(255);
+                blob.resize(at + bytes);
+                std::memcpy(blob.data() + at, src, bytes);
+                return at;
+            };
+            auto addv = [&](const auto& v) { return add(v.data(), sizeof(v[0]) * v.size()); };
+            const size_t o_d64 = addv(h64), o_d32 = addv(h32), o_pp64 = addv(pp), o_pp32 = addv(pp32),
+                         o_lpp = addv(lpp), o_r64 = addv(rpp), o_r32 = addv(rpp32), o_nd = addv(nodes),
+                         o_yg = addv(yg), o_xg = addv(xg), o_ig = addv(ig);
+            check(cudaMalloc(&ps->d_blob, blob.size()), "cudaMalloc");
+            check(cudaMemcpy(ps->d_blob, blob.data(), blob.size(), cudaMemcpyHostToDevice), "h2d");
+            const char* base = (const char*)ps->d_blob;
+            dp.data64 = (const double*)(base + o_d64);
+            dp.data32 = (const float*)(base + o_d32);
+            dp.pp64 = (const double*)(base + o_pp64);
+            dp.pp32 = (const float*)(base + o_pp32);
+            dp.lpp64 = (const double*)(base + o_lpp);
+            dp.rpp64 = (const double*)(base + o_r64);
+            dp.rpp32 = (const float*)(base + o_r32);
+            dp.nodes = (const DevNode*)(base + o_nd);
+            dp.ygrid = (const double*)(base + o_yg);
+            dp.xgrid = (const double*)(base + o_xg);
+            dp.index_grid = (const int32_t*)(base + o_ig);
             dp.n_nodes = nn;
             dp.gny = (int32_t)yg.size();
             dp.gnx = (int32_t)xg.size();
-            dp.data64 = ps->d_data64;
-            dp.data32 = ps->d_data32;
-            dp.pp64 = ps->d_pp64;
-            dp.pp32 = ps->d_pp32;
-            dp.lpp64 = ps->d_lpp64;
-            dp.nodes = ps->d_nodes;
-            dp.ygrid = ps->d_ygrid;
-            dp.xgrid = ps->d_xgrid;
-            dp.index_grid = ps->d_index_grid;
             dp.total_elems = (int64_t)h64.size();
             ps->h_nodes = nodes;
             ps->h_data64 = h64;
@@ -361,15 +382,7 @@ int cpb_psf_upload(cpb_ctx* ctx, const cpb_psf_desc* d, cpb_psf** out) {
             ps->smem_bytes64 = (int64_t)h64.size() * 8;
             ps->smem_bytes32 = (int64_t)h64.size() * 4;
         } catch (...) {
-            cudaFree(ps->d_data64);
-            cudaFree(ps->d_data32);
-            cudaFree(ps->d_pp64);
-            cudaFree(ps->d_pp32);
-            cudaFree(ps->d_lpp64);
-            cudaFree(ps->d_nodes);
-            cudaFree(ps->d_ygrid);
-            cudaFree(ps->d_xgrid);
-            cudaFree(ps->d_index_grid);
+            cudaFree(ps->d_blob);
             delete ps;
             throw;
         }
@@ -382,15 +395,7 @@ int cpb_psf_free(cpb_ctx* ctx, cpb_psf* ps) {
     if (!ps) return CPB_OK;
     return guarded(ctx, [&]() -> int {
         cudaStreamSynchronize(ctx->stream);
-        cudaFree(ps->d_data64);
-        cudaFree(ps->d_data32);
-        cudaFree(ps->d_pp64);
-        cudaFree(ps->d_pp32);
-        cudaFree(ps->d_lpp64);
-        cudaFree(ps->d_nodes);
-        cudaFree(ps->d_ygrid);
-        cudaFree(ps->d_xgrid);
-        cudaFree(ps->d_index_grid);
+        cudaFree(ps->d_blob);
         delete ps;
         return CPB_OK;
     });

@@ -44,6 +44,17 @@ struct DevNode {
     //       + (i + 1) / isy + ((k + 1) / isx) * LPY.
     int64_t lpoff;
     int32_t LPY, LPX;   // ceil((ny + 2) / isy), ceil((nx + 2) / isx)
+    // row-phase copies (the stamp kernels that stage the node in shared memory): the
+    // node with one replicated sample before and two after each axis, columns in
+    // order, rows regrouped by their index modulo GH * isy, GH the rows of a stamp
+    // granule (copy 0: FP64, GH = 2; copy 1: FP32, GH = 4); padded sample (p, q)
+    // (0 is the replicate before sample 1) lives at
+    //   rpoff[c] + ((p % (GH isy)) * RPY[c] + p / (GH isy)) * RPX + q.
+    // The four column taps of a stencil row are adjacent, and at the same row of
+    // consecutive granules they are RPX apart: RPX is odd, so the lanes of a warp
+    // meet no shared-memory bank twice.
+    int64_t rpoff[2];
+    int32_t RPY[2], RPX;   // ceil((ny + 3) / (GH isy)), the odd number >= nx + 3
 };
 
 constexpr int kMaxNodes = 64;
@@ -58,6 +69,8 @@ struct DevPsf {
     const double* pp64;       // polyphase copies of the node data (see DevNode)
     const float* pp32;
     const double* lpp64;      // edge-padded polyphase copies (see DevNode)
+    const double* rpp64;      // row-phase copies (see DevNode)
+    const float* rpp32;
     const DevNode* nodes;     // n_nodes
     const double* ygrid;      // gny
     const double* xgrid;      // gnx
@@ -174,6 +187,36 @@ __device__ __forceinline__ void corner_eval(const D* __restrict__ data, const De
         pdv = inb ? dpdv : (M)0;
         pdu = inb ? dpdu : (M)0;
     }
+}
+
+// One axis of a star's box over a node: the pixels first + i, i in [0, n), whose
+// grid coordinate s (first + i - centre) + origin lies in [1, samples] are i in
+// [lo, hi] (hi < lo: none).  The oversampling s is an integer, so every pixel has
+// the fraction f of pixel lo and pixel i starts its stencil at sample
+// l0 + s (i - lo); l0 = samples happens only with f = 0, where the two replicates
+// after the last sample (row-phase copies) stand in for the clamped stencil.
+// Called by a whole warp; every lane gets the result.
+struct AxisSpan {
+    int lo, hi, l0;
+    double f;
+};
+__device__ __forceinline__ AxisSpan axis_span(double s, double centre, double origin, int samples, int first, int n) {
+    const int lane = threadIdx.x & 31;
+    AxisSpan a;
+    a.lo = 0;
+    a.hi = -1;
+    for (int i0 = 0; i0 < n; i0 += 32) {
+        const double u = s * ((double)(first + i0 + lane) - centre) + origin;
+        const unsigned m = __ballot_sync(0xffffffffu, i0 + lane < n && u >= 1.0 && u <= (double)samples);
+        if (m) {
+            if (a.hi < 0) a.lo = i0 + __ffs(m) - 1;
+            a.hi = i0 + 31 - __clz(m);
+        }
+    }
+    const double u = a.hi < 0 ? 1.0 : s * ((double)(first + a.lo) - centre) + origin;
+    a.l0 = (int)floor(u);
+    a.f = u - (double)a.l0;
+    return a;
 }
 
 template <typename D>
@@ -631,15 +674,7 @@ __device__ inline void spread_disk_block(const DevPsf& P, double param, int kh, 
 // ---------------------------------------------------------------------------
 struct cpb_psf {
     cpb::DevPsf dev;
-    double* d_data64 = nullptr;
-    float* d_data32 = nullptr;
-    double* d_pp64 = nullptr;
-    float* d_pp32 = nullptr;
-    double* d_lpp64 = nullptr;
-    cpb::DevNode* d_nodes = nullptr;
-    double* d_ygrid = nullptr;
-    double* d_xgrid = nullptr;
-    int32_t* d_index_grid = nullptr;
+    void* d_blob = nullptr;  // every device table of the PSF (dev points into it)
     std::vector<cpb::DevNode> h_nodes;
     int64_t smem_bytes64 = 0;  // padded bytes of all nodes in FP64
     int64_t smem_bytes32 = 0;

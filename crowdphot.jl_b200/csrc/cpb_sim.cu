@@ -1086,6 +1086,241 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 3) k_eval_warp(const
     }
 }
 
+// Stamp evaluation of single-node ePSFs whose row-phase copy fits shared memory,
+// for boxes within 2 x 2 regions (k_eval_warp otherwise): one persistent block an
+// SM stages the node once; one warp a star, a lane one granule row (GH image rows)
+// of every column it takes, so its row constants are set once a star, the addresses
+// of a column advance by additions and every store is 16 bytes a lane, consecutive
+// down the column.  The oversampling is an integer, so all
+// pixels of a star share one fraction and one set of cubic weights an axis
+// (axis_span), which live in registers; a pixel costs its 16 sample loads
+// (immediate offsets from four row addresses) and about 60 FP64 operations.
+// Bound: shared-memory bandwidth (128 B of FP64 samples a pixel, none shared at
+// 4x oversampling; 76 % of it reached by the value-only form) and the FP64 pipe.
+// Measured against k_eval_warp, which reads two 88-byte axis tables a pixel from
+// shared memory and its samples through L1 (2048^2 field, 50,000 stars, 25 x 25
+// boxes, FP64, mean of a fit's launches): stamps 428 -> 202 us, model values 178 ->
+// 86 us, Gram blocks 566 -> 279 us; on the 613 x 421 field of 1,400 stars 27 -> 17,
+// 23 -> 13 and 27 -> 17 us, so every list size takes it.  512 threads (128
+// registers) for the derivative forms: 640 threads spilled (stamps 277 us).
+template <typename T, bool GRAD>
+struct NodeThreads {
+    static constexpr int N = GRAD ? 512 : (sizeof(T) == 4 ? 768 : 640);  // one block an SM
+};
+
+// one 16-byte granule store
+__device__ __forceinline__ void st_gran(float* p, const float (&v)[4]) {
+    *(float4*)p = make_float4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ void st_gran(double* p, const double (&v)[2]) { *(double2*)p = make_double2(v[0], v[1]); }
+
+// P3: y, x and flux are all free (p == 3, gradient columns in order).
+template <bool GRAD, typename T, bool GRAM, bool P3>
+__global__ void __launch_bounds__(NodeThreads<T, GRAD>::N, 1)
+    k_eval_node(const int32_t* __restrict__ list, int64_t nlist, FitConst fc, DevNode nd, const T* __restrict__ samples,
+                const StarCoef* __restrict__ coef, const int32_t* __restrict__ ay, const int32_t* __restrict__ ax,
+                const double* __restrict__ sw, T* __restrict__ V, RectMap vmap, double* __restrict__ colnorm,
+                double* __restrict__ gram, T* __restrict__ M, RectMap mmap, int Rmax,
+                const int32_t* __restrict__ Rs) {
+    constexpr int NTH = NodeThreads<T, GRAD>::N, NWP = NTH / 32;
+    constexpr int GH = Gran<T>::H, CP = GH == 2 ? 0 : 1;
+    constexpr bool wantV = GRAD && !GRAM;
+    const bool wantM = !GRAM && M != nullptr;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ StorePlan plans[NWP];
+    T* node = (T*)smem_raw;
+    const int RPY = nd.RPY[CP], RPX = nd.RPX, NPH = GH * nd.isy;
+    {
+        const int n16 = (NPH * RPY * RPX + GH - 1) / GH;  // the copy is padded to a multiple of four
+#pragma unroll 4
+        for (int k = threadIdx.x; k < n16; k += NTH) ((int4*)node)[k] = __ldg((const int4*)samples + k);
+        __syncthreads();
+    }
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    StorePlan& plan = plans[wid];
+    const T nfill = (T)nd.fill, nsy = (T)nd.sy, nsx = (T)nd.sx;
+    const int p = P3 ? 3 : fc.p;
+    const int g0 = fc.gc[0] - 1, g1 = fc.gc[1] - 1, g2 = fc.gc[2] - 1;
+    // consecutive stars go to different SMs first, so that a short list uses them all
+    for (int64_t li = blockIdx.x + (int64_t)wid * gridDim.x; li < nlist; li += (int64_t)NWP * gridDim.x) {
+        const int j = list ? list[li] : (int)li;
+        const StarCoef& cg = coef[j];
+        const double cy = cg.y, cx = cg.x;
+        const T flux = (T)cg.flux, bkg = (T)cg.bkg;
+        const T w0 = (T)cg.w[0], dwy = (T)cg.dwdy[0], dwx = (T)cg.dwdx[0];
+        const int Rb = Rs ? Rs[j] : Rmax;
+        const int Sb = 2 * Rb + 1;
+        const int a_y = ay[j], a_x = ax[j];
+        const int oy = a_y - Rb, ox = a_x - Rb;
+        int ty0 = 0, ty1 = -1, tx0 = 0, tx1 = -1;
+        star_tiles(a_y, a_x, Rb, fc.ny, fc.nx, ty0, ty1, tx0, tx1);
+        const int nrect = (ty1 - ty0 + 1) * (tx1 - tx0 + 1);
+        store_plan(plan, lane, nrect, j, a_y, a_x, Rb, ty0, ty1, tx0, GH, wantV ? &vmap : nullptr,
+                   wantM ? &mmap : nullptr);
+        __syncwarp();
+        const int top0 = oy - 1, so = top0 - gran_base(top0, GH);
+        const AxisSpan sy = axis_span(nd.sy, cy, nd.oy, nd.ny, oy, Sb);
+        const AxisSpan sx = axis_span(nd.sx, cx, nd.ox, nd.nx, ox, Sb);
+        T wx[4], dx[4], wy[4], dy[4];
+        {
+            double w[4], d[4];
+            keys_weights(sx.f, w, d);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                wx[k] = (T)w[k];
+                dx[k] = (T)d[k];
+            }
+            keys_weights(sy.f, w, d);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                wy[k] = (T)w[k];
+                dy[k] = (T)d[k];
+            }
+        }
+        // the lane's granule: storage rows GH k .. GH k + GH - 1 of every column it takes
+        // (KW lanes a column, so that a half warp's sample loads stay in one column)
+        const int NK = gran_rows(Sb, GH) / GH;
+        const int KW = NK <= 8 ? 8 : (NK <= 16 ? 16 : 32), CW = 32 / KW;
+        const int k = lane & (KW - 1), cg0 = lane / KW;
+        const int row0 = GH * k - so, y0 = top0 + row0;  // first box row and 0-based image row
+        // sample (row tap r, first column tap) of granule row h, box column col: rb[h][r] + col * isx
+        int rb[GH][4];
+        bool rin[GH], yin[GH], wrow[GH];
+        {
+            const int x0 = sx.l0 - 1 - nd.isx * sx.lo;
+            const int q0 = sy.l0 - 1 + nd.isy * (row0 - sy.lo);
+#pragma unroll
+            for (int h = 0; h < GH; ++h) {
+                const int row = row0 + h;
+                rin[h] = row >= 0 && row < Sb;
+                yin[h] = row >= sy.lo && row <= sy.hi;
+                wrow[h] = rin[h] && y0 + h >= 0 && y0 + h < fc.ny;
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const int q = max(q0 + h * nd.isy + r, 0), e = q / NPH;  // q >= 0 wherever yin
+                    rb[h][r] = ((q - e * NPH) * RPY + e) * RPX + x0;
+                }
+            }
+        }
+        const int nty_j = ty1 - ty0 + 1;
+        const int vr = y0 / TY - ty0;  // the lane's vertical region of the star's (y0 < 0: none)
+        const bool live = k < NK && y0 >= 0 && vr < nty_j;
+        double acc[GRAM ? 6 : 3] = {};
+        for (int hr = 0; hr <= tx1 - tx0; ++hr) {
+            const int l = hr * nty_j + (live ? vr : 0);
+            const int nrows = plan.nrows[l], ps = plan.ps[l];
+            int col = plan.c_lo[l] + cg0;
+            const int cend = plan.c_lo[l] + (nrows > 0 ? ps / nrows : 0);
+            int64_t at = (int64_t)cg0 * nrows + (GH * k - plan.s_lo[l]);  // within the rectangle's plane
+            T* vp = wantV ? V + plan.offV[l] : nullptr;
+            T* mp = wantM ? M + plan.offM[l] : nullptr;
+            const double* swc = sw + ((int64_t)(ox + col - 1) * fc.ny + y0);
+            const T* xp = node + col * nd.isx;
+            double swn[GH];
+            // sw = sqrt(w): positive exactly where the weight is; the rectangles of the last
+            // regions reach past the image's last column and row, where there is none
+            const int cimg = min(cend, fc.nx + 1 - ox);
+            auto load_sw = [&](bool ok) {
+#pragma unroll
+                for (int h = 0; h < GH; ++h)
+                    swn[h] = ok && wrow[h] && CPB_CHECK(swc + h - sw < (int64_t)fc.ny * fc.nx, 0x53) ? __ldg(swc + h)
+                                                                                                     : 0.0;
+            };
+            if (GRAD) load_sw(live && col < cimg);
+            for (; live && col < cend; col += CW, xp += CW * nd.isx, at += CW * nrows) {
+                double swq[GH];
+                if (GRAD) {  // the next column's weights load behind this column's arithmetic
+#pragma unroll
+                    for (int h = 0; h < GH; ++h) swq[h] = swn[h];
+                    swc += (int64_t)CW * fc.ny;
+                    load_sw(col + CW < cimg);
+                }
+                const bool cin = col >= sx.lo && col <= sx.hi;
+                T vm[GH], v0[GH], v1[GH], v2[GH];
+#pragma unroll
+                for (int h = 0; h < GH; ++h) {
+                    T pv = nfill, pdv = 0, pdu = 0;
+                    if (cin && yin[h]) {
+                        T rv[4], rd[4];
+#pragma unroll
+                        for (int r = 0; r < 4; ++r) {
+                            const T* q = xp + rb[h][r];
+                            const T a = q[0], b = q[1], c = q[2], e = q[3];
+                            rv[r] = wx[0] * a + wx[1] * b + wx[2] * c + wx[3] * e;
+                            if (GRAD) rd[r] = dx[0] * a + dx[1] * b + dx[2] * c + dx[3] * e;
+                        }
+                        pv = wy[0] * rv[0] + wy[1] * rv[1] + wy[2] * rv[2] + wy[3] * rv[3];
+                        if (GRAD) {
+                            pdv = dy[0] * rv[0] + dy[1] * rv[1] + dy[2] * rv[2] + dy[3] * rv[3];
+                            pdu = wy[0] * rd[0] + wy[1] * rd[1] + wy[2] * rd[2] + wy[3] * rd[3];
+                        }
+                    }
+                    const T s = w0 * pv;
+                    vm[h] = rin[h] ? flux * s + bkg : (T)0;
+                    if (GRAD) {
+                        // zero where the pixel is off the box, off the image or unweighted
+                        const T sq = (T)swq[h];
+                        const bool use = swq[h] > 0;
+                        T g[3];
+                        g[0] = flux * (dwy * pv - w0 * nsy * pdv);
+                        g[1] = flux * (dwx * pv - w0 * nsx * pdu);
+                        g[2] = s;
+                        const T ga = P3 ? g[0] : (g0 == 0 ? g[0] : (g0 == 1 ? g[1] : g[2]));
+                        const T gb = P3 ? g[1] : (g1 == 0 ? g[0] : (g1 == 1 ? g[1] : g[2]));
+                        const T gc = P3 ? g[2] : (g2 == 0 ? g[0] : (g2 == 1 ? g[1] : g[2]));
+                        v0[h] = use ? sq * ga : (T)0;
+                        v1[h] = use ? sq * gb : (T)0;
+                        v2[h] = use ? sq * gc : (T)0;
+                        const double d0 = v0[h], d1 = p > 1 ? (double)v1[h] : 0.0, d2 = p > 2 ? (double)v2[h] : 0.0;
+                        if constexpr (GRAM) {
+                            acc[0] += d0 * d0;
+                            acc[1] += d0 * d1;
+                            acc[2] += d0 * d2;
+                            acc[3] += d1 * d1;
+                            acc[4] += d1 * d2;
+                            acc[5] += d2 * d2;
+                        } else {
+                            acc[0] += d0 * d0;
+                            acc[1] += d1 * d1;
+                            acc[2] += d2 * d2;
+                        }
+                    }
+                }
+                if (wantM && CPB_CHECK(plan.offM[l] + at + GH <= mmap.len, 0x51)) st_gran(mp + at, vm);
+                if (wantV && CPB_CHECK(plan.offV[l] + at + (int64_t)(p - 1) * ps + GH <= vmap.len, 0x52)) {
+                    st_gran(vp + at, v0);
+                    if (p > 1) st_gran(vp + at + ps, v1);
+                    if (p > 2) st_gran(vp + at + 2 * ps, v2);
+                }
+            }
+        }
+        if constexpr (GRAM) {
+#pragma unroll
+            for (int k = 0; k < 6; ++k) acc[k] = warp_sum(acc[k]);
+            if (lane == 0) {
+                double* gj = gram + (int64_t)j * 6;
+                if (p == 1) gj[0] = acc[0];
+                else if (p == 2) {
+                    gj[0] = acc[0];
+                    gj[1] = acc[1];
+                    gj[2] = acc[3];
+                } else {
+                    for (int k = 0; k < 6; ++k) gj[k] = acc[k];
+                }
+            }
+        } else if constexpr (GRAD) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                acc[k] = warp_sum(acc[k]);
+                double cn = sqrt(k < p ? acc[k] : 1.0);
+                cn = cn < kEps64 ? kEps64 : cn;
+                if (lane == 0 && k < p) colnorm[(int64_t)j * p + k] = cn;
+            }
+        }
+        __syncwarp();
+    }
+}
+
 // Per-region pixel gather over the region's star list (stars in Morton
 // order), the deterministic replacement of the reference's scatter-adds.
 // A block owns a TY x TX pixel region; warp w takes the region's stars
@@ -2020,6 +2255,28 @@ void launch_eval_warp(bool plan, unsigned grid, unsigned thr, size_t smem, cudaS
     else go(k_eval_warp<GRAD, TS, false, GRAM>);
 }
 
+template <typename T>
+const T* rpp_host(const DevPsf& P);
+template <>
+const double* rpp_host<double>(const DevPsf& P) { return P.rpp64; }
+template <>
+const float* rpp_host<float>(const DevPsf& P) { return P.rpp32; }
+
+// k_eval_node over the node of a single-node ePSF.
+template <bool GRAD, typename T, bool GRAM, typename... A>
+void launch_eval_node(const DevPsf& dp, const DevNode& nd, int n_sm, cudaStream_t st, const int32_t* list, int64_t nlist,
+                      const FitConst& fc, A... args) {
+    constexpr int GH = Gran<T>::H, CP = GH == 2 ? 0 : 1;
+    const size_t smem = sizeof(T) * (size_t)((GH * nd.isy * nd.RPY[CP] * nd.RPX + 3) / 4 * 4);
+    auto go = [&](auto kern) {
+        check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attr");
+        const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(nlist, n_sm));
+        kern<<<grid, NodeThreads<T, GRAD>::N, smem, st>>>(list, nlist, fc, nd, rpp_host<T>(dp) + nd.rpoff[CP], args...);
+    };
+    if (!GRAD || fc.p == 3) go(k_eval_node<GRAD, T, GRAM, true>);
+    else go(k_eval_node<GRAD, T, GRAM, false>);
+}
+
 template <bool GRAD, typename T, typename... A>
 void launch_k_eval(int64_t S2, unsigned grid, size_t smem, cudaStream_t st, A... args) {
     auto go = [&](auto kern, int threads) {
@@ -2311,6 +2568,13 @@ class SimFit {
     template <typename TS, typename TU>
     void outer_loop(Form<TS, TU>& F, int it_first, int it_last, bool initial);
     void finish();
+    // whether k_eval_node takes this PSF: one node whose row-phase copy (elements of
+    // `item` bytes) fits the block's shared memory beside its static tables
+    bool node_eval(size_t item) const {
+        return dp.kind != CPB_PSF_CIRCULAR_GAUSSIAN && dp.n_nodes == 1 &&
+               (int64_t)item * (item == 8 ? 2 : 4) * node0.isy * node0.RPY[item == 8 ? 0 : 1] * node0.RPX + 8192 <=
+                   smem_optin;
+    }
     void warp_shape(int Sx, size_t tab_size, unsigned& threads, size_t& smem) const;
     void arena_precheck();
     void launch_coef(const double* delta, StarCoef* dst);
@@ -2362,6 +2626,7 @@ class SimFit {
     size_t live_tmp_bytes = 0;
     int64_t n_live = 0;
     bool warp_eval = false;
+    DevNode node0{};  // the node of a single-node ePSF
     int smem_optin = 0;
     int Sm = 0;
     unsigned jt_blocks = 1;
@@ -2465,7 +2730,11 @@ void SimFit::launch_fill(Form<TS, TU>& F, const int32_t* list, int64_t nlist) {
                                      std::min<double>((double)fc.S2, (double)h_ucnt / std::max<int64_t>(n_act, 1)) * 16 +
                                      sizeof(StarCoef)));
     TS* Mo = writeM ? F.M : nullptr;
-    if (warp_eval) {
+    if (node_eval(sizeof(TS)) && F.vmap.srect && (!Mo || F.mmap.srect)) {
+        launch_eval_node<true, TS, false>(dp, node0, ctx->n_sm, st, list, nlist, F.fc, (const StarCoef*)coef, ay, ax, sw,
+                                          F.V, F.vmap, cn, (double*)nullptr, Mo, F.mmap, fc.R,
+                                          (const int32_t*)nullptr);
+    } else if (warp_eval) {
         unsigned thr;
         size_t sm_bytes;
         warp_shape(fc.S, sizeof(AxisTab<TS>), thr, sm_bytes);
@@ -2491,7 +2760,11 @@ void SimFit::launch_eval_model(const FitConst& f, TS* M, const RectMap& mmap, co
                                const StarCoef* cf) {
     if (nlist <= 0) return;
     KernelScope ks_(ctx, "k_eval_model", (double)nlist * ((double)Sm * Sm * sizeof(TS) + sizeof(StarCoef)));
-    if (warp_eval) {
+    if (node_eval(sizeof(TS)) && mmap.srect) {
+        launch_eval_node<false, TS, false>(dp, node0, ctx->n_sm, st, list, nlist, f, cf, ay, ax, sw, (TS*)nullptr,
+                                           RectMap{}, cn, (double*)nullptr, M, mmap, model_R,
+                                           (const int32_t*)d_modelR);
+    } else if (warp_eval) {
         unsigned thr;
         size_t sm_bytes;
         warp_shape(Sm, sizeof(AxisTab<TS>), thr, sm_bytes);
@@ -2825,6 +3098,7 @@ bool SimFit::setup() {
     live_tmp = scratch(ctx, "live_tmp", live_tmp_bytes);
 
     warp_eval = dp.kind == CPB_PSF_CIRCULAR_GAUSSIAN || dp.n_nodes == 1;
+    if (dp.kind != CPB_PSF_CIRCULAR_GAUSSIAN) node0 = psf->h_nodes[0];
     check(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device), "attr");
     jt_blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>((n_act + 7) / 8, (int64_t)ctx->n_sm * 8));
     lam = P->lambda_init;
@@ -3088,7 +3362,11 @@ void SimFit::finish() {
     const FitConst& f64 = fc;
     {
         KernelScope ks_(ctx, "k_eval_gram", (double)n_act * (48.0 + sizeof(StarCoef)));
-        if (warp_eval) {
+        if (node_eval(sizeof(double)) && 2 * fc.R + 1 <= TX + 1 && 2 * fc.R + 1 <= TY + 1) {
+            launch_eval_node<true, double, true>(dp, node0, ctx->n_sm, st, (const int32_t*)nullptr, n_act, f64,
+                                                 (const StarCoef*)coef, ay, ax, sw, (double*)nullptr, RectMap{}, cn,
+                                                 gram, (double*)nullptr, RectMap{}, fc.R, (const int32_t*)nullptr);
+        } else if (warp_eval) {
             unsigned thr;
             size_t sm_bytes;
             warp_shape(fc.S, sizeof(AxisTab<double>), thr, sm_bytes);

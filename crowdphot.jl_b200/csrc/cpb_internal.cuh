@@ -826,11 +826,13 @@ int fit_simultaneous_dev(cpb_ctx* ctx, const cpb_psf* psf, const cpb_sim_params*
 // again inside the fit once the radii are known.
 size_t sim_scratch_bound(const cpb_sim_params* P, int64_t ny, int64_t nx, int64_t n, bool dbg_pixels);
 
-// model_rad = :auto (psf_photometry_simultaneous.jl:192-243), host side
-// (cpb_radii.cu): per-star model radii from the unit PSF's curve of growth and
-// the background noise of the weight sample.
-void model_radii_auto(const cpb_psf* psf, double fwhm, double nsigma, int R_fit, int R_cap,
-                      std::vector<double>& w_sample, const std::vector<double>& flux, std::vector<int32_t>& out);
+// model_rad = :auto (psf_photometry_simultaneous.jl:192-243, cpb_radii.cu):
+// per-star model radii from the unit PSF's curve of growth and the background
+// noise of the weight sample w[1 : max(1, npix / 65536) : end].  d_buf: npix,
+// d_sb: R_cap + 2 doubles of scratch; the radii go to d_R and, after a synchronisation, to out.
+void model_radii_auto(cpb_ctx* ctx, const cpb_psf* psf, double fwhm, double nsigma, int R_fit, int R_cap,
+                      const double* d_w, int64_t npix, double* d_buf, double* d_sb, const int32_t* d_act,
+                      int64_t n_act, const double* d_f0, int32_t* d_R, std::vector<int32_t>& out);
 
 // spread_model reference disk (cpb_spread.cu): the separable components of
 // the band-limited exponential disk with support half = ceil(fit_rad); false

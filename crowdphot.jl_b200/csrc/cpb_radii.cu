@@ -1,4 +1,5 @@
-// cpb_radii.cu -- model_rad = :auto: per-star model-render radii (host side).
+// cpb_radii.cu -- model_rad = :auto: per-star model-render radii (the PSF's curve of
+// growth on the host, the noise quantile and the radii on the device).
 //
 // Restates, for the library's device path,
 //   _model_radii (:auto branch)       src/photometry/psf_photometry_simultaneous.jl:209-243
@@ -241,20 +242,138 @@ std::vector<double> unit_sb(const cpb_psf* ps, double fwhm, int R_cap) {
 
 }  // namespace
 
-void model_radii_auto(const cpb_psf* psf, double fwhm, double nsigma, int R_fit, int R_cap,
-                      std::vector<double>& w_sample, const std::vector<double>& flux, std::vector<int32_t>& out) {
-    // sigma_bg from the 0.84 quantile (type 7) of the positive finite weights
-    std::vector<double> ws;
-    ws.reserve(w_sample.size());
-    for (double v : w_sample)
-        if (v > 0 && std::isfinite(v)) ws.push_back(v);
-    if (ws.empty()) throw ArgError{"model_rad=:auto found no positive finite weights to estimate the noise"};
-    std::sort(ws.begin(), ws.end());
-    const double h = (double)(ws.size() - 1) * 0.84;
-    const size_t lo = (size_t)std::floor(h);
-    const size_t hi = std::min(lo + 1, ws.size() - 1);
-    const double wval = ws[lo] + (h - (double)lo) * (ws[hi] - ws[lo]);
-    const double sigma_bg = wval > 0 ? std::sqrt(1.0 / wval) : 1.0;
+namespace {
+
+constexpr int kQuantThreads = 1024, kDigit = 11, kBins = 1 << kDigit;
+
+// sigma_bg of _model_radii (:192-225): the 0.84 quantile (type 7) of the positive
+// finite weights of the sample w[0], w[step], ... (nsamp of them), then
+// sqrt(1 / quantile).  One block: the sample is copied to `buf` once and the two
+// order statistics found by a radix select, 11 bits a pass (positive doubles order
+// as their bit patterns), counting in shared memory with one atomic per distinct
+// digit of a warp.  res[0] = sigma_bg, res[1] = the number of positive weights.
+// Rounding steps are those of the host arithmetic (no contraction).
+// Bound by the latency of one block's passes over at most 131,071 samples; a strided
+// read-back and a host sort of them took half of a 613 x 421 field's call (whole call
+// 9.9 -> 5.1 ms).
+__global__ void __launch_bounds__(kQuantThreads) k_noise_quantile(const double* __restrict__ w, int64_t step,
+                                                                  int64_t nsamp, double* buf, double* res) {
+    __shared__ unsigned hist[kBins];
+    __shared__ unsigned wsum[kQuantThreads / 32];
+    __shared__ unsigned long long s_prefix;
+    __shared__ unsigned s_rank, s_cnt;
+    __shared__ unsigned long long s_next;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    if (tid == 0) s_cnt = 0;
+    __syncthreads();
+    unsigned good = 0;
+    for (int64_t i = tid; i < nsamp; i += kQuantThreads) {
+        double v = w[i * step];
+        const bool ok = v > 0 && isfinite(v);
+        good += ok;
+        buf[i] = ok ? v : 0.0;  // 0: not in the sample
+    }
+    good = __reduce_add_sync(0xffffffffu, good);
+    if (lane == 0 && good) atomicAdd(&s_cnt, good);
+    __syncthreads();
+    const unsigned n = s_cnt;
+    if (tid == 0) res[1] = (double)n;
+    if (n == 0) {
+        if (tid == 0) res[0] = 1.0;
+        return;
+    }
+    const double h = __dmul_rn((double)(n - 1), 0.84);
+    const unsigned lo = (unsigned)floor(h);
+    if (tid == 0) {
+        s_prefix = 0;
+        s_rank = lo;
+    }
+    unsigned long long mask = 0;
+    for (int shift = 64 - kDigit; ; shift = shift > kDigit ? shift - kDigit : 0) {
+        for (int b = tid; b < kBins; b += kQuantThreads) hist[b] = 0;
+        __syncthreads();
+        const unsigned long long prefix = s_prefix;
+        for (int64_t i0 = 0; i0 < nsamp; i0 += kQuantThreads) {
+            const int64_t i = i0 + tid;
+            const unsigned long long key = i < nsamp ? (unsigned long long)__double_as_longlong(buf[i]) : 0ull;
+            const bool in = key != 0 && (key & mask) == prefix;
+            const unsigned d = in ? (unsigned)(key >> shift) & (kBins - 1) : kBins;
+            const unsigned same = __match_any_sync(0xffffffffu, d);
+            if (in && lane == __ffs(same) - 1) atomicAdd(&hist[d], __popc(same));
+        }
+        __syncthreads();
+        // the bin holding rank s_rank: two bins a thread, block prefix sums
+        const unsigned c0 = hist[2 * tid], c1 = hist[2 * tid + 1];
+        unsigned incl = c0 + c1;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+        }
+        if (lane == 31) wsum[wid] = incl;
+        __syncthreads();
+        unsigned before = 0;
+        for (int q = 0; q < wid; ++q) before += wsum[q];
+        const unsigned excl = before + incl - (c0 + c1), rank = s_rank;
+        __syncthreads();  // every thread has read s_rank
+        if (rank >= excl && rank < excl + c0 + c1) {
+            const bool second = rank >= excl + c0;
+            s_prefix = prefix | (unsigned long long)(2 * tid + (second ? 1 : 0)) << shift;
+            s_rank = rank - excl - (second ? c0 : 0);
+        }
+        mask |= (unsigned long long)(kBins - 1) << shift;
+        __syncthreads();
+        if (shift == 0) break;
+    }
+    // ws[lo] = the selected value; ws[lo + 1]: the same value when more than one
+    // sample past rank lo has it, else the smallest larger one
+    const unsigned long long key_lo = s_prefix;
+    if (tid == 0) {
+        s_next = ~0ull;
+        s_cnt = 0;
+    }
+    __syncthreads();
+    unsigned long long nxt = ~0ull;
+    unsigned le = 0;
+    for (int64_t i = tid; i < nsamp; i += kQuantThreads) {
+        const unsigned long long key = (unsigned long long)__double_as_longlong(buf[i]);
+        if (key == 0) continue;
+        if (key <= key_lo) ++le;
+        else nxt = key < nxt ? key : nxt;
+    }
+    le = __reduce_add_sync(0xffffffffu, le);
+    if (lane == 0) atomicAdd(&s_cnt, le);
+    atomicMin(&s_next, nxt);
+    __syncthreads();
+    if (tid == 0) {
+        const double a = __longlong_as_double((long long)key_lo);
+        const double b = lo + 1 >= n || s_cnt > lo + 1 ? a : __longlong_as_double((long long)s_next);
+        const double wval = __dadd_rn(a, __dmul_rn(h - (double)lo, b - a));
+        res[0] = wval > 0 ? sqrt(1.0 / wval) : 1.0;
+    }
+}
+
+// Per active star: the radius where its flux times the unit annular surface
+// brightness falls below nsigma * sigma_bg (:237-243).
+__global__ void k_model_radii(int64_t n_act, const int32_t* __restrict__ act, const double* __restrict__ f0,
+                              const double* __restrict__ sb, const double* __restrict__ res, double nsigma, int R_fit,
+                              int R_cap, int32_t* out) {
+    const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (j >= n_act) return;
+    const double thr = __dmul_rn(nsigma, res[0]);
+    const double F = fmax(f0[act[j]], 0.0);
+    int r = R_fit;
+    while (r < R_cap && __dmul_rn(F, sb[r - 1]) > thr) ++r;
+    out[j] = r;
+}
+
+}  // namespace
+
+void model_radii_auto(cpb_ctx* ctx, const cpb_psf* psf, double fwhm, double nsigma, int R_fit, int R_cap,
+                      const double* d_w, int64_t npix, double* d_buf, double* d_sb, const int32_t* d_act,
+                      int64_t n_act, const double* d_f0, int32_t* d_R, std::vector<int32_t>& out) {
+    cudaStream_t st = ctx->stream;
+    const int64_t step = std::max<int64_t>(1, npix / 65536), nsamp = (npix + step - 1) / step;
     cpb_psf* ps = const_cast<cpb_psf*>(psf);
     std::vector<double> sb;
     {
@@ -264,14 +383,19 @@ void model_radii_auto(const cpb_psf* psf, double fwhm, double nsigma, int R_fit,
         if (it == ps->cog_sb.end()) it = ps->cog_sb.emplace(key, unit_sb(psf, fwhm, R_cap)).first;
         sb = it->second;
     }
-    const double thr = nsigma * sigma_bg;
-    out.resize(flux.size());
-    for (size_t j = 0; j < flux.size(); ++j) {
-        const double F = std::max(flux[j], 0.0);
-        int r = R_fit;
-        while (r < R_cap && F * sb[r - 1] > thr) ++r;
-        out[j] = r;
-    }
+    double* d_res = d_sb + sb.size();
+    check(cudaMemcpyAsync(d_sb, sb.data(), sizeof(double) * sb.size(), cudaMemcpyHostToDevice, st), "h2d");
+    k_noise_quantile<<<1, kQuantThreads, 0, st>>>(d_w, step, nsamp, d_buf, d_res);
+    check(cudaGetLastError(), "k_noise_quantile");
+    k_model_radii<<<(unsigned)((n_act + 255) / 256), 256, 0, st>>>(n_act, d_act, d_f0, d_sb, d_res, nsigma, R_fit,
+                                                                   R_cap, d_R);
+    check(cudaGetLastError(), "k_model_radii");
+    out.resize(n_act);
+    double res[2] = {0, 0};
+    check(cudaMemcpyAsync(res, d_res, sizeof(res), cudaMemcpyDeviceToHost, st), "d2h");
+    check(cudaMemcpyAsync(out.data(), d_R, sizeof(int32_t) * n_act, cudaMemcpyDeviceToHost, st), "d2h");
+    check(cudaStreamSynchronize(st), "sync");
+    if (res[1] == 0) throw ArgError{"model_rad=:auto found no positive finite weights to estimate the noise"};
 }
 
 }  // namespace cpb

@@ -2401,6 +2401,10 @@ int64_t rect_offsets(cpb_ctx* ctx, const char* tag, const TileLists& tl, int nty
 // ---------------------------------------------------------------------------
 namespace {
 
+// Whether the :auto radii's table (R_cap + 2 doubles) fits the disk table's buffer, which
+// is not used before the final pass.
+bool radii_in_spread_tab(int R_cap, int R) { return R_cap + 2 <= spread_tab_len(R); }
+
 // Bytes arena_carve reserves for one named buffer of `bytes`.
 size_t carve_size(size_t bytes) { return (std::max<size_t>(bytes, 256) + 255) & ~size_t(255); }
 
@@ -2491,7 +2495,11 @@ size_t sim_scratch_bound(const cpb_sim_params* P, int64_t ny, int64_t nx, int64_
     b += 2 * carve_size(4 * n) + carve_size(8 * np);                              // ay, ax, theta
     b += carve_size(npix) + carve_size(8);                                         // umask, ucnt
     if (dbg_pixels) b += carve_size(4 * S2 * n);
-    if (P->model_rad_auto) b += carve_size(4 * n);
+    if (P->model_rad_auto) {
+        b += carve_size(4 * n);
+        const int R_cap = (int)std::ceil(P->model_rad_max < 0 ? 10 * P->fit_rad : P->model_rad_max);
+        if (!radii_in_spread_tab(R_cap, R)) b += carve_size(8 * ((size_t)std::max(R_cap, 0) + 2));
+    }
     b += tiles_bound(n, R, ntiles);
     if (Rm != R || P->model_rad_auto) b += tiles_bound(n, Rm, ntiles);
     b += (P->solver == CPB_SOLVER_LSMR ? 9 : 8) * carve_size(8 * np) +           // solver state (lsmr: hbar)
@@ -3032,24 +3040,13 @@ bool SimFit::setup() {
     double model_box_sum = 0;  // sum over active stars of (2 R_j + 1)^2
     if (P->model_rad_auto) {
         const int R_cap = (int)std::ceil(model_rad_max);
-        // the noise sample w[1 : step : end] and the active stars' catalogue fluxes
-        const int64_t step = std::max<int64_t>(1, npix / 65536);
-        const int64_t nsamp = (npix + step - 1) / step;
-        std::vector<double> wsamp(nsamp), f0(n_stars);
-        std::vector<int32_t> h_act_order(n_act);
-        check(cudaMemcpy2DAsync(wsamp.data(), sizeof(double), w, step * sizeof(double), sizeof(double), nsamp,
-                                cudaMemcpyDeviceToHost, st), "d2h weight sample");
-        check(cudaMemcpyAsync(f0.data(), d_flux0, sizeof(double) * n_stars, cudaMemcpyDeviceToHost, st), "d2h");
-        check(cudaMemcpyAsync(h_act_order.data(), act, sizeof(int32_t) * n_act, cudaMemcpyDeviceToHost, st), "d2h");
-        check(cudaStreamSynchronize(st), "sync");
-        std::vector<double> fl(n_act);
-        for (int64_t j = 0; j < n_act; ++j) fl[j] = f0[h_act_order[j]];
-        model_radii_auto(psf, P->fixed_fwhm, P->model_rad_nsigma, fc.R, R_cap, wsamp, fl, h_modelR);
-        model_R = *std::max_element(h_modelR.begin(), h_modelR.end());
         d_modelR = S_<int32_t>("model_R", n_act);
-        check(cudaMemcpyAsync(d_modelR, h_modelR.data(), sizeof(int32_t) * n_act, cudaMemcpyHostToDevice, st),
-              "h2d model radii");
-        check(cudaStreamSynchronize(st), "sync");
+        // buffers of the final pass (residual, disk table) serve :auto, which runs before any render
+        double* d_sb = radii_in_spread_tab(R_cap, fc.R) ? S_<double>("spread_tab", spread_tab_len(fc.R))
+                                                        : S_<double>("radii_sb", R_cap + 2);
+        model_radii_auto(ctx, psf, P->fixed_fwhm, P->model_rad_nsigma, fc.R, R_cap, w, npix,
+                         S_<double>("resid", npix), d_sb, act, n_act, d_flux0, d_modelR, h_modelR);
+        model_R = *std::max_element(h_modelR.begin(), h_modelR.end());
         for (int32_t r : h_modelR) model_box_sum += (double)(2 * r + 1) * (2 * r + 1);
     } else {
         const int R_cap = (int)std::ceil(std::max(P->model_rad, P->fit_rad));
@@ -3133,9 +3130,15 @@ void SimFit::arena_precheck() {
         form(sizeof(double), Gran<double>::H);
     }
     need += carve_size(sizeof(Scalars)) + carve_size(live_tmp_bytes);  // scalars_freeze, newf_tmp
-    need += carve_size(48 * n_act) + carve_size(8 * n) + carve_size(8 * npix);
+    need += carve_size(48 * n_act) + carve_size(8 * n);
     need += carve_size(model_entries(Gran<double>::H) * 8) + rect_map_bound(tmod.npairs, n_act);
-    need += carve_size(8 * kSpreadRuleLen) + carve_size(8 * spread_tab_len(fc.R)) + carve_size(56 * n_act);
+    need += carve_size(8 * kSpreadRuleLen) + carve_size(56 * n_act);
+    // the residual and the disk table, unless :auto carved them already
+    auto later = [&](const char* name, size_t bytes) {
+        if (!ctx->arena->slots.count(name)) need += carve_size(bytes);
+    };
+    later("resid", 8 * npix);
+    later("spread_tab", 8 * spread_tab_len(fc.R));
     const size_t used = (ctx->arena->used + 255) & ~size_t(255);
     if (used + need > ctx->arena->cap)
         throw ArgError{"field too large for the no-allocation entry point: needs about " +

@@ -135,6 +135,7 @@ int cpb_ctx_destroy(cpb_ctx* ctx) {
         std::lock_guard<std::mutex> lk(ctx->mu);
         cudaSetDevice(ctx->device);
         if (ctx->copy_stream) cudaStreamSynchronize(ctx->copy_stream);
+        ctx->copier.reset();
         for (auto& kv : ctx->bufs)
             if (kv.second.p) cudaFreeAsync(kv.second.p, ctx->stream);
         ctx->bufs.clear();
@@ -429,9 +430,8 @@ int cpb_fit_simultaneous(cpb_ctx* ctx, const cpb_psf* psf, const cpb_sim_params*
         double* d_y = (double*)scratch(ctx, "in_y", sizeof(double) * std::max<int64_t>(n, 1));
         double* d_x = (double*)scratch(ctx, "in_x", sizeof(double) * std::max<int64_t>(n, 1));
         double* d_f = (double*)scratch(ctx, "in_flux", sizeof(double) * std::max<int64_t>(n, 1));
-        check(cudaMemcpyAsync(d_img, image, bytes, cudaMemcpyHostToDevice, st), "h2d image");
-        if (d_iv) check(cudaMemcpyAsync(d_iv, inv_var, bytes, cudaMemcpyHostToDevice, st), "h2d inv_var");
-        if (d_bk) check(cudaMemcpyAsync(d_bk, background, bytes, cudaMemcpyHostToDevice, st), "h2d background");
+        const HostCopy in[3] = {{d_img, image, bytes}, {d_iv, inv_var, bytes}, {d_bk, background, bytes}};
+        host_to_device(ctx, in, 3);
         if (n > 0) {
             check(cudaMemcpyAsync(d_y, y0, sizeof(double) * n, cudaMemcpyHostToDevice, st), "h2d y");
             check(cudaMemcpyAsync(d_x, x0, sizeof(double) * n, cudaMemcpyHostToDevice, st), "h2d x");
@@ -581,8 +581,8 @@ int cpb_fit_all_stars(cpb_ctx* ctx, const cpb_psf* psf, const cpb_lm_params* par
         const size_t bytes = (eltype == CPB_F64 ? 8 : 4) * (size_t)ny * (size_t)nx;
         void* d_img = scratch(ctx, "mp_in_image", bytes);
         void* d_iv = inv_var ? scratch(ctx, "mp_in_inv_var", bytes) : nullptr;
-        check(cudaMemcpyAsync(d_img, image, bytes, cudaMemcpyHostToDevice, ctx->stream), "h2d image");
-        if (d_iv) check(cudaMemcpyAsync(d_iv, inv_var, bytes, cudaMemcpyHostToDevice, ctx->stream), "h2d inv_var");
+        const HostCopy in[2] = {{d_img, image, bytes}, {d_iv, inv_var, bytes}};
+        host_to_device(ctx, in, 2);
         return fit_all_stars_dev(ctx, psf, params, fit_rad, n_passes, spread_model_fwhm, d_img, eltype, ny, nx, d_iv,
                                  n, init, out);
     });

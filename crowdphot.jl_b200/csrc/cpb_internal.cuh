@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <exception>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -687,6 +688,14 @@ struct cpb_psf {
     std::map<std::pair<int, double>, std::vector<double>> cog_sb;
 };
 
+namespace cpb {
+// Worker threads for large pageable host copies (cpb_hostcopy.cu).
+class HostCopier;
+struct HostCopierDelete {
+    void operator()(HostCopier* p) const;
+};
+}  // namespace cpb
+
 struct cpb_ctx {
     int device = 0;
     int n_sm = 0;
@@ -705,6 +714,7 @@ struct cpb_ctx {
     static constexpr int kCopyEvents = 16;
     cudaEvent_t copy_ev[kCopyEvents] = {};
     void* pinned = nullptr;  // small pinned staging for scalar readbacks
+    std::unique_ptr<cpb::HostCopier, cpb::HostCopierDelete> copier;  // made at the first large pageable copy
     // kernel instrumentation: launch counter (always on) and, when profiling is
     // enabled, CUDA-event timing of every launch on this context's stream
     int64_t launches = 0;
@@ -752,6 +762,34 @@ struct KernelScope {
     cudaEvent_t a = nullptr, b = nullptr;
     KernelScope(cpb_ctx* c, const char* n, double by);
     ~KernelScope();
+};
+// Host <-> device copies of user arrays (cpb_hostcopy.cu): large pageable ones run
+// over worker threads, the rest through the driver.  host_to_device: the host memory
+// may be reused on return, the context's stream continues behind the transfers.
+struct HostCopy {
+    void* device;
+    const void* host;  // null: nothing to copy
+    size_t bytes;
+};
+void host_to_device(cpb_ctx* ctx, const HostCopy* parts, int n);
+// One copy to the host, begun behind what the context's stream holds when it is
+// constructed; later work on the stream runs beside it and must not write `device`.
+// finish() ends it (small or pinned copies are queued there instead: synchronise the
+// stream after it).
+class DeviceToHost {
+  public:
+    DeviceToHost(cpb_ctx* ctx, void* host, const void* device, size_t bytes);
+    DeviceToHost(const DeviceToHost&) = delete;
+    DeviceToHost& operator=(const DeviceToHost&) = delete;
+    ~DeviceToHost();
+    void finish();
+
+  private:
+    cpb_ctx* ctx_;
+    HostCopier* copier_ = nullptr;
+    void* host_ = nullptr;
+    const void* device_ = nullptr;
+    size_t bytes_ = 0;
 };
 // Resolves pending event pairs into ctx->kstats (after a stream sync).
 void resolve_kernel_events(cpb_ctx* ctx);

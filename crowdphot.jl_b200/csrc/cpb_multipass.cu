@@ -875,6 +875,7 @@ int fit_all_stars_dev(cpb_ctx* ctx, const cpb_psf* psf, const cpb_lm_params* P, 
         check(cudaGetLastError(), "k_mp_validate");
     }
     check(cudaEventRecord(ctx->ev1, st), "event");
+    DeviceToHost res_copy(ctx, out->residual, resid, sizeof(double) * npix);
     check(cudaMemcpyAsync(prm.data(), d_prm, sizeof(double) * n * np, cudaMemcpyDeviceToHost, st), "d2h");
     check(cudaMemcpyAsync(valid.data(), d_valid, (size_t)n, cudaMemcpyDeviceToHost, st), "d2h");
     check(cudaMemcpyAsync(conv.data(), d_conv, (size_t)n, cudaMemcpyDeviceToHost, st), "d2h");
@@ -884,8 +885,7 @@ int fit_all_stars_dev(cpb_ctx* ctx, const cpb_psf* psf, const cpb_lm_params* P, 
     check(cudaMemcpyAsync(chisq.data(), d_chisq, sizeof(double) * n, cudaMemcpyDeviceToHost, st), "d2h");
     check(cudaMemcpyAsync(niter.data(), d_niter, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st), "d2h");
     check(cudaMemcpyAsync(&nfail, d_nfail, sizeof(int), cudaMemcpyDeviceToHost, st), "d2h");
-    if (out->residual)
-        check(cudaMemcpyAsync(out->residual, resid, sizeof(double) * npix, cudaMemcpyDeviceToHost, st), "d2h");
+    res_copy.finish();
     check(cudaStreamSynchronize(st), "sync");
     float ms = 0;
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);

@@ -3408,6 +3408,8 @@ void SimFit::finish() {
             nullptr, 0.0, nullptr, resid, umask, w, sw, data, sc, red, nullptr);
         check(cudaGetLastError(), "k_gather_final");
     }
+    // the residual image goes to the host beside the diagnostics, which only read it
+    DeviceToHost res_copy(ctx, out->residual, resid, sizeof(double) * npix);
     // spread_model reference disk, on the device: its width comes from the first
     // catalogue star's final parameters (k_spread_disk)
     const int kh = (int)std::ceil(P->fit_rad);
@@ -3475,8 +3477,7 @@ void SimFit::finish() {
     check(cudaMemcpyAsync(y0.data(), d_y0, sizeof(double) * n_stars, cudaMemcpyDeviceToHost, st), "d2h");
     check(cudaMemcpyAsync(x0.data(), d_x0, sizeof(double) * n_stars, cudaMemcpyDeviceToHost, st), "d2h");
     check(cudaMemcpyAsync(f0.data(), d_flux0, sizeof(double) * n_stars, cudaMemcpyDeviceToHost, st), "d2h");
-    if (out->residual)
-        check(cudaMemcpyAsync(out->residual, resid, sizeof(double) * npix, cudaMemcpyDeviceToHost, st), "d2h");
+    res_copy.finish();
     if (out->dbg_pixels)
         check(cudaMemcpyAsync(out->dbg_pixels, dbg_pix, sizeof(int32_t) * fc.S2 * n_act, cudaMemcpyDeviceToHost, st),
               "d2h");

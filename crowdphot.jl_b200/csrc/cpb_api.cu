@@ -309,13 +309,13 @@ int cpb_psf_upload(cpb_ctx* ctx, const cpb_psf_desc* d, cpb_psf** out) {
             std::vector<double> lpp;
             for (int k = 0; k < nn; ++k) {
                 DevNode& nd = nodes[k];
-                nd.LPY = (nd.ny + 2 + nd.isy - 1) / nd.isy;
-                nd.LPX = (nd.nx + 2 + nd.isx - 1) / nd.isx;
+                nd.LPY = (nd.ny + 3 + nd.isy - 1) / nd.isy;
+                nd.LPX = (nd.nx + 3 + nd.isx - 1) / nd.isx;
                 nd.lpoff = (int64_t)lpp.size();
                 const int64_t plane = (int64_t)nd.LPY * nd.LPX;
                 lpp.resize(lpp.size() + (size_t)(plane * nd.isy * nd.isx + 3) / 4 * 4, 0.0);
-                for (int64_t kk = 0; kk < nd.nx + 2; ++kk)
-                    for (int64_t ii = 0; ii < nd.ny + 2; ++ii) {
+                for (int64_t kk = 0; kk < nd.nx + 3; ++kk)
+                    for (int64_t ii = 0; ii < nd.ny + 3; ++ii) {
                         const int64_t si = std::min<int64_t>(std::max<int64_t>(ii - 1, 0), nd.ny - 1);
                         const int64_t sk = std::min<int64_t>(std::max<int64_t>(kk - 1, 0), nd.nx - 1);
                         lpp[nd.lpoff + ((ii % nd.isy) + (kk % nd.isx) * nd.isy) * plane + ii / nd.isy +
@@ -343,6 +343,7 @@ int cpb_psf_upload(cpb_ctx* ctx, const cpb_psf_desc* d, cpb_psf** out) {
                 };
                 fill(rpp, 0, 2);
                 fill(rpp32, 1, 4);
+                fill(rpp, 2, 1);
             }
             for (size_t q = 0; q < pp.size(); ++q) pp32[q] = (float)pp[q];
             // one device block and one copy for every table (256-byte aligned pieces)

@@ -38,24 +38,26 @@ struct DevNode {
     int64_t poff;
     int32_t PY, PX;     // ceil(ny / isy), ceil(nx / isx)
     int32_t isy, isx;   // integer oversampling (the reference's oversampling is a pair of Ints)
-    // edge-padded polyphase copy (fit_star): the node with one replicated sample
-    // on every side, so that a clamped stencil (empirical_models.jl:270-285) reads
-    // the same values as an interior one; padded sample (i + 1, k + 1) lives at
+    // edge-padded polyphase copy (fit_star, nodes too large for shared memory): the
+    // node with one replicated sample before and two after each axis, so that a
+    // clamped stencil (empirical_models.jl:270-285) reads the same values as an
+    // interior one; padded sample (i + 1, k + 1) lives at
     // lpoff + (((i + 1) % isy) + ((k + 1) % isx) * isy) * LPY * LPX
     //       + (i + 1) / isy + ((k + 1) / isx) * LPY.
     int64_t lpoff;
-    int32_t LPY, LPX;   // ceil((ny + 2) / isy), ceil((nx + 2) / isx)
-    // row-phase copies (the stamp kernels that stage the node in shared memory): the
-    // node with one replicated sample before and two after each axis, columns in
-    // order, rows regrouped by their index modulo GH * isy, GH the rows of a stamp
-    // granule (copy 0: FP64, GH = 2; copy 1: FP32, GH = 4); padded sample (p, q)
+    int32_t LPY, LPX;   // ceil((ny + 3) / isy), ceil((nx + 3) / isx)
+    // row-phase copies (the kernels that stage the node in shared memory): the node
+    // with one replicated sample before and two after each axis, columns in order,
+    // rows regrouped by their index modulo GH * isy, GH the pixel rows a lane takes
+    // (copy 0: FP64 stamps, GH = 2; copy 1: FP32 stamps, GH = 4; copy 2: fit_star,
+    // FP64, GH = 1; copies 0 and 2 in rpp64, copy 1 in rpp32); padded sample (p, q)
     // (0 is the replicate before sample 1) lives at
     //   rpoff[c] + ((p % (GH isy)) * RPY[c] + p / (GH isy)) * RPX + q.
     // The four column taps of a stencil row are adjacent, and at the same row of
     // consecutive granules they are RPX apart: RPX is odd, so the lanes of a warp
     // meet no shared-memory bank twice.
-    int64_t rpoff[2];
-    int32_t RPY[2], RPX;   // ceil((ny + 3) / (GH isy)), the odd number >= nx + 3
+    int64_t rpoff[3];
+    int32_t RPY[3], RPX;   // ceil((ny + 3) / (GH isy)), the odd number >= nx + 3
 };
 
 constexpr int kMaxNodes = 64;
@@ -218,6 +220,20 @@ __device__ __forceinline__ AxisSpan axis_span(double s, double centre, double or
     a.l0 = (int)floor(u);
     a.f = u - (double)a.l0;
     return a;
+}
+
+// Value and derivative weights of the four samples of Keys' cubic convolution
+// (empirical_models.jl:185-196, a = -1/2) at fraction t.
+__device__ __forceinline__ void keys_weights(double t, double w[4], double d[4]) {
+    const double t2 = t * t, t3 = t2 * t;
+    w[0] = -0.5 * t + t2 - 0.5 * t3;
+    w[1] = 1.0 - 2.5 * t2 + 1.5 * t3;
+    w[2] = 0.5 * t + 2.0 * t2 - 1.5 * t3;
+    w[3] = -0.5 * t2 + 0.5 * t3;
+    d[0] = -0.5 + 2.0 * t - 1.5 * t2;
+    d[1] = -5.0 * t + 4.5 * t2;
+    d[2] = 0.5 + 4.0 * t - 4.5 * t2;
+    d[3] = -t + 1.5 * t2;
 }
 
 template <typename D>

@@ -710,9 +710,10 @@ __global__ void __launch_bounds__(256) k_lm_irls(int64_t n_cut, LMConst L, DevPs
 // cutouts.  Arithmetic per pixel is corner_eval's (psf_fitting.jl:1233-1321
 // restated); only the order of the per-lane sums differs.
 // ---------------------------------------------------------------------------
+// Cholesky factor of A (upper triangle U, reciprocal diagonal Ri: one division per
+// row instead of one per use); false unless positive definite.
 template <int NF>
-__device__ __forceinline__ bool chol_solve_t(const double* A, const double* b, double* x) {
-    double U[NF * NF];
+__device__ __forceinline__ bool chol_factor_t(const double* A, double* U, double* Ri) {
 #pragma unroll
     for (int j = 0; j < NF; ++j)
 #pragma unroll
@@ -722,27 +723,30 @@ __device__ __forceinline__ bool chol_solve_t(const double* A, const double* b, d
             for (int k = 0; k < i; ++k) s -= U[k + i * NF] * U[k + j * NF];
             if (i == j) {
                 if (!(s > 0)) return false;
-                U[j + j * NF] = sqrt(s);
+                Ri[j] = 1.0 / sqrt(s);
             } else {
-                U[i + j * NF] = s / U[i + i * NF];
+                U[i + j * NF] = s * Ri[i];
             }
         }
+    return true;
+}
+template <int NF>
+__device__ __forceinline__ void chol_back_t(const double* U, const double* Ri, const double* b, double* x) {
     double y[NF];
 #pragma unroll
     for (int i = 0; i < NF; ++i) {
         double s = b[i];
 #pragma unroll
         for (int k = 0; k < i; ++k) s -= U[k + i * NF] * y[k];
-        y[i] = s / U[i + i * NF];
+        y[i] = s * Ri[i];
     }
 #pragma unroll
     for (int i = NF - 1; i >= 0; --i) {
         double s = y[i];
 #pragma unroll
         for (int k = i + 1; k < NF; ++k) s -= U[i + k * NF] * x[k];
-        x[i] = s / U[i + i * NF];
+        x[i] = s * Ri[i];
     }
-    return true;
 }
 
 // v[idx] for a register array v and a runtime index, without local memory.
@@ -754,108 +758,73 @@ __device__ __forceinline__ double pick(const double* v, int idx) {
     return r;
 }
 
-// Stencil row / column taps of one axis in the polyphase copy: with the 0-based
-// sample index i0 of the first tap, the four taps i0..i0+3 live at
-// (i % is) * pstride + (i / is) * qstride.
-__device__ __forceinline__ void pp_taps(int i0, int is, float inv_is, int pstride, int qstride, int* t) {
-    int q = __float2int_rz(__int2float_rn(i0) * inv_is);
-    int r = i0 - q * is;
-    if (r < 0) {
-        r += is;
-        --q;
-    } else if (r >= is) {
-        r -= is;
-        ++q;
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        t[k] = r * pstride + q * qstride;
-        if (++r == is) {
-            r = 0;
-            ++q;
-        }
-    }
-}
-
 struct PPNode {
-    const double* pp;   // this node's edge-padded polyphase block (DevNode::lpoff)
+    const double* pp;   // this node's samples: row-phase copy 2 (staged in shared memory) or the
+                        // edge-padded polyphase copy (read from global memory) (DevNode)
     DevNode nd;
     int plane;          // LPY * LPX
-    float inv_isy, inv_isx;
+    int nel;            // doubles of the row-phase copy (0: not staged)
 };
 
-// Stencil offsets of the previous pixel a lane evaluated (ly = lx = 0: none).
-struct TapCursor {
-    int ly, lx;
-    int ry[4], cx[4];
-};
+// A single-node star over a box of ny x nx pixels whose first pixel is (y1, x1): the
+// pixels its table reaches, the cubic weights every pixel of it shares (axis_span) and
+// the sample addresses.  SMEM: row-phase copy (the column taps are adjacent), else the
+// polyphase copy (consecutive rows are adjacent, whatever the tap).  Set by a whole warp.
+template <bool SMEM>
+struct NodeStar {
+    AxisSpan sy, sx;
+    double wx[4], dx[4], wy[4], dy[4];
+    int rb[4], cb[4], rs, cs;  // tap (r, c) of box pixel (i, j): rb[r] + cb[c] + i * rs + j * cs
 
-// Single-node image profile and its derivatives in the detector frame:
-// s, dsdY = -sy * dp/dv, dsdX = -sx * dp/du (grid_profile with weights (1, 0, 0, 0)).
-// pp: the node's edge-padded polyphase samples (shared or global memory), so the
-// clamped stencils at the grid's border need no special case.  (di, dj): how far
-// the cutout row / column moved since the lane's previous pixel; when the
-// stencil origin moved by whole oversampling periods the cached tap offsets are
-// advanced instead of recomputed.
-__device__ __forceinline__ void pp_profile(const PPNode& N, const double* pp, TapCursor& T, int di, int dj, double Y,
-                                           double X, double py, double px, double& s, double& dY, double& dX) {
-    const DevNode& nd = N.nd;
-    const double u = nd.sx * (px - X) + nd.ox;
-    const double v = nd.sy * (py - Y) + nd.oy;
-    const int nyd = nd.ny, nxd = nd.nx;
-    // NaN and infinite u, v fail these range tests, as isfinite would
-    const bool inb = u >= 1.0 && u <= (double)nxd && v >= 1.0 && v <= (double)nyd;
-    if (!inb) {
-        s = nd.fill;
-        dY = 0.0;
-        dX = 0.0;
-        T.ly = T.lx = 0;
-        return;
-    }
-    const int lx = clampi((int)floor(u), 1, nxd - 1);
-    const int ly = clampi((int)floor(v), 1, nyd - 1);
-    const double du = u - (double)lx, dv = v - (double)ly;
-    if (T.ly != 0 && ly == T.ly + nd.isy * di) {
+    __device__ __forceinline__ void set(const PPNode& N, double Y, double X, int y1, int x1, int ny, int nx) {
+        const DevNode& nd = N.nd;
+        sy = axis_span(nd.sy, Y, nd.oy, nd.ny, y1, ny);
+        sx = axis_span(nd.sx, X, nd.ox, nd.nx, x1, nx);
+        keys_weights(sy.f, wy, dy);
+        keys_weights(sx.f, wx, dx);
+        int q = sy.l0 - 1, e = q / nd.isy, ph = q - e * nd.isy;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) T.ry[k] += di;
-    } else {
-        pp_taps(ly - 1, nd.isy, N.inv_isy, N.plane, 1, T.ry);  // padded index of sample ly - 2
-    }
-    if (T.lx != 0 && lx == T.lx + nd.isx * dj) {
+        for (int r = 0; r < 4; ++r) {
+            rb[r] = SMEM ? (ph * nd.RPY[2] + e - sy.lo) * nd.RPX + sx.l0 - 1 - nd.isx * sx.lo : ph * N.plane + e - sy.lo;
+            if (++ph == nd.isy) {
+                ph = 0;
+                ++e;
+            }
+        }
+        rs = SMEM ? nd.RPX : 1;
+        cs = SMEM ? nd.isx : nd.LPY;
+        q = sx.l0 - 1;
+        e = q / nd.isx;
+        ph = q - e * nd.isx;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) T.cx[k] += dj * nd.LPY;
-    } else {
-        pp_taps(lx - 1, nd.isx, N.inv_isx, nd.isy * N.plane, nd.LPY, T.cx);
+        for (int c = 0; c < 4; ++c) {
+            cb[c] = SMEM ? c : ph * nd.isy * N.plane + (e - sx.lo) * nd.LPY;
+            if (++ph == nd.isx) {
+                ph = 0;
+                ++e;
+            }
+        }
     }
-    T.ly = ly;
-    T.lx = lx;
-    double row[4], drow[4];
+    // the four interpolated rows (and their column derivatives) of in-table pixel (i, j)
+    template <bool GRAD>
+    __device__ __forceinline__ void rows(const double* pp, int i, int j, double (&rv)[4], double (&rd)[4]) const {
+        const double* at = pp + (i * rs + j * cs);
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const double* q = pp + T.ry[r];
-        const double a = q[T.cx[0]], b = q[T.cx[1]], c = q[T.cx[2]], e = q[T.cx[3]];
-        const double k1 = (c - a) / 2;
-        const double k4 = c - b - k1;
-        const double k2 = 3 * k4 - (e - b) / 2 + k1;
-        const double k3 = k4 - k2;
-        row[r] = du * (du * (du * k3 + k2) + k1) + b;
-        drow[r] = du * (3 * du * k3 + 2 * k2) + k1;
+        for (int r = 0; r < 4; ++r) {
+            const double* q = at + rb[r];
+            const double a = q[SMEM ? 0 : cb[0]], b = q[SMEM ? 1 : cb[1]], c = q[SMEM ? 2 : cb[2]],
+                         e = q[SMEM ? 3 : cb[3]];
+            rv[r] = wx[0] * a + wx[1] * b + wx[2] * c + wx[3] * e;
+            if (GRAD) rd[r] = dx[0] * a + dx[1] * b + dx[2] * c + dx[3] * e;
+        }
     }
-    const double v1 = (row[2] - row[0]) / 2;
-    const double v4 = row[2] - row[1] - v1;
-    const double v2 = 3 * v4 - (row[3] - row[1]) / 2 + v1;
-    const double v3 = v4 - v2;
-    const double pv = dv * (dv * (dv * v3 + v2) + v1) + row[1];
-    const double pdv = dv * (3 * dv * v3 + 2 * v2) + v1;
-    const double u1 = (drow[2] - drow[0]) / 2;
-    const double u4 = drow[2] - drow[1] - u1;
-    const double u2 = 3 * u4 - (drow[3] - drow[1]) / 2 + u1;
-    const double u3 = u4 - u2;
-    const double pdu = dv * (dv * (dv * u3 + u2) + u1) + drow[1];
-    s = pv;
-    dY = -(nd.sy * pdv);
-    dX = -(nd.sx * pdu);
-}
+    __device__ __forceinline__ double value(const PPNode& N, const double* pp, int i, int j) const {
+        if (i < sy.lo || i > sy.hi || j < sx.lo || j > sx.hi) return N.nd.fill;
+        double rv[4], rd[4];
+        rows<false>(pp, i, j, rv, rd);
+        return wy[0] * rv[0] + wy[1] * rv[1] + wy[2] * rv[2] + wy[3] * rv[3];
+    }
+};
 
 // A cutout is fitted by a team of WPC warps (1: one warp a cutout, the
 // throughput form for large batches; 4: a 128-thread team, the latency form for
@@ -896,37 +865,46 @@ __device__ __forceinline__ void team_sum(double (&v)[K], double* red) {
 // the free set (A: NF x NF column-major, b: NF); every thread of the team returns
 // the same cost.  (qs, rs): the column / row step of a 32 * WPC pixel stride;
 // red: the team's reduction scratch (WPC * (1 + NF + NF (NF + 1) / 2) doubles).
-template <typename TI, int NP, int NF, int WPC>
-__device__ double lm_accum_t(const PPNode& N, const double* pp, const LMConst& L, const TI* __restrict__ pix,
-                             const TI* __restrict__ iv, int ny, int nx, int y1, int x1, int qs, int rs,
+// One element into shared memory, asynchronously (cp.async.wait_all completes it).
+template <typename TI>
+__device__ __forceinline__ void stage_async(TI* dst, const TI* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+                 "n"(sizeof(TI))
+                 : "memory");
+}
+
+// ID: the free parameters are the first NF (L.fidx[k] == k), so only their entries
+// are summed; otherwise all NP are and the free ones picked at the end.
+template <typename TI, int NP, int NF, bool SMEM, int WPC, bool ID>
+__device__ double lm_accum_t(const PPNode& N, const double* pp, const LMConst& L, const TI* pix,
+                             const TI* iv, int ny, int nx, int y1, int x1, int qs, int rs,
                              const double* fv, double* A, double* b, double* red) {
-    constexpr int NT = NP * (NP + 1) / 2;
+    constexpr int NA = ID ? NF : NP;
+    constexpr int NT = NA * (NA + 1) / 2;
     constexpr int TS = 32 * WPC;  // team size = pixel stride
     const int lane = threadIdx.x % TS;
     const int q32 = qs, r32 = rs;
-    double Af[NT], bf[NP], cost = 0;
+    double Af[NT], bf[NA], cost = 0;
 #pragma unroll
     for (int q = 0; q < NT; ++q) Af[q] = 0;
 #pragma unroll
-    for (int q = 0; q < NP; ++q) bf[q] = 0;
+    for (int q = 0; q < NA; ++q) bf[q] = 0;
     const int npx = ny * nx;
     // one pixel's contribution: cost, b and the upper triangle of A
-    auto acc = [&](int e, double mval, const double* gv) {
-        const double r = mval - (double)pix[e];
+    auto acc = [&](double d, double vv, double mval, const double* gv) {
+        const double r = mval - d;
         double w = 1.0;
-        if (iv) {
-            const double vv = (double)iv[e];
-            w = (isfinite(vv) && vv > 0) ? vv : 0.0;
-        }
+        if (iv) w = (isfinite(vv) && vv > 0) ? vv : 0.0;
         const double wr = w * r;
         cost = wr * r + cost;
         int t = 0;
 #pragma unroll
-        for (int q = 0; q < NP; ++q) {
+        for (int q = 0; q < NA; ++q) {
             bf[q] = wr * gv[q] + bf[q];
+            const double wg = w * gv[q];
 #pragma unroll
             for (int pq = 0; pq <= q; ++pq) {
-                Af[t] = (w * gv[pq]) * gv[q] + Af[t];
+                Af[t] = wg * gv[pq] + Af[t];
                 ++t;
             }
         }
@@ -950,7 +928,7 @@ __device__ double lm_accum_t(const PPNode& N, const double* pp, const LMConst& L
             gv[2] = -2 * Ag * (1 + gp * sq) / fwhm;
             gv[3] = g / norm;
             gv[NP - 1] = 1.0;
-            acc(e, amp * g + bkg, gv);
+            acc((double)pix[e], iv ? (double)iv[e] : 1.0, amp * g + bkg, gv);
             i += r32;
             j += q32;
             if (i >= ny) {
@@ -961,51 +939,60 @@ __device__ double lm_accum_t(const PPNode& N, const double* pp, const LMConst& L
     } else {
         const DevNode& nd = N.nd;
         const double Y = fv[0], X = fv[1], flux = fv[2], bkg = fv[3];
-        // Cutout pixels outside [ilo, ihi] x [jlo, jhi] are at least one pixel
-        // (>= one grid sample) beyond the grid, so their profile is the fill
-        // value with zero derivatives; the rectangle is evaluated in full.
-        int ilo = 0, ihi = ny - 1, jlo = 0, jhi = nx - 1;
-        if (isfinite(Y) && isfinite(X)) {
-            const double ya = Y - (double)y1 + (1.0 - nd.oy) / nd.sy;
-            const double yb = Y - (double)y1 + ((double)nd.ny - nd.oy) / nd.sy;
-            const double xa = X - (double)x1 + (1.0 - nd.ox) / nd.sx;
-            const double xb = X - (double)x1 + ((double)nd.nx - nd.ox) / nd.sx;
-            ilo = (int)fmin(fmax(0.0, floor(ya) - 1.0), (double)ny);
-            ihi = (int)fmax(fmin((double)(ny - 1), ceil(yb) + 1.0), -1.0);
-            jlo = (int)fmin(fmax(0.0, floor(xa) - 1.0), (double)nx);
-            jhi = (int)fmax(fmin((double)(nx - 1), ceil(xb) + 1.0), -1.0);
+        NodeStar<SMEM> T;
+        T.set(N, Y, X, y1, x1, ny, nx);
+        // the derivatives by Y and X carry -flux * oversampling: in the weights
+        {
+            const double fy = -(flux * nd.sy), fx = -(flux * nd.sx);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                T.dy[k] *= fy;
+                T.dx[k] *= fx;
+            }
         }
+        // pixels outside [ilo, ihi] x [jlo, jhi] are beyond the table: the fill value
+        // with zero derivatives
+        const int ilo = T.sy.lo, ihi = T.sy.hi, jlo = T.sx.lo, jhi = T.sx.hi;
         const int ni = ihi - ilo + 1, nj = jhi - jlo + 1;
         if (ni > 0 && nj > 0) {
             const int nr = ni * nj, rq = TS / ni, rr = TS % ni;
-            int ii = lane % ni, jj = lane / ni, di = 0, dj = 0;
-            TapCursor T;
-            T.ly = T.lx = 0;
+            int i = ilo + lane % ni, j = jlo + lane / ni;
+            // the next pixel's data and weight load behind this one's arithmetic
+            double dn = 0.0, vn = 1.0;
+            if (lane < nr) {
+                dn = (double)pix[i + j * ny];
+                if (iv) vn = (double)iv[i + j * ny];
+            }
             for (int k = lane; k < nr; k += TS) {
-                const int i = ilo + ii, j = jlo + jj;
-                double s, dY, dX;
-                pp_profile(N, pp, T, di, dj, Y, X, (double)(y1 + i), (double)(x1 + j), s, dY, dX);
-                const double gv[NP] = {flux * dY, flux * dX, s, 1.0};
-                acc(i + j * ny, flux * s + bkg, gv);
-                ii += rr;
-                jj += rq;
-                di = rr;
-                dj = rq;
-                if (ii >= ni) {
-                    ii -= ni;
-                    ++jj;
-                    di -= ni;
-                    ++dj;
+                const double d = dn, vv = vn;
+                const int ic = i, jc = j;
+                i += rr;
+                j += rq;
+                if (i > ihi) {
+                    i -= ni;
+                    ++j;
                 }
+                if (k + TS < nr) {
+                    dn = (double)pix[i + j * ny];
+                    if (iv) vn = (double)iv[i + j * ny];
+                }
+                double rv[4], rd[4], gv[4];
+                T.template rows<true>(pp, ic, jc, rv, rd);
+                const double s = T.wy[0] * rv[0] + T.wy[1] * rv[1] + T.wy[2] * rv[2] + T.wy[3] * rv[3];
+                gv[0] = T.dy[0] * rv[0] + T.dy[1] * rv[1] + T.dy[2] * rv[2] + T.dy[3] * rv[3];
+                gv[1] = T.wy[0] * rd[0] + T.wy[1] * rd[1] + T.wy[2] * rd[2] + T.wy[3] * rd[3];
+                gv[2] = s;
+                gv[3] = 1.0;
+                acc(d, vv, flux * s + bkg, gv);
             }
         }
         if (ni < ny || nj < nx) {
-            const double s = nd.fill, dY = 0.0, dX = 0.0;
-            const double gv[NP] = {flux * dY, flux * dX, s, 1.0};
-            const double mval = flux * s + bkg;
+            const double gv[4] = {flux * 0.0, flux * 0.0, nd.fill, 1.0};
+            const double mval = flux * nd.fill + bkg;
             int i = lane % ny, j = lane / ny;
             for (int e = lane; e < npx; e += TS) {
-                if (!(i >= ilo && i <= ihi && j >= jlo && j <= jhi)) acc(e, mval, gv);
+                if (!(i >= ilo && i <= ihi && j >= jlo && j <= jhi))
+                    acc((double)pix[e], iv ? (double)iv[e] : 1.0, mval, gv);
                 i += r32;
                 j += q32;
                 if (i >= ny) {
@@ -1021,12 +1008,21 @@ __device__ double lm_accum_t(const PPNode& N, const double* pp, const LMConst& L
         int t = 0;
 #pragma unroll
         for (int jq = 0; jq < NF; ++jq) {
-            bp[jq] = pick<NP>(bf, L.fidx[jq]);
+            if (ID) {
+                bp[jq] = bf[jq];
+            } else {
+                bp[jq] = pick<NA>(bf, L.fidx[jq]);
+            }
 #pragma unroll
             for (int iq = 0; iq <= jq; ++iq) {
-                const int a = L.fidx[iq], c = L.fidx[jq];
-                const int lo = min(a, c), hi = max(a, c);
-                Ap[t++] = pick<NT>(Af, hi * (hi + 1) / 2 + lo);
+                if (ID) {
+                    Ap[t] = Af[t];
+                } else {
+                    const int a = L.fidx[iq], c = L.fidx[jq];
+                    const int lo = min(a, c), hi = max(a, c);
+                    Ap[t] = pick<NT>(Af, hi * (hi + 1) / 2 + lo);
+                }
+                ++t;
             }
         }
     }
@@ -1058,17 +1054,19 @@ __device__ double lm_accum_t(const PPNode& N, const double* pp, const LMConst& L
 // fallback is the general one.
 template <int NF>
 __device__ void lm_cov_t(const double* A, double* cov) {
-    double e[NF], x[NF];
-    bool ok = true;
+    double U[NF * NF], Ri[NF], e[NF], x[NF];
+    if (!chol_factor_t<NF>(A, U, Ri)) {
+        lm_cov(A, NF, cov);
+        return;
+    }
 #pragma unroll
     for (int c = 0; c < NF; ++c) {
 #pragma unroll
         for (int i = 0; i < NF; ++i) e[i] = (i == c) ? 1.0 : 0.0;
-        ok = ok && chol_solve_t<NF>(A, e, x);
+        chol_back_t<NF>(U, Ri, e, x);
 #pragma unroll
         for (int i = 0; i < NF; ++i) cov[i + c * NF] = x[i];
     }
-    if (!ok) lm_cov(A, NF, cov);
 }
 
 // LM bookkeeping of one cutout, kept in shared memory between normal-equation
@@ -1162,11 +1160,11 @@ __device__ __forceinline__ bool lm_step(LMState<NP, NF>& S, const LMConst& L, do
             break;
         }
         ++iter;
-        double gcos = 0;
+        bool gsmall = true;  // the largest gradient cosine is within g_tol (false with a NaN)
 #pragma unroll
         for (int k = 0; k < NF; ++k)
-            gcos = nan_max(gcos, fabs(b[k]) / (sqrt(A[k + k * NF] * cost) + 2.220446049250313e-16));
-        if (gcos <= L.g_tol) {
+            gsmall = gsmall && fabs(b[k]) <= L.g_tol * (sqrt(A[k + k * NF] * cost) + 2.220446049250313e-16);
+        if (gsmall) {
             gconv = conv = 1;
             done = true;
             break;
@@ -1181,10 +1179,12 @@ __device__ __forceinline__ bool lm_step(LMState<NP, NF>& S, const LMConst& L, do
 #pragma unroll
             for (int k = 0; k < NF; ++k) Ad[k + k * NF] += lam;
         }
-        if (!chol_solve_t<NF>(Ad, b, d)) {
+        double U[NF * NF], Ri[NF];
+        if (!chol_factor_t<NF>(Ad, U, Ri)) {
             lam = fmin(lam * L.lambda_up, L.lambda_max);
             continue;
         }
+        chol_back_t<NF>(U, Ri, b, d);
 #pragma unroll
         for (int k = 0; k < NF; ++k) d[k] = -d[k];
         double db = 0, dAd = 0;
@@ -1241,20 +1241,37 @@ __device__ __forceinline__ bool lm_step(LMState<NP, NF>& S, const LMConst& L, do
     return done;
 }
 
-constexpr int kLMThreads = 256;
+// Threads of a block, one block an SM (128 registers a thread): one staged node serves
+// every team and the rest of the shared memory holds the teams' cutouts.
+constexpr int kLMThreads = 512;
 
 // fit_star of one cutout by a team (pixels pix / weights iv, column-major
 // ny x nx whose first pixel is image pixel (y1, x1); init: the NP model
 // parameters, fixed ones replaced by L.fixv).  Returns 0 with the result in S,
 // or CPB_ERR_ARGUMENT when the inputs fail _prepare_fit_star_inputs's checks
 // (psf_fitting.jl:61-90) or lm_irls's dof test (:461-467).
-template <typename TI, int NP, int NF, int WPC>
-__device__ int lm_team_fit(const PPNode& N, const double* pp, const LMConst& L, const TI* __restrict__ pix,
-                           const TI* __restrict__ iv, int ny, int nx, int y1, int x1, const double* init,
-                           LMState<NP, NF>& S, double* red, int lane) {
+template <typename TI, int NP, int NF, bool SMEM, int WPC, bool ID>
+__device__ int lm_team_fit(const PPNode& N, const double* pp, const LMConst& L, const TI* pix,
+                           const TI* iv, int ny, int nx, int y1, int x1, const double* init,
+                           LMState<NP, NF>& S, double* red, int lane, unsigned char* stage, int stage_bytes) {
     constexpr int TS = 32 * WPC;
     const int64_t nobs = (int64_t)ny * nx;
     if (ny <= 0 || nx <= 0) return CPB_ERR_ARGUMENT;
+    // the cutout goes to the team's shared memory, every pixel in flight at once: each
+    // pass over it would otherwise wait for L2 pixel by pixel
+    if (nobs * (iv ? 2 : 1) * (int64_t)sizeof(TI) <= stage_bytes) {
+        TI* sp = (TI*)stage;
+        TI* si = sp + nobs;
+        team_sync<WPC>();  // the previous cutout is no longer read
+        for (int e = lane; e < (int)nobs; e += TS) {
+            stage_async(sp + e, pix + e);
+            if (iv) stage_async(si + e, iv + e);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        team_sync<WPC>();
+        pix = sp;
+        if (iv) iv = si;
+    }
     bool bad = !(nobs - NF > 0);
     if (iv) {
         double nv[1] = {0.0};
@@ -1287,25 +1304,25 @@ __device__ int lm_team_fit(const PPNode& N, const double* pp, const LMConst& L, 
         double fc[NP], Ac[NF * NF], bc[NF];
 #pragma unroll
         for (int q = 0; q < NP; ++q) fc[q] = S.fc[q];
-        const double cost_c = lm_accum_t<TI, NP, NF, WPC>(N, pp, L, pix, iv, ny, nx, y1, x1, qs, rs, fc, Ac, bc, red);
+        const double cost_c = lm_accum_t<TI, NP, NF, SMEM, WPC, ID>(N, pp, L, pix, iv, ny, nx, y1, x1, qs, rs, fc, Ac, bc, red);
         if (lm_step<NP, NF, WPC>(S, L, cost_c, Ac, bc, lane)) break;
     }
     return 0;
 }
 
-template <typename TI, int NP, int NF, bool SMEM, int WPC>
-__global__ void __launch_bounds__(kLMThreads, 2) k_lm_t(int64_t n_cut, LMConst L, PPNode N,
+template <typename TI, int NP, int NF, bool SMEM, int WPC, bool ID>
+__global__ void __launch_bounds__(kLMThreads, 1) k_lm_t(int64_t n_cut, LMConst L, PPNode N,
                                              const int64_t* __restrict__ offs, const int32_t* __restrict__ cny,
                                              const int32_t* __restrict__ cnx, const int32_t* __restrict__ cy1,
                                              const int32_t* __restrict__ cx1, const TI* __restrict__ pixels,
                                              const TI* __restrict__ ivs, const double* __restrict__ init, LMOut out,
-                                             unsigned long long* __restrict__ queue) {
+                                             unsigned long long* __restrict__ queue, int stage_bytes) {
     constexpr int TS = 32 * WPC;
     constexpr int KR = 1 + NF + NF * (NF + 1) / 2;
     __shared__ LMState<NP, NF> states[kLMThreads / TS];
     __shared__ double red_all[(kLMThreads / 32) * KR];
     __shared__ unsigned long long cut_sh[kLMThreads / TS];
-    extern __shared__ double node_smem[];
+    extern __shared__ __align__(16) double node_smem[];
     const int team = threadIdx.x / TS;
     LMState<NP, NF>& S = states[team];
     double* red = red_all + team * WPC * KR;
@@ -1314,8 +1331,8 @@ __global__ void __launch_bounds__(kLMThreads, 2) k_lm_t(int64_t n_cut, LMConst L
     // loads: a 1-D bulk asynchronous copy measured 4.5 % slower for the whole kernel)
     const double* pp = N.pp;
     if (SMEM && NP == 4) {
-        const int nel = N.plane * N.nd.isy * N.nd.isx;
-        for (int k = threadIdx.x; k < nel; k += blockDim.x) node_smem[k] = N.pp[k];
+        for (int k = threadIdx.x; k < N.nel / 2; k += blockDim.x)  // padded to a multiple of four
+            ((double2*)node_smem)[k] = __ldg((const double2*)N.pp + k);
         __syncthreads();
         pp = node_smem;
     }
@@ -1333,8 +1350,9 @@ __global__ void __launch_bounds__(kLMThreads, 2) k_lm_t(int64_t n_cut, LMConst L
         const int64_t c = (int64_t)cc;
         const int ny = cny[c], nx = cnx[c];
         const int64_t o = (ny > 0 && nx > 0) ? offs[c] : 0;
-        const int st = lm_team_fit<TI, NP, NF, WPC>(N, pp, L, pixels + o, ivs ? ivs + o : nullptr, ny, nx, cy1[c],
-                                                    cx1[c], init + c * NP, S, red, lane);
+        const int st = lm_team_fit<TI, NP, NF, SMEM, WPC, ID>(N, pp, L, pixels + o, ivs ? ivs + o : nullptr, ny, nx, cy1[c],
+                                                    cx1[c], init + c * NP, S, red, lane,
+                                                    (unsigned char*)(node_smem + N.nel) + team * stage_bytes, stage_bytes);
         if (st != 0) {
             if (lane == 0) out.status[c] = st;
             team_sync<WPC>();
@@ -1388,26 +1406,30 @@ constexpr long long kDagSpinLimit = 1ll << 26;  // default: ~64 M polls of >= 64
 // three passes, against 58.2 ms with 1 and 41.0 ms with 8).
 constexpr int kDagWarps = 4;
 
-template <typename TIV, int NP, int NF, bool SMEM>
-__global__ void __launch_bounds__(kLMThreads, 2) k_mp_dag(LMConst L, PPNode N, DevPsf P, DagArgs A) {
+template <typename TIV, int NP, int NF, bool SMEM, bool ID>
+__global__ void __launch_bounds__(kLMThreads, 1) k_mp_dag(LMConst L, PPNode N, DevPsf P, DagArgs A,
+                                                               int stage_bytes) {
     constexpr int WPC = kDagWarps, TS = 32 * kDagWarps;
     constexpr int KR = 1 + NF + NF * (NF + 1) / 2;
     __shared__ LMState<NP, NF> states[kLMThreads / TS];
     __shared__ double red_all[(kLMThreads / 32) * KR];
     __shared__ int pos_sh[kLMThreads / TS];
-    extern __shared__ double node_smem[];
+    extern __shared__ __align__(16) double node_smem[];
     const int team = threadIdx.x / TS;
     LMState<NP, NF>& S = states[team];
     double* red = red_all + team * WPC * KR;
     const int lane = threadIdx.x % TS;
     const int gteam = blockIdx.x * (kLMThreads / TS) + team;
-    double* cpix = A.cpix + (int64_t)gteam * A.box_max;
-    double* civ = A.civ ? A.civ + (int64_t)gteam * A.box_max : nullptr;
+    // the team's cutout: in shared memory when every box of the pass fits
+    const bool staged = (int64_t)A.box_max * (A.civ ? 16 : 8) <= stage_bytes;
+    double* stage = node_smem + N.nel + team * (stage_bytes / 8);
+    double* cpix = staged ? stage : A.cpix + (int64_t)gteam * A.box_max;
+    double* civ = !A.civ ? nullptr : (staged ? stage + A.box_max : A.civ + (int64_t)gteam * A.box_max);
     const TIV* ivimg = (const TIV*)A.iv;
     const double* pp = N.pp;
     if (SMEM && NP == 4) {  // the node's polyphase samples, staged once per block
-        const int nel = N.plane * N.nd.isy * N.nd.isx;
-        for (int k = threadIdx.x; k < nel; k += blockDim.x) node_smem[k] = N.pp[k];
+        for (int k = threadIdx.x; k < N.nel / 2; k += blockDim.x)  // padded to a multiple of four
+            ((double2*)node_smem)[k] = __ldg((const double2*)N.pp + k);
         __syncthreads();
         pp = node_smem;
     }
@@ -1441,20 +1463,34 @@ __global__ void __launch_bounds__(kLMThreads, 2) k_mp_dag(LMConst L, PPNode N, D
         const int4 b = A.box[k];
         const int nb = b.z * b.w;
         const double* pin = A.pin + (int64_t)k * np;
+        // a star's model over its box: the staged node's weights once a star
+        NodeStar<SMEM> T;
+        double mflux = 0.0, mbkg = 0.0;
+        auto model_of = [&](const double* pr) {
+            if (NP != 4) return;
+            T.set(N, pr[0], pr[1], b.x, b.y, b.z, b.w);
+            mflux = pr[2];
+            mbkg = pr[3];
+        };
+        auto model_at = [&](const double* pr, int i, int j) {
+            return NP == 4 ? mflux * T.value(N, pp, i, j) + mbkg : mp_model(P, A.M, pr, b.x + i, b.y + j);
+        };
         // passes 2+: the previous model back in (:360-365), and the cutout
+        if (A.pass > 1) model_of(pin);
         for (int e = lane; e < nb; e += TS) {
             const int i = b.x + e % b.z, j = b.y + e / b.z;
             const int64_t q = (i - 1) + (int64_t)(j - 1) * A.ny;
             double r = __ldcg(A.resid + q);
             if (A.pass > 1) {
-                r = r + mp_model(P, A.M, pin, i, j);
+                r = r + model_at(pin, i - b.x, j - b.y);
                 __stcg(A.resid + q, r);
             }
             cpix[e] = r;
             if (civ) civ[e] = (double)ivimg[q];
         }
         team_sync<WPC>();
-        const int st = lm_team_fit<double, NP, NF, WPC>(N, pp, L, cpix, civ, b.z, b.w, b.x, b.y, pin, S, red, lane);
+        const int st = lm_team_fit<double, NP, NF, SMEM, WPC, ID>(N, pp, L, cpix, civ, b.z, b.w, b.x, b.y, pin, S, red, lane,
+                                                                     nullptr, 0);
         // bookkeeping (:373-401)
         const int64_t s = A.idx[k];
         double* ps = A.psub + (int64_t)k * np;
@@ -1486,10 +1522,11 @@ __global__ void __launch_bounds__(kLMThreads, 2) k_mp_dag(LMConst L, PPNode N, D
             double pr[NP];
 #pragma unroll
             for (int q = 0; q < NP; ++q) pr[q] = ps[q];
+            model_of(pr);
             for (int e = lane; e < nb; e += TS) {
                 const int i = b.x + e % b.z, j = b.y + e / b.z;
                 const int64_t q = (i - 1) + (int64_t)(j - 1) * A.ny;
-                const double r = __ldcg(A.resid + q) - mp_model(P, A.M, pr, i, j);
+                const double r = __ldcg(A.resid + q) - model_at(pr, i - b.x, j - b.y);
                 __stcg(A.resid + q, r);
                 if (A.snap) A.snap[A.snap_off[k] + e] = r;
             }
@@ -1570,6 +1607,40 @@ LMConst lm_const(const cpb_psf* psf, const cpb_lm_params* P, bool have_iv) {
     return L;
 }
 
+// The node as the fast forms read it: the row-phase copy for staging in shared memory
+// when two copies fit an SM, else the polyphase copy in global memory.
+PPNode pp_node(const cpb_psf* psf, bool staged_wanted, size_t& smem_bytes) {
+    PPNode N{};
+    smem_bytes = 0;
+    if (psf->dev.kind == CPB_PSF_CIRCULAR_GAUSSIAN) return N;
+    N.nd = psf->h_nodes[0];
+    N.plane = N.nd.LPY * N.nd.LPX;
+    const int nel = (N.nd.isy * N.nd.RPY[2] * N.nd.RPX + 3) / 4 * 4;
+    if (staged_wanted && sizeof(double) * (size_t)nel <= 100 * 1024) {
+        N.nel = nel;
+        N.pp = psf->dev.rpp64 + N.nd.rpoff[2];
+        smem_bytes = sizeof(double) * (size_t)nel;
+    } else {
+        N.pp = psf->dev.lpp64 + N.nd.lpoff;
+    }
+    return N;
+}
+
+// Shared memory of each of a block's teams for its cutout, beside the staged node.
+int lm_stage_bytes(cpb_ctx* ctx, size_t node_bytes, int teams) {
+    int optin = 0;
+    check(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device), "attr");
+    const int64_t left = (int64_t)optin - 16 * 1024 - (int64_t)node_bytes;  // 16 KB: the static state
+    return left <= 0 ? 0 : (int)(left / teams / 16 * 16);
+}
+
+// Whether the free parameters are the model's first nf (their sums need no picking).
+bool lm_ident(const LMConst& L) {
+    for (int k = 0; k < L.nf; ++k)
+        if (L.fidx[k] != k) return false;
+    return true;
+}
+
 // One launch of k_lm over device-resident cutouts; `pix_elems` (the cutout
 // pixels in total, for the instrumentation's byte count) may be 0.
 // Launch configuration: persistent blocks per SM (1 or 2; 0 = 2) and whether the
@@ -1611,75 +1682,73 @@ void launch_lm(cpb_ctx* ctx, const cpb_psf* psf, const LMConst& L, int64_t n_cut
     }
     if (gauss || psf->dev.n_nodes == 1) {
         // fast form: compile-time parameter counts, polyphase taps, work queue
-        PPNode N{};
-        if (!gauss) {
-            N.nd = psf->h_nodes[0];
-            N.pp = psf->dev.lpp64 + N.nd.lpoff;
-            N.plane = N.nd.LPY * N.nd.LPX;
-            N.inv_isy = 1.0f / (float)N.nd.isy;
-            N.inv_isx = 1.0f / (float)N.nd.isx;
-        }
+        size_t node_bytes = 0;
+        const PPNode N = pp_node(psf, cfg.smem_node != 0, node_bytes);
+        const bool smem = node_bytes > 0, ident = lm_ident(L);
         auto* queue = cfg.queue ? cfg.queue
                                 : (unsigned long long*)scratch(ctx, "lm_queue", sizeof(unsigned long long));
         if (!(cfg.queue && cfg.queue_zeroed)) check(cudaMemsetAsync(queue, 0, sizeof(unsigned long long), st), "memset");
         // two persistent 256-thread blocks an SM (128 registers a thread); the
         // node's samples go to shared memory when two copies fit an SM
-        const size_t node_bytes = gauss ? 0 : sizeof(double) * (size_t)N.plane * N.nd.isy * N.nd.isx;
-        const bool smem = !gauss && node_bytes <= 100 * 1024 && cfg.smem_node != 0;
-        const int per_sm = cfg.blocks_per_sm == 1 ? 1 : 2;
+        // one block an SM, of half the threads with cfg.blocks_per_sm == 1
+        const int threads = cfg.blocks_per_sm == 1 ? kLMThreads / 2 : kLMThreads;
         // one warp a cutout while the batch fills the GPU's warps; a batch too
         // small for that (the late batches of fit_all_stars) gets 128-thread
         // teams, which cut each LM iteration's latency instead
-        const int64_t warps_total = (int64_t)ctx->n_sm * per_sm * (kLMThreads / 32);
+        const int64_t warps_total = (int64_t)ctx->n_sm * (threads / 32);
         const int wpc = cfg.team_warps == 4 || cfg.team_warps == 1 ? cfg.team_warps
                                                                   : (n_cut * 4 <= warps_total ? 4 : 1);
-        const unsigned blocks = (unsigned)std::min<int64_t>((n_cut * 32 * wpc + kLMThreads - 1) / kLMThreads,
-                                                            (int64_t)ctx->n_sm * per_sm);
+        const int teams = threads / (32 * wpc);
+        // small batches spread over the SMs before they fill one
+        const unsigned blocks = (unsigned)std::min<int64_t>(n_cut, (int64_t)ctx->n_sm);
+        const int stage_bytes = lm_stage_bytes(ctx, node_bytes, teams);
+        const size_t smem_bytes = node_bytes + (size_t)teams * stage_bytes;
         KernelScope ks_(ctx, "k_lm", bytes);
-#define CPB_LM_LAUNCH_W(TI, NP, NF, W)                                                                             \
-    do {                                                                                                          \
-        if (smem) {                                                                                               \
-            check(cudaFuncSetAttribute(k_lm_t<TI, NP, NF, true, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
-                                       (int)node_bytes),                                                         \
-                  "smem attribute");                                                                             \
-            k_lm_t<TI, NP, NF, true, W><<<blocks, kLMThreads, node_bytes, st>>>(                                  \
-                n_cut, L, N, d_off, d_ny, d_nx, d_y1, d_x1, (const TI*)d_pix, (const TI*)d_iv, d_init, o, queue); \
-        } else {                                                                                                  \
-            k_lm_t<TI, NP, NF, false, W><<<blocks, kLMThreads, 0, st>>>(                                          \
-                n_cut, L, N, d_off, d_ny, d_nx, d_y1, d_x1, (const TI*)d_pix, (const TI*)d_iv, d_init, o, queue); \
-        }                                                                                                         \
+        auto go = [&](auto ti, auto kern) {
+            using TI = decltype(ti);
+            check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes),
+                  "smem attribute");
+            kern<<<blocks, threads, smem_bytes, st>>>(n_cut, L, N, d_off, d_ny, d_nx, d_y1, d_x1, (const TI*)d_pix,
+                                                      (const TI*)d_iv, d_init, o, queue, stage_bytes);
+        };
+#define CPB_LM_W(TI, NP, NF, SM, ID)                                \
+    do {                                                            \
+        if (wpc == 4) go(TI(0), k_lm_t<TI, NP, NF, SM, 4, ID>);     \
+        else go(TI(0), k_lm_t<TI, NP, NF, SM, 1, ID>);              \
     } while (0)
-#define CPB_LM_LAUNCH(TI, NP, NF)             \
-    do {                                      \
-        if (wpc == 4)                         \
-            CPB_LM_LAUNCH_W(TI, NP, NF, 4);   \
-        else                                  \
-            CPB_LM_LAUNCH_W(TI, NP, NF, 1);   \
+#define CPB_LM_S(TI, NF, ID)                        \
+    do {                                            \
+        if (smem) CPB_LM_W(TI, 4, NF, true, ID);    \
+        else CPB_LM_W(TI, 4, NF, false, ID);        \
     } while (0)
-#define CPB_LM_NF(TI, NP)                          \
-    switch (L.nf) {                                \
-        case 1: CPB_LM_LAUNCH(TI, NP, 1); break;   \
-        case 2: CPB_LM_LAUNCH(TI, NP, 2); break;   \
-        case 3: CPB_LM_LAUNCH(TI, NP, 3); break;   \
-        case 4: CPB_LM_LAUNCH(TI, NP, 4); break;   \
-        default: CPB_LM_LAUNCH(TI, NP, NP); break; \
+#define CPB_LM_NF(TI)                                       \
+    if (gauss) {                                            \
+        switch (L.nf) {                                     \
+            case 1: CPB_LM_W(TI, 5, 1, false, false); break; \
+            case 2: CPB_LM_W(TI, 5, 2, false, false); break; \
+            case 3: CPB_LM_W(TI, 5, 3, false, false); break; \
+            case 4: CPB_LM_W(TI, 5, 4, false, false); break; \
+            default: CPB_LM_W(TI, 5, 5, false, true); break; \
+        }                                                   \
+    } else {                                                \
+        switch (L.nf) {                                     \
+            case 1: CPB_LM_S(TI, 1, false); break;          \
+            case 2: CPB_LM_S(TI, 2, false); break;          \
+            case 3:                                         \
+                if (ident) CPB_LM_S(TI, 3, true);           \
+                else CPB_LM_S(TI, 3, false);                \
+                break;                                      \
+            default: CPB_LM_S(TI, 4, true); break;          \
+        }                                                   \
     }
         if (eltype == CPB_F64) {
-            if (gauss) {
-                CPB_LM_NF(double, 5)
-            } else {
-                CPB_LM_NF(double, 4)
-            }
+            CPB_LM_NF(double)
         } else {
-            if (gauss) {
-                CPB_LM_NF(float, 5)
-            } else {
-                CPB_LM_NF(float, 4)
-            }
+            CPB_LM_NF(float)
         }
 #undef CPB_LM_NF
-#undef CPB_LM_LAUNCH
-#undef CPB_LM_LAUNCH_W
+#undef CPB_LM_S
+#undef CPB_LM_W
         check(cudaGetLastError(), "k_lm");
         return;
     }
@@ -1762,8 +1831,9 @@ void lm_batch_enqueue(cpb_ctx* ctx, LMBatch* b, cudaStream_t st, int blocks_per_
 bool lm_batch_smem_possible(const LMBatch* b) {
     const cpb_psf* psf = b->psf;
     if (psf->dev.kind == CPB_PSF_CIRCULAR_GAUSSIAN || psf->dev.n_nodes != 1) return false;
-    const DevNode& nd = psf->h_nodes[0];
-    return sizeof(double) * (size_t)nd.LPY * nd.LPX * nd.isy * nd.isx <= 100 * 1024;
+    size_t bytes = 0;
+    pp_node(psf, true, bytes);
+    return bytes > 0;
 }
 
 int64_t lm_batch_size(const LMBatch* b) { return b->n_cut; }
@@ -1936,7 +2006,7 @@ bool mp_dag_supported(const cpb_psf* psf, const cpb_lm_params* P) {
     return (gauss || psf->dev.n_nodes == 1) && P->reweight == CPB_LOSS_NONE && P->precision == CPB_PREC_FP64;
 }
 
-int mp_dag_teams(cpb_ctx* ctx) { return ctx->n_sm * 2 * (kLMThreads / (32 * kDagWarps)); }
+int mp_dag_teams(cpb_ctx* ctx) { return ctx->n_sm * (kLMThreads / (32 * kDagWarps)); }
 
 void mp_dag_launch(cpb_ctx* ctx, const cpb_psf* psf, const cpb_lm_params* P, int32_t iv_eltype,
                    const DagArgs& A_in) {
@@ -1945,52 +2015,51 @@ void mp_dag_launch(cpb_ctx* ctx, const cpb_psf* psf, const cpb_lm_params* P, int
     const LMConst L = lm_const(psf, P, A.iv != nullptr);
     cudaStream_t st = ctx->stream;
     const bool gauss = psf->dev.kind == CPB_PSF_CIRCULAR_GAUSSIAN;
-    PPNode N{};
-    if (!gauss) {
-        N.nd = psf->h_nodes[0];
-        N.pp = psf->dev.lpp64 + N.nd.lpoff;
-        N.plane = N.nd.LPY * N.nd.LPX;
-        N.inv_isy = 1.0f / (float)N.nd.isy;
-        N.inv_isx = 1.0f / (float)N.nd.isx;
-    }
-    const size_t node_bytes = gauss ? 0 : sizeof(double) * (size_t)N.plane * N.nd.isy * N.nd.isx;
-    const bool smem = !gauss && node_bytes <= 100 * 1024;
-    const unsigned blocks = (unsigned)(ctx->n_sm * 2);  // persistent: every team resident
+    size_t node_bytes = 0;
+    const PPNode N = pp_node(psf, true, node_bytes);
+    const bool smem = node_bytes > 0, ident = lm_ident(L);
+    const int teams = kLMThreads / (32 * kDagWarps);
+    const int stage_bytes = lm_stage_bytes(ctx, node_bytes, teams);
+    const size_t smem_bytes = node_bytes + (size_t)teams * stage_bytes;
+    const unsigned blocks = (unsigned)ctx->n_sm;  // persistent: every team resident
     KernelScope ks_(ctx, "k_mp_dag", 0.0);
-#define CPB_DAG(TIV, NP, NF)                                                                                    \
-    do {                                                                                                        \
-        if (smem) {                                                                                             \
-            check(cudaFuncSetAttribute(k_mp_dag<TIV, NP, NF, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                       (int)node_bytes),                                                       \
-                  "smem attribute");                                                                           \
-            k_mp_dag<TIV, NP, NF, true><<<blocks, kLMThreads, node_bytes, st>>>(L, N, psf->dev, A);             \
-        } else {                                                                                                \
-            k_mp_dag<TIV, NP, NF, false><<<blocks, kLMThreads, 0, st>>>(L, N, psf->dev, A);                     \
-        }                                                                                                       \
+    auto go = [&](auto kern) {
+        check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes),
+              "smem attribute");
+        kern<<<blocks, kLMThreads, smem_bytes, st>>>(L, N, psf->dev, A, stage_bytes);
+    };
+#define CPB_DAG_S(TIV, NF, ID)                          \
+    do {                                                \
+        if (smem) go(k_mp_dag<TIV, 4, NF, true, ID>);   \
+        else go(k_mp_dag<TIV, 4, NF, false, ID>);       \
     } while (0)
-#define CPB_DAG_NF(TIV, NP)                     \
-    switch (L.nf) {                             \
-        case 1: CPB_DAG(TIV, NP, 1); break;     \
-        case 2: CPB_DAG(TIV, NP, 2); break;     \
-        case 3: CPB_DAG(TIV, NP, 3); break;     \
-        case 4: CPB_DAG(TIV, NP, 4); break;     \
-        default: CPB_DAG(TIV, NP, NP); break;   \
+#define CPB_DAG_NF(TIV)                                     \
+    if (gauss) {                                            \
+        switch (L.nf) {                                     \
+            case 1: go(k_mp_dag<TIV, 5, 1, false, false>); break; \
+            case 2: go(k_mp_dag<TIV, 5, 2, false, false>); break; \
+            case 3: go(k_mp_dag<TIV, 5, 3, false, false>); break; \
+            case 4: go(k_mp_dag<TIV, 5, 4, false, false>); break; \
+            default: go(k_mp_dag<TIV, 5, 5, false, true>); break; \
+        }                                                   \
+    } else {                                                \
+        switch (L.nf) {                                     \
+            case 1: CPB_DAG_S(TIV, 1, false); break;        \
+            case 2: CPB_DAG_S(TIV, 2, false); break;        \
+            case 3:                                         \
+                if (ident) CPB_DAG_S(TIV, 3, true);         \
+                else CPB_DAG_S(TIV, 3, false);              \
+                break;                                      \
+            default: CPB_DAG_S(TIV, 4, true); break;        \
+        }                                                   \
     }
     if (iv_eltype == CPB_F64) {
-        if (gauss) {
-            CPB_DAG_NF(double, 5)
-        } else {
-            CPB_DAG_NF(double, 4)
-        }
+        CPB_DAG_NF(double)
     } else {
-        if (gauss) {
-            CPB_DAG_NF(float, 5)
-        } else {
-            CPB_DAG_NF(float, 4)
-        }
+        CPB_DAG_NF(float)
     }
 #undef CPB_DAG_NF
-#undef CPB_DAG
+#undef CPB_DAG_S
     check(cudaGetLastError(), "k_mp_dag");
 }
 

@@ -539,18 +539,6 @@ __global__ void k_coef(int64_t n_act, FitConst fc, DevPsf P, const double* theta
 // T is the arithmetic / storage type of the stamps (double for the plain
 // form, float for the mixed-precision form); positions and weights are
 // always derived in double and rounded once.
-__device__ __forceinline__ void keys_weights(double t, double w[4], double d[4]) {
-    const double t2 = t * t, t3 = t2 * t;
-    w[0] = -0.5 * t + t2 - 0.5 * t3;
-    w[1] = 1.0 - 2.5 * t2 + 1.5 * t3;
-    w[2] = 0.5 * t + 2.0 * t2 - 1.5 * t3;
-    w[3] = -0.5 * t2 + 0.5 * t3;
-    d[0] = -0.5 + 2.0 * t - 1.5 * t2;
-    d[1] = -5.0 * t + 4.5 * t2;
-    d[2] = 0.5 + 4.0 * t - 4.5 * t2;
-    d[3] = -t + 1.5 * t2;
-}
-
 // One axis of one node at one stamp row or column: clamped sample offsets
 // (times the axis stride), weights, derivative weights, and the in-bounds
 // half of bicubic_interpolate's `_inbound` test.

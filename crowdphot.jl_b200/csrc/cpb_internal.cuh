@@ -236,6 +236,85 @@ __device__ __forceinline__ void keys_weights(double t, double w[4], double d[4])
     d[3] = -t + 1.5 * t2;
 }
 
+struct PPNode {
+    const double* pp;   // this node's samples: row-phase copy 2 (staged in shared memory) or the
+                        // edge-padded polyphase copy (read from global memory) (DevNode)
+    DevNode nd;
+    int plane;          // LPY * LPX
+    int nel;            // doubles of the row-phase copy (0: not staged)
+};
+
+// A single-node star over a box of ny x nx pixels whose first pixel is (y1, x1): the
+// pixels its table reaches, the cubic weights every pixel of it shares (axis_span) and
+// the sample addresses.  SMEM: row-phase copy (the column taps are adjacent), else the
+// polyphase copy (consecutive rows are adjacent, whatever the tap).  Set by a whole warp.
+template <bool SMEM>
+struct NodeStar {
+    AxisSpan sy, sx;
+    double wx[4], dx[4], wy[4], dy[4];
+    int rb[4], cb[4], rs, cs;  // tap (r, c) of box pixel (i, j): rb[r] + cb[c] + i * rs + j * cs
+
+    __device__ __forceinline__ void set(const PPNode& N, double Y, double X, int y1, int x1, int ny, int nx) {
+        const DevNode& nd = N.nd;
+        sy = axis_span(nd.sy, Y, nd.oy, nd.ny, y1, ny);
+        sx = axis_span(nd.sx, X, nd.ox, nd.nx, x1, nx);
+        keys_weights(sy.f, wy, dy);
+        keys_weights(sx.f, wx, dx);
+        int q = sy.l0 - 1, e = q / nd.isy, ph = q - e * nd.isy;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            rb[r] = SMEM ? (ph * nd.RPY[2] + e - sy.lo) * nd.RPX + sx.l0 - 1 - nd.isx * sx.lo : ph * N.plane + e - sy.lo;
+            if (++ph == nd.isy) {
+                ph = 0;
+                ++e;
+            }
+        }
+        rs = SMEM ? nd.RPX : 1;
+        cs = SMEM ? nd.isx : nd.LPY;
+        q = sx.l0 - 1;
+        e = q / nd.isx;
+        ph = q - e * nd.isx;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            cb[c] = SMEM ? c : ph * nd.isy * N.plane + (e - sx.lo) * nd.LPY;
+            if (++ph == nd.isx) {
+                ph = 0;
+                ++e;
+            }
+        }
+    }
+    // the four interpolated rows (and their column derivatives) of in-table pixel (i, j)
+    template <bool GRAD>
+    __device__ __forceinline__ void rows(const double* pp, int i, int j, double (&rv)[4], double (&rd)[4]) const {
+        const double* at = pp + (i * rs + j * cs);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const double* q = at + rb[r];
+            const double a = q[SMEM ? 0 : cb[0]], b = q[SMEM ? 1 : cb[1]], c = q[SMEM ? 2 : cb[2]],
+                         e = q[SMEM ? 3 : cb[3]];
+            rv[r] = wx[0] * a + wx[1] * b + wx[2] * c + wx[3] * e;
+            if (GRAD) rd[r] = dx[0] * a + dx[1] * b + dx[2] * c + dx[3] * e;
+        }
+    }
+    __device__ __forceinline__ double value(const PPNode& N, const double* pp, int i, int j) const {
+        if (i < sy.lo || i > sy.hi || j < sx.lo || j > sx.hi) return N.nd.fill;
+        double rv[4], rd[4];
+        rows<false>(pp, i, j, rv, rd);
+        return wy[0] * rv[0] + wy[1] * rv[1] + wy[2] * rv[2] + wy[3] * rv[3];
+    }
+};
+
+// A single-node star's unit profile over a box from the PSF's polyphase copy (the
+// diagnostics' stamps); false for other PSFs.
+__device__ __forceinline__ bool node_of(const DevPsf& P, PPNode& N) {
+    if (P.kind == CPB_PSF_CIRCULAR_GAUSSIAN || P.n_nodes != 1) return false;
+    N.nd = P.nodes[0];
+    N.plane = N.nd.LPY * N.nd.LPX;
+    N.nel = 0;
+    N.pp = P.lpp64 + N.nd.lpoff;
+    return true;
+}
+
 template <typename D>
 __device__ __forceinline__ const D* node_data(const DevPsf& P);
 template <>
@@ -504,22 +583,122 @@ __device__ __forceinline__ double spread_ypass(const SpreadDev& D, const double*
     return g;
 }
 
-// Threads of a diagnostics block (one block a star) and its shared memory when
-// spread_model is on.  Mode 1 (the usual): the model stamp, six x-pass planes
-// and the profiles, (7 boxmax + 6 (2 kh + 1)) doubles; mode 2 (large boxes):
-// the model stamp, one x-pass plane and the correlated stamp, one component at
-// a time, 3 boxmax doubles.  Boxes beyond both within 200 KB (fit_rad above
-// ~45 px) leave spread_model NaN (mode 0).
-constexpr int kDiagThreads = 256;
-inline size_t spread_smem_bytes(int mode, int boxmax, int kh) {
-    return mode == 1 ? ((size_t)7 * boxmax + 6 * (2 * (size_t)kh + 1)) * sizeof(double)
-                     : (mode == 2 ? (size_t)3 * boxmax * sizeof(double) : 0);
+// One line of a component's correlation, by one thread: dst[k] = sum_q I(q) src[k + q]
+// over the line's n values, q ascending from -L to L.  The line lives in registers and
+// every index is fixed at compile time, so a tap is one multiply-add and one profile
+// value (the same address for the whole warp) serves half the line.
+constexpr int kLine = 28, kLineL = 13;
+// MODE 0 stores the line, 1 stores alpha times it, 2 adds alpha times it.
+template <int MODE>
+__device__ __forceinline__ void spread_line(const double* I, int L, const double* src, int sstride, int n, double* dst,
+                                            int dstride, double alpha = 1.0) {
+    double m[kLine];
+#pragma unroll
+    for (int k = 0; k < kLine; ++k) m[k] = k < n ? src[k * sstride] : 0.0;
+#pragma unroll
+    for (int k0 = 0; k0 < kLine; k0 += kLine / 2) {
+        if (k0 >= n) break;
+        double t[kLine / 2];
+#pragma unroll
+        for (int j = 0; j < kLine / 2; ++j) t[j] = 0.0;
+#pragma unroll
+        for (int q = -kLineL; q <= kLineL; ++q) {
+            if (q < -L || q > L) continue;
+            const double iq = I[q];
+#pragma unroll
+            for (int j = 0; j < kLine / 2; ++j)
+                if (k0 + j + q >= 0 && k0 + j + q < kLine) t[j] += iq * m[k0 + j + q];
+        }
+#pragma unroll
+        for (int j = 0; j < kLine / 2; ++j)
+            if (k0 + j < n) {
+                double& d = dst[(k0 + j) * dstride];
+                d = MODE == 0 ? t[j] : (MODE == 1 ? 0.0 : d) + alpha * t[j];
+            }
+    }
 }
-inline int spread_mode(int boxmax, int kh) {
+// The disk-correlated stamp G[r + col * ldh] of the bh x bw stamp M (bh, bw <= kLine) by
+// one warp, component by component in order: its lanes the rows into the scratch plane
+// X, then the columns into G (ldh odd).  Bound by the FP64 pipe (2 (2 L + 1)
+// multiply-adds a pixel and component); the general passes load each value and profile
+// entry again for every tap.
+__device__ __forceinline__ void spread_lines_warp(const SpreadDev& D, const double* Is, const double* M, double* X,
+                                                  double* G, int ldh, int bh, int bw) {
+    const int lane = threadIdx.x & 31, n = 2 * D.kh + 1;
+#pragma unroll 1
+    for (int c = 0; c < 6; ++c) {
+        int L = 0;
+        double alpha = 0.0;
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+            L = q == c ? D.L[q] : L;
+            alpha = q == c ? D.alpha[q] : alpha;
+        }
+        const double* I = Is + c * n + D.kh;
+        __syncwarp();
+        if (lane < bh) spread_line<0>(I, L, M + lane, bh, bw, X + lane, ldh);
+        __syncwarp();
+        if (lane < bw) {
+            if (c == 0) spread_line<1>(I, L, X + lane * ldh, 1, bh, G + lane * ldh, 1, alpha);
+            else spread_line<2>(I, L, X + lane * ldh, 1, bh, G + lane * ldh, 1, alpha);
+        }
+    }
+    __syncwarp();
+}
+
+// Who works a star's diagnostics and its shared memory when spread_model is on.  Mode 3
+// (boxes up to kLine px, fit radii up to 13): a warp a star with the model stamp and two
+// planes of odd column stride (spread_plane doubles each), kDiagWarps stars a block
+// sharing the profiles; the other modes a block a star: mode 1 (larger boxes) the model
+// stamp, six x-pass planes and the profiles, (7 boxmax + 6 (2 kh + 1)) doubles; mode 2
+// (the largest) the model stamp, one x-pass plane and the correlated stamp, one
+// component at a time, 3 boxmax doubles.  Boxes beyond 200 KB of these (fit_rad above
+// ~45 px) leave spread_model NaN (mode 0).
+// The correlation is FP64 multiply-adds; a block a star spends its time on loading
+// profile and stamp values for each and on barriers.  Measured on the B200, block then
+// warp form: k_diag 4.43 and 2.37 ms on a 50,000-star catalogue of 25 px boxes, 107 and
+// 62 us on 1,400 stars of 19 px; k_mp_diag 1.07 and 0.65 ms on 12,500 of 25 px.  A warp's
+// star takes about twice as long as a block's, so with few stars the block form is the
+// faster (200 stars: 22 us against 48): the line lies at kDiagFew stars an SM, two waves
+// of the block form's two blocks an SM.
+constexpr int kDiagThreads = 256;
+constexpr int kDiagWarps = 4;
+constexpr int kDiagFew = 4;
+inline int spread_threads(int mode) { return mode == 3 ? 32 * kDiagWarps : kDiagThreads; }
+__host__ __device__ inline int spread_plane(int boxmax, int kh) { return boxmax + 2 * kh + 2; }
+inline size_t spread_smem_bytes(int mode, int boxmax, int kh) {
+    const size_t prof = 6 * (2 * (size_t)kh + 1);
+    return mode == 3   ? (kDiagWarps * ((size_t)boxmax + 2 * (size_t)spread_plane(boxmax, kh)) + prof) * sizeof(double)
+           : mode == 1 ? ((size_t)7 * boxmax + prof) * sizeof(double)
+                       : (mode == 2 ? (size_t)3 * boxmax * sizeof(double) : 0);
+}
+inline int spread_mode(int boxmax, int kh, int64_t n_stars, int n_sm) {
+    if (2 * kh + 2 <= kLine && kh <= kLineL && n_stars > (int64_t)kDiagFew * n_sm) return 3;
     if (spread_smem_bytes(1, boxmax, kh) <= 200 * 1024) return 1;
     if (spread_smem_bytes(2, boxmax, kh) <= 200 * 1024) return 2;
     return 0;
 }
+
+// The threads of one star's diagnostics: a warp (WARP) or the block.
+template <bool WARP>
+struct DiagTeam {
+    static __device__ __forceinline__ int t0() { return WARP ? threadIdx.x & 31 : threadIdx.x; }
+    static __device__ __forceinline__ int ts() { return WARP ? 32 : blockDim.x; }
+    static __device__ __forceinline__ void sync() {
+        if (WARP) __syncwarp();
+        else __syncthreads();
+    }
+    // sums in thread t0() == 0; sh: K * (blockDim.x / 32) doubles (block form)
+    template <int K>
+    static __device__ __forceinline__ void sum(double (&v)[K], double* sh) {
+        if (WARP) {
+#pragma unroll
+            for (int k = 0; k < K; ++k) v[k] = warp_sum(v[k]);
+        } else {
+            block_sum_n<K>(v, sh);
+        }
+    }
+};
 
 // A spread_model disk built on the device, for fits whose disk width depends on
 // a fitted position (the simultaneous fit sizes it from the first catalogue

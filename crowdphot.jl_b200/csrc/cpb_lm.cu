@@ -703,12 +703,15 @@ __global__ void __launch_bounds__(256) k_lm_irls(int64_t n_cut, LMConst L, DevPs
 
 // ---------------------------------------------------------------------------
 // Fast form: compile-time parameter counts (every small matrix in registers),
-// single-node image PSFs read through the edge-padded polyphase copy (the 16
-// stencil taps of the 32 lanes' pixels -- consecutive cutout rows -- are
-// adjacent doubles, staged in shared memory), only the cutout rectangle that
-// can reach the ePSF grid evaluated in full, and a device work queue over the
-// cutouts.  Arithmetic per pixel is corner_eval's (psf_fitting.jl:1233-1321
-// restated); only the order of the per-lane sums differs.
+// single-node image PSFs through the star's constant cubic weights (NodeStar) and an
+// edge-padded copy of the node, in shared memory where it fits; only the cutout
+// rectangle that can reach the ePSF grid is evaluated in full; the cutout's pixels and
+// weights are staged in shared memory while they fit; a device work queue over the
+// cutouts.  Per pixel the sums are psf_fitting.jl:1233-1321's, with the weights taken
+// out of the pixel loop.  What bounds it: FP64 operations and their latency (16 warps an
+// SM).  100,000 cutouts of 9-41 px, Float32 pixels, measured on the B200: 8.0 ms when
+// every pixel worked its own weights out and read the cutout again each iteration,
+// 4.0 ms now.
 // ---------------------------------------------------------------------------
 // Cholesky factor of A (upper triangle U, reciprocal diagonal Ri: one division per
 // row instead of one per use); false unless positive definite.
@@ -757,74 +760,6 @@ __device__ __forceinline__ double pick(const double* v, int idx) {
     for (int q = 0; q < N; ++q) r = (q == idx) ? v[q] : r;
     return r;
 }
-
-struct PPNode {
-    const double* pp;   // this node's samples: row-phase copy 2 (staged in shared memory) or the
-                        // edge-padded polyphase copy (read from global memory) (DevNode)
-    DevNode nd;
-    int plane;          // LPY * LPX
-    int nel;            // doubles of the row-phase copy (0: not staged)
-};
-
-// A single-node star over a box of ny x nx pixels whose first pixel is (y1, x1): the
-// pixels its table reaches, the cubic weights every pixel of it shares (axis_span) and
-// the sample addresses.  SMEM: row-phase copy (the column taps are adjacent), else the
-// polyphase copy (consecutive rows are adjacent, whatever the tap).  Set by a whole warp.
-template <bool SMEM>
-struct NodeStar {
-    AxisSpan sy, sx;
-    double wx[4], dx[4], wy[4], dy[4];
-    int rb[4], cb[4], rs, cs;  // tap (r, c) of box pixel (i, j): rb[r] + cb[c] + i * rs + j * cs
-
-    __device__ __forceinline__ void set(const PPNode& N, double Y, double X, int y1, int x1, int ny, int nx) {
-        const DevNode& nd = N.nd;
-        sy = axis_span(nd.sy, Y, nd.oy, nd.ny, y1, ny);
-        sx = axis_span(nd.sx, X, nd.ox, nd.nx, x1, nx);
-        keys_weights(sy.f, wy, dy);
-        keys_weights(sx.f, wx, dx);
-        int q = sy.l0 - 1, e = q / nd.isy, ph = q - e * nd.isy;
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            rb[r] = SMEM ? (ph * nd.RPY[2] + e - sy.lo) * nd.RPX + sx.l0 - 1 - nd.isx * sx.lo : ph * N.plane + e - sy.lo;
-            if (++ph == nd.isy) {
-                ph = 0;
-                ++e;
-            }
-        }
-        rs = SMEM ? nd.RPX : 1;
-        cs = SMEM ? nd.isx : nd.LPY;
-        q = sx.l0 - 1;
-        e = q / nd.isx;
-        ph = q - e * nd.isx;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            cb[c] = SMEM ? c : ph * nd.isy * N.plane + (e - sx.lo) * nd.LPY;
-            if (++ph == nd.isx) {
-                ph = 0;
-                ++e;
-            }
-        }
-    }
-    // the four interpolated rows (and their column derivatives) of in-table pixel (i, j)
-    template <bool GRAD>
-    __device__ __forceinline__ void rows(const double* pp, int i, int j, double (&rv)[4], double (&rd)[4]) const {
-        const double* at = pp + (i * rs + j * cs);
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const double* q = at + rb[r];
-            const double a = q[SMEM ? 0 : cb[0]], b = q[SMEM ? 1 : cb[1]], c = q[SMEM ? 2 : cb[2]],
-                         e = q[SMEM ? 3 : cb[3]];
-            rv[r] = wx[0] * a + wx[1] * b + wx[2] * c + wx[3] * e;
-            if (GRAD) rd[r] = dx[0] * a + dx[1] * b + dx[2] * c + dx[3] * e;
-        }
-    }
-    __device__ __forceinline__ double value(const PPNode& N, const double* pp, int i, int j) const {
-        if (i < sy.lo || i > sy.hi || j < sx.lo || j > sx.hi) return N.nd.fill;
-        double rv[4], rd[4];
-        rows<false>(pp, i, j, rv, rd);
-        return wy[0] * rv[0] + wy[1] * rv[1] + wy[2] * rv[2] + wy[3] * rv[3];
-    }
-};
 
 // A cutout is fitted by a team of WPC warps (1: one warp a cutout, the
 // throughput form for large batches; 4: a 128-thread team, the latency form for
@@ -1244,6 +1179,7 @@ __device__ __forceinline__ bool lm_step(LMState<NP, NF>& S, const LMConst& L, do
 // Threads of a block, one block an SM (128 registers a thread): one staged node serves
 // every team and the rest of the shared memory holds the teams' cutouts.
 constexpr int kLMThreads = 512;
+static_assert(kLMThreads % 256 == 0, "half a block must still hold whole 128-thread teams");
 
 // fit_star of one cutout by a team (pixels pix / weights iv, column-major
 // ny x nx whose first pixel is image pixel (y1, x1); init: the NP model
@@ -1402,8 +1338,11 @@ __global__ void __launch_bounds__(kLMThreads, 1) k_lm_t(int64_t n_cut, LMConst L
 // fit only holds back the stars that overlap it.  The residual image is read
 // and written around L1 (ld/st.cg): other SMs change it between uses.
 constexpr long long kDagSpinLimit = 1ll << 26;  // default: ~64 M polls of >= 64 ns before a team gives up
-// Warps of one team: 4 measured fastest on the 2048^2 field (k_mp_dag 34.6 ms for
-// three passes, against 58.2 ms with 1 and 41.0 ms with 8).
+// Warps of one team: 4 measured fastest on a 2048^2 field when each pixel worked its own
+// weights out (34.6 ms for three passes, against 58.2 ms with 1 and 41.0 ms with 8).
+// With the star's weights, staged cutouts and fewer divisions in the serial steps, three
+// passes over 12,500 stars of a 1024^2 field take 8.4 ms, from 12.9 (bound by the chain
+// of overlapping stars, one fit's latency a link).
 constexpr int kDagWarps = 4;
 
 template <typename TIV, int NP, int NF, bool SMEM, bool ID>
@@ -1608,7 +1547,8 @@ LMConst lm_const(const cpb_psf* psf, const cpb_lm_params* P, bool have_iv) {
 }
 
 // The node as the fast forms read it: the row-phase copy for staging in shared memory
-// when two copies fit an SM, else the polyphase copy in global memory.
+// up to 100 KB (the rest holds the teams' cutouts), else the polyphase copy in global
+// memory.
 PPNode pp_node(const cpb_psf* psf, bool staged_wanted, size_t& smem_bytes) {
     PPNode N{};
     smem_bytes = 0;
@@ -1688,9 +1628,7 @@ void launch_lm(cpb_ctx* ctx, const cpb_psf* psf, const LMConst& L, int64_t n_cut
         auto* queue = cfg.queue ? cfg.queue
                                 : (unsigned long long*)scratch(ctx, "lm_queue", sizeof(unsigned long long));
         if (!(cfg.queue && cfg.queue_zeroed)) check(cudaMemsetAsync(queue, 0, sizeof(unsigned long long), st), "memset");
-        // two persistent 256-thread blocks an SM (128 registers a thread); the
-        // node's samples go to shared memory when two copies fit an SM
-        // one block an SM, of half the threads with cfg.blocks_per_sm == 1
+        // one persistent block an SM, of half the threads with cfg.blocks_per_sm == 1
         const int threads = cfg.blocks_per_sm == 1 ? kLMThreads / 2 : kLMThreads;
         // one warp a cutout while the batch fills the GPU's warps; a batch too
         // small for that (the late batches of fit_all_stars) gets 128-thread

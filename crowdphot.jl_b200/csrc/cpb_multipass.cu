@@ -60,14 +60,15 @@ __global__ void k_mp_addcut(int nL, const int4* __restrict__ boxes, const double
 // box: image is the original data, residual the star's fit residual (every
 // model subtracted, its own included), star_model its best-fit render, kept in
 // shared memory with its disk-correlated copy for spread_model (D.I null:
-// spread_model off).  One block of kDiagThreads a star (grid-stride).  out:
+// spread_model off).  A warp (WARP) or a block of kDiagThreads a star
+// (spread_mode; grid-stride).  out:
 // qfit, qfit_expected, qfit_z, crowding, spread_model, spread_model_err per
 // star (NaN where undefined).  snap (nullable): the star's residual box saved
 // right after its subtraction (snap_off per position), used in place of the
 // residual image when the diagnostics run after the whole pass.
-template <typename TI>
-__global__ void __launch_bounds__(kDiagThreads, 3) k_mp_diag(int nL, const int4* __restrict__ boxes,
-                                                         const double* __restrict__ params,
+template <typename TI, bool WARP>
+__global__ void __launch_bounds__(WARP ? 32 * kDiagWarps : kDiagThreads, WARP ? 4 : 2) 
+    k_mp_diag(int nL, const int4* __restrict__ boxes,    const double* __restrict__ params,
                                                          const uint8_t* __restrict__ flags,
                                                          const TI* __restrict__ img,
                                                          const double* __restrict__ residual,
@@ -76,31 +77,53 @@ __global__ void __launch_bounds__(kDiagThreads, 3) k_mp_diag(int nL, const int4*
                                                          const TI* __restrict__ iv, DevPsf P, MPConst M, int n_free,
                                                          int ny, SpreadDev D, int smode, int boxmax,
                                                          const int32_t* __restrict__ idx, double* __restrict__ out) {
-    extern __shared__ double stamp[];  // model stamp, x-pass scratch, disk-correlated stamp
+    extern __shared__ double diag_smem[];
     __shared__ double red[12 * (kDiagThreads / 32)];
     const double NaN = __longlong_as_double(0x7ff8000000000000LL);
+    using T = DiagTeam<WARP>;
+    const int t0 = T::t0(), ts = T::ts(), unit = WARP ? threadIdx.x >> 5 : 0, nunit = WARP ? kDiagWarps : 1;
     const int mode = D.I ? smode : 0;
-    double* Is = stamp + 7 * boxmax;  // mode 1: the six profiles
-    if (mode == 1)
-        for (int i = threadIdx.x; i < 6 * (2 * D.kh + 1); i += blockDim.x) Is[i] = D.I[i];
-    for (int s = blockIdx.x; s < nL; s += gridDim.x) {
-        __syncthreads();  // the previous star's stamps are no longer read
+    // the star's stamp and planes, and the six profiles behind them all
+    const int ld = WARP ? spread_plane(boxmax, D.kh) : boxmax;
+    double* stamp = diag_smem + (WARP ? unit * (boxmax + 2 * ld) : 0);
+    double* Ts = stamp + boxmax;
+    double* Is = diag_smem + (WARP ? kDiagWarps * (boxmax + 2 * ld) : 7 * boxmax);
+    if (WARP || mode == 1)
+        for (int i = threadIdx.x; i < 6 * (2 * D.kh + 1); i += blockDim.x) Is[i] = D.I ? D.I[i] : 0.0;
+    __syncthreads();
+    PPNode N;
+    const bool one_node = node_of(P, N);
+    for (int s = blockIdx.x * nunit + unit; s < nL; s += gridDim.x * nunit) {
+        T::sync();  // the previous star's stamps are no longer read
         double* o = out + (int64_t)idx[s] * 6;  // star order
         const double* pr = params + (int64_t)s * M.np;
         const double flux = pr[M.rf], bkg = pr[M.rb];
         if (flags[s] != 2 || !(flux > 0)) {  // 2: fitted in this batch
-            if (threadIdx.x == 0) o[0] = o[1] = o[2] = o[3] = o[4] = o[5] = NaN;
+            if (t0 == 0) o[0] = o[1] = o[2] = o[3] = o[4] = o[5] = NaN;
             continue;
         }
         const int4 b = boxes[s];
         const int nb = b.z * b.w;
-        const bool spread = mode != 0 && nb <= boxmax;
-        double* G = stamp + 2 * boxmax;  // mode 2: the correlated stamp
+        const float inv_h = 1.0f / (float)max(b.z, 1);
+        auto col_of = [&](int e) { return WARP ? (int)(((float)e + 0.5f) * inv_h) : e / b.z; };  // exact below 2^22
+        const bool spread = mode != 0 && nb <= boxmax && (!WARP || (b.z <= kLine && b.w <= kLine));
+        double* G = WARP ? Ts + ld : stamp + 2 * boxmax;  // the correlated stamp (not mode 1)
         if (spread) {
-            for (int e = threadIdx.x; e < nb; e += blockDim.x) stamp[e] = mp_model(P, M, pr, b.x + e % b.z, b.y + e / b.z);
-            __syncthreads();
-            if (mode == 1) {
-                spread_xpass_all(D, Is, stamp, stamp + boxmax, boxmax, b.z, b.w);
+            if (one_node) {
+                NodeStar<false> S;
+                S.set(N, pr[M.ry], pr[M.rx], b.x, b.y, b.z, b.w);
+                for (int e = t0; e < nb; e += ts) {
+                    const int col = col_of(e);
+                    stamp[e] = flux * S.value(N, N.pp, e - col * b.z, col) + bkg;
+                }
+            } else {
+                for (int e = t0; e < nb; e += ts) stamp[e] = mp_model(P, M, pr, b.x + e % b.z, b.y + e / b.z);
+            }
+            T::sync();
+            if (WARP) {
+                spread_lines_warp(D, Is, stamp, Ts, G, b.z | 1, b.z, b.w);
+            } else if (mode == 1) {
+                spread_xpass_all(D, Is, stamp, Ts, boxmax, b.z, b.w);
                 __syncthreads();
             } else {
                 spread_stamp_block(D, stamp, stamp + boxmax, G, b.z, b.w);
@@ -109,8 +132,9 @@ __global__ void __launch_bounds__(kDiagThreads, 3) k_mp_diag(int nL, const int4*
         const double inv_flux = 1.0 / flux;
         // qv ncl ndi den ss ss2 Sp Sq Sp0 Sq0 SqG ngood
         double v[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-        for (int e = threadIdx.x; e < nb; e += blockDim.x) {
-            const int i = b.x + e % b.z, j = b.y + e / b.z;
+        for (int e = t0; e < nb; e += ts) {
+            const int cc = col_of(e);
+            const int i = b.x + e - cc * b.z, j = b.y + cc;
             const int64_t q = (i - 1) + (int64_t)(j - 1) * ny;
             const double wp = iv ? (double)iv[q] : 1.0;
             if (isfinite(wp) && wp > 0) {
@@ -124,7 +148,9 @@ __global__ void __launch_bounds__(kDiagThreads, 3) k_mp_diag(int nL, const int4*
                 v[2] += wP * ((double)img[q] - bkg);
                 v[3] += wP * Pp;
                 if (spread) {
-                    const double gm = mode == 1 ? spread_ypass(D, Is, stamp + boxmax, boxmax, b.z, e) : G[e];
+                    const double gm = WARP        ? G[e + cc * ((b.z | 1) - b.z)]
+                                      : mode == 1 ? spread_ypass(D, Is, Ts, boxmax, b.z, e)
+                                                  : G[e];
                     const double g_i = (gm - bkg) * inv_flux;
                     v[6] += wP * p_i;
                     v[7] += wp * g_i * p_i;
@@ -143,8 +169,8 @@ __global__ void __launch_bounds__(kDiagThreads, 3) k_mp_diag(int nL, const int4*
                 }
             }
         }
-        block_sum_n<12>(v, red);
-        if (threadIdx.x == 0) {
+        T::sum(v, red);
+        if (t0 == 0) {
             const double qv = v[0], ncl = v[1], ndi = v[2], den = v[3], ss = v[4], ss2 = v[5];
             const double Sp = v[6], Sq = v[7], Sp0 = v[8], Sq0 = v[9], SqG = v[10];
             const int ngood = (int)v[11];
@@ -618,7 +644,7 @@ int fit_all_stars_dev(cpb_ctx* ctx, const cpb_psf* psf, const cpb_lm_params* P, 
     const int boxmax = (int)box_max;
     int smode = 0;
     if (spread_kernel(psf, psf->dev.fwhm, spread_model_fwhm, init[0], init[1], fit_rad, sh) &&
-        (smode = spread_mode(boxmax, sh.kh)) != 0) {
+        (smode = spread_mode(boxmax, sh.kh, n, ctx->n_sm)) != 0) {
         double* d_I = (double*)scratch(ctx, "mp_spread_I", sizeof(double) * sh.I.size());
         check(cudaMemcpyAsync(d_I, sh.I.data(), sizeof(double) * sh.I.size(), cudaMemcpyHostToDevice, st), "h2d");
         sd.I = d_I;
@@ -626,12 +652,12 @@ int fit_all_stars_dev(cpb_ctx* ctx, const cpb_psf* psf, const cpb_lm_params* P, 
         for (int c = 0; c < 6; ++c) sd.alpha[c] = sh.alpha[c], sd.L[c] = sh.L[c];
     }
     const size_t diag_smem = spread_smem_bytes(smode, boxmax, sd.kh);
-    if (diag_smem > 48 * 1024) {
-        check(cudaFuncSetAttribute(k_mp_diag<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)diag_smem),
-              "smem attr");
-        check(cudaFuncSetAttribute(k_mp_diag<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)diag_smem),
-              "smem attr");
-    }
+    auto diag_attr = [&](auto kern) {
+        if (diag_smem > 48 * 1024)
+            check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)diag_smem), "smem attr");
+    };
+    if (smode == 3) diag_attr(k_mp_diag<double, true>), diag_attr(k_mp_diag<float, true>);
+    else diag_attr(k_mp_diag<double, false>), diag_attr(k_mp_diag<float, false>);
     const unsigned gs = (unsigned)((n + 255) / 256);
     std::vector<int32_t> lev_start;
     std::vector<int64_t> lev_pix;
@@ -741,14 +767,19 @@ int fit_all_stars_dev(cpb_ctx* ctx, const cpb_psf* psf, const cpb_lm_params* P, 
                 if (pass == n_passes) {  // diagnostics of the fitted stars (:381-389), from the snapshots
                     KernelScope ks_(ctx, "k_mp_diag", (double)tot_all * (d_iv ? 24 : 16));
                     const unsigned g = (unsigned)std::min<int64_t>(npos, (int64_t)ctx->n_sm * 16);
-                    if (eltype == CPB_F64)
-                        k_mp_diag<double><<<g, kDiagThreads, diag_smem, st>>>(
-                            npos, d_box, d_psub, d_flag, (const double*)d_img, resid, d_snap, d_scan,
-                            (const double*)d_iv, dp, M, nf, ny, sd, smode, boxmax, d_order, d_diagS);
-                    else
-                        k_mp_diag<float><<<g, kDiagThreads, diag_smem, st>>>(
-                            npos, d_box, d_psub, d_flag, (const float*)d_img, resid, d_snap, d_scan,
-                            (const float*)d_iv, dp, M, nf, ny, sd, smode, boxmax, d_order, d_diagS);
+                    auto go = [&](auto kern, auto ti) {
+                        using TI = decltype(ti);
+                        kern<<<g, spread_threads(smode), diag_smem, st>>>(
+                            npos, d_box, d_psub, d_flag, (const TI*)d_img, resid, d_snap, d_scan,
+                            (const TI*)d_iv, dp, M, nf, ny, sd, smode, boxmax, d_order, d_diagS);
+                    };
+                    if (eltype == CPB_F64) {
+                        if (smode == 3) go(k_mp_diag<double, true>, 0.0);
+                        else go(k_mp_diag<double, false>, 0.0);
+                    } else {
+                        if (smode == 3) go(k_mp_diag<float, true>, 0.0f);
+                        else go(k_mp_diag<float, false>, 0.0f);
+                    }
                     check(cudaGetLastError(), "k_mp_diag");
                 }
                 int32_t dc[4] = {0, 0, 0, 0};
@@ -858,14 +889,19 @@ int fit_all_stars_dev(cpb_ctx* ctx, const cpb_psf* psf, const cpb_lm_params* P, 
             if (pass == n_passes) {  // diagnostics of the fitted stars (:381-389)
                 KernelScope ks_(ctx, "k_mp_diag", (double)tot * (d_iv ? 24 : 16));
                 const unsigned g = (unsigned)std::min<int64_t>(nL, (int64_t)ctx->n_sm * 16);
-                if (eltype == CPB_F64)
-                    k_mp_diag<double><<<g, kDiagThreads, diag_smem, st>>>(
-                        nL, bx, d_psub + p0 * np, d_flag + p0, (const double*)d_img, resid, nullptr, nullptr,
-                        (const double*)d_iv, dp, M, nf, ny, sd, smode, boxmax, d_idx + p0, d_diagS);
-                else
-                    k_mp_diag<float><<<g, kDiagThreads, diag_smem, st>>>(
-                        nL, bx, d_psub + p0 * np, d_flag + p0, (const float*)d_img, resid, nullptr, nullptr,
-                        (const float*)d_iv, dp, M, nf, ny, sd, smode, boxmax, d_idx + p0, d_diagS);
+                auto go = [&](auto kern, auto ti) {
+                    using TI = decltype(ti);
+                    kern<<<g, spread_threads(smode), diag_smem, st>>>(
+                        nL, bx, d_psub + p0 * np, d_flag + p0, (const TI*)d_img, resid, nullptr, nullptr,
+                        (const TI*)d_iv, dp, M, nf, ny, sd, smode, boxmax, d_idx + p0, d_diagS);
+                };
+                if (eltype == CPB_F64) {
+                    if (smode == 3) go(k_mp_diag<double, true>, 0.0);
+                    else go(k_mp_diag<double, false>, 0.0);
+                } else {
+                    if (smode == 3) go(k_mp_diag<float, true>, 0.0f);
+                    else go(k_mp_diag<float, false>, 0.0f);
+                }
                 check(cudaGetLastError(), "k_mp_diag");
             }
         }

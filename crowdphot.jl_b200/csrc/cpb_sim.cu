@@ -2098,37 +2098,47 @@ __global__ void __launch_bounds__(256) k_spread_disk(DevPsf P, double param, int
 }
 
 // chisq and the qfit / crowding / spread_model diagnostics per active star
-// (:1358-1397, psf_photometry_diagnostics.jl:154-231); one block of
-// kDiagThreads a star (grid-stride), the star's model stamp over its box and
-// its disk-correlated copy kept in shared memory.  stab: the disk table
+// (:1358-1397, psf_photometry_diagnostics.jl:154-231); a warp (WARP) or a block
+// of kDiagThreads a star (spread_mode; grid-stride), the star's model stamp over
+// its box and its disk-correlated copy kept in shared memory.  stab: the disk table
 // (spread_disk_block; null or off: spread_model NaN), smode its layout.
-template <typename TI>
-__global__ void __launch_bounds__(kDiagThreads, 3) k_diag(int64_t n_act, FitConst fc, DevPsf P, double fit_rad,
-                                                      const StarCoef* __restrict__ coef,
+template <typename TI, bool WARP>
+__global__ void __launch_bounds__(WARP ? 32 * kDiagWarps : kDiagThreads, WARP ? 4 : 2)
+    k_diag(int64_t n_act, FitConst fc, DevPsf P, double fit_rad,                       const StarCoef* __restrict__ coef,
                                                       const double* __restrict__ resid, const TI* __restrict__ img,
                                                       const TI* __restrict__ bkgimg, const TI* __restrict__ iv,
                                                       const double* __restrict__ stab, int kh, int smode,
                                                       int boxmax,
                                                       double* out /* n_act x 7: chisq qfit qfit_exp qfit_z crowding
                                                                      spread spread_err */) {
-    extern __shared__ double stamp[];  // model stamp, x-pass scratch, disk-correlated stamp
+    extern __shared__ double diag_smem[];
     __shared__ double red[14 * (kDiagThreads / 32)];
-    __shared__ StarCoef c;
+    __shared__ StarCoef cs[WARP ? kDiagWarps : 1];
+    using T = DiagTeam<WARP>;
+    const int t0 = T::t0(), ts = T::ts(), unit = WARP ? threadIdx.x >> 5 : 0, nunit = WARP ? kDiagWarps : 1;
+    StarCoef& c = cs[unit];
     const double NaN = __longlong_as_double(0x7ff8000000000000LL);
     const bool on = stab != nullptr && spread_tab_on(stab);
     const SpreadDev D = on ? spread_dev(stab, kh) : SpreadDev{};
     const int mode = on ? smode : 0;
-    double* Is = stamp + 7 * boxmax;  // mode 1: the six profiles
-    if (mode == 1)
-        for (int i = threadIdx.x; i < 6 * (2 * D.kh + 1); i += blockDim.x) Is[i] = D.I[i];
-    for (int64_t j = blockIdx.x; j < n_act; j += gridDim.x) {
-        __syncthreads();  // the previous star's c and stamps are no longer read
-        if (threadIdx.x == 0) c = coef[j];
-        __syncthreads();
+    // the star's stamp and planes, and the six profiles behind them all
+    const int ld = WARP ? spread_plane(boxmax, kh) : boxmax;
+    double* stamp = diag_smem + (WARP ? unit * (boxmax + 2 * ld) : 0);
+    double* Ts = stamp + boxmax;
+    double* Is = diag_smem + (WARP ? kDiagWarps * (boxmax + 2 * ld) : 7 * boxmax);
+    if (WARP || mode == 1)
+        for (int i = threadIdx.x; i < 6 * (2 * D.kh + 1); i += blockDim.x) Is[i] = on ? D.I[i] : 0.0;
+    __syncthreads();
+    PPNode N;
+    const bool one_node = node_of(P, N);
+    for (int64_t j = (int64_t)blockIdx.x * nunit + unit; j < n_act; j += (int64_t)gridDim.x * nunit) {
+        T::sync();  // the previous star's c and stamps are no longer read
+        if (t0 == 0) c = coef[j];
+        T::sync();
         double* o = out + j * 7;
         const bool validp = isfinite(c.y) && isfinite(c.x) && isfinite(c.flux) && c.flux > 0;
         if (!validp) {
-            if (threadIdx.x == 0) {
+            if (t0 == 0) {
                 o[0] = 0.0;
                 o[1] = o[2] = o[3] = o[4] = o[5] = o[6] = NaN;
             }
@@ -2139,14 +2149,27 @@ __global__ void __launch_bounds__(kDiagThreads, 3) k_diag(int64_t n_act, FitCons
         const int h = max(yhi - ylo + 1, 0), wd = max(xhi - xlo + 1, 0);
         const int nb = h * wd;
         const double inv_flux = 1.0 / c.flux;
-        const bool spread = mode != 0 && nb > 0 && nb <= boxmax;
-        double* G = stamp + 2 * boxmax;  // mode 2: the correlated stamp
+        const float inv_h = 1.0f / (float)max(h, 1);
+        auto col_of = [&](int e) { return WARP ? (int)(((float)e + 0.5f) * inv_h) : e / h; };  // exact below 2^22
+        const bool spread = mode != 0 && nb > 0 && nb <= boxmax && (!WARP || (h <= kLine && wd <= kLine));
+        double* G = WARP ? Ts + ld : stamp + 2 * boxmax;  // the correlated stamp (not mode 1)
         if (spread) {
-            for (int e = threadIdx.x; e < nb; e += blockDim.x)
-                stamp[e] = model_value<double, double>(P, P.data64, c, (double)(ylo + e % h), (double)(xlo + e / h));
-            __syncthreads();
-            if (mode == 1) {
-                spread_xpass_all(D, Is, stamp, stamp + boxmax, boxmax, h, wd);
+            if (one_node) {
+                NodeStar<false> S;
+                S.set(N, c.y, c.x, ylo, xlo, h, wd);
+                for (int e = t0; e < nb; e += ts) {
+                    const int col = col_of(e);
+                    stamp[e] = c.flux * S.value(N, N.pp, e - col * h, col) + c.bkg;
+                }
+            } else {
+                for (int e = t0; e < nb; e += ts)
+                    stamp[e] = model_value<double, double>(P, P.data64, c, (double)(ylo + e % h), (double)(xlo + e / h));
+            }
+            T::sync();
+            if (WARP) {
+                spread_lines_warp(D, Is, stamp, Ts, G, h | 1, h, wd);
+            } else if (mode == 1) {
+                spread_xpass_all(D, Is, stamp, Ts, boxmax, h, wd);
                 __syncthreads();
             } else {
                 spread_stamp_block(D, stamp, stamp + boxmax, G, h, wd);
@@ -2154,25 +2177,36 @@ __global__ void __launch_bounds__(kDiagThreads, 3) k_diag(int64_t n_act, FitCons
         }
         // num qv ncl ndi den ss ss2 Sp Sq Sp0 Sq0 SqG ng ngi
         double v[14] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-        for (int e = threadIdx.x; e < nb; e += blockDim.x) {
-            const int gy = ylo + e % h, gx = xlo + e / h;
-            const int64_t q = (gy - 1) + (int64_t)(gx - 1) * fc.ny;
-            const double r = resid[q];
-            const double wp = iv ? (double)iv[q] : 1.0;
+        // the next pixel's values load behind this one's sums
+        double rn = 0.0, wn = 1.0, imn = 0.0;
+        auto load = [&](int e) {
+            const int col = col_of(e);
+            const int64_t q = (ylo - 1 + e - col * h) + (int64_t)(xlo - 1 + col) * fc.ny;
+            rn = resid[q];
+            if (iv) wn = (double)iv[q];
+            imn = (double)img[q] - (bkgimg ? (double)bkgimg[q] : 0.0);
+        };
+        if (t0 < nb) load(t0);
+        for (int e = t0; e < nb; e += ts) {
+            const double r = rn, wp = wn, im = imn;
+            if (e + ts < nb) load(e + ts);
             if (isfinite(wp) && wp > 0) {
                 v[0] += wp * (r * r);
                 v[12] += 1.0;
-                const double mv = spread ? stamp[e] : model_value<double, double>(P, P.data64, c, (double)gy, (double)gx);
+                const double mv = spread ? stamp[e]
+                                         : model_value<double, double>(P, P.data64, c, (double)(ylo + e % h),
+                                                                       (double)(xlo + e / h));
                 v[1] += fabs(r);
                 const double Pp = (mv - c.bkg) * inv_flux;
                 const double wP = wp * Pp;
                 const double p_i = r + mv - c.bkg;
                 v[2] += wP * p_i;
-                const double im = (double)img[q] - (bkgimg ? (double)bkgimg[q] : 0.0);
                 v[3] += wP * (im - c.bkg);
                 v[4] += wP * Pp;
                 if (spread) {
-                    const double gm = mode == 1 ? spread_ypass(D, Is, stamp + boxmax, boxmax, h, e) : G[e];
+                    const double gm = WARP        ? G[e + col_of(e) * ((h | 1) - h)]
+                                      : mode == 1 ? spread_ypass(D, Is, Ts, boxmax, h, e)
+                                                  : G[e];
                     const double g_i = (gm - c.bkg) * inv_flux;
                     v[7] += wP * p_i;
                     v[8] += wp * g_i * p_i;
@@ -2188,8 +2222,8 @@ __global__ void __launch_bounds__(kDiagThreads, 3) k_diag(int64_t n_act, FitCons
                 }
             }
         }
-        block_sum_n<14>(v, red);
-        if (threadIdx.x == 0) {
+        T::sum(v, red);
+        if (t0 == 0) {
             const double num = v[0], qv = v[1], ncl = v[2], ndi = v[3], den = v[4], ss = v[5], ss2 = v[6];
             const double Sp = v[7], Sq = v[8], Sp0 = v[9], Sq0 = v[10], SqG = v[11];
             const int ng = (int)v[12], ngi = (int)v[13];
@@ -3406,7 +3440,7 @@ void SimFit::finish() {
     int smode = 0;
     double* d_stab = nullptr;
     if (n_stars > 0 && (std::isnan(sp_param) || (std::isfinite(sp_param) && sp_param > 0)) &&
-        (smode = spread_mode(boxmax, kh)) != 0) {
+        (smode = spread_mode(boxmax, kh, n_act, ctx->n_sm)) != 0) {
         double h_rule[kSpreadRuleLen];
         spread_rule(h_rule);
         double* d_rule = S_<double>("spread_rule", kSpreadRuleLen);
@@ -3431,20 +3465,22 @@ void SimFit::finish() {
     {
         KernelScope ks_(ctx, "k_diag",
                         (double)n_act * boxmax * (8.0 + (d_inv_var ? 2.0 : 1.0) * (eltype == CPB_F64 ? 8 : 4)));
+        auto go = [&](auto kern, auto ti) {
+            using TI = decltype(ti);
+            if (diag_smem > 48 * 1024)
+                check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)diag_smem),
+                      "smem attr");
+            kern<<<dgrid, spread_threads(smode), diag_smem, st>>>(n_act, fc, dp, P->fit_rad, coef, resid,
+                                                                  (const TI*)d_image, (const TI*)d_background,
+                                                                  (const TI*)d_inv_var, d_stab, kh, smode, boxmax,
+                                                                  diag);
+        };
         if (eltype == CPB_F64) {
-            if (diag_smem > 48 * 1024)
-                check(cudaFuncSetAttribute(k_diag<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)diag_smem),
-                      "smem attr");
-            k_diag<double><<<dgrid, kDiagThreads, diag_smem, st>>>(n_act, fc, dp, P->fit_rad, coef, resid,
-                                                               (const double*)d_image, (const double*)d_background,
-                                                               (const double*)d_inv_var, d_stab, kh, smode, boxmax, diag);
+            if (smode == 3) go(k_diag<double, true>, 0.0);
+            else go(k_diag<double, false>, 0.0);
         } else {
-            if (diag_smem > 48 * 1024)
-                check(cudaFuncSetAttribute(k_diag<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)diag_smem),
-                      "smem attr");
-            k_diag<float><<<dgrid, kDiagThreads, diag_smem, st>>>(n_act, fc, dp, P->fit_rad, coef, resid,
-                                                              (const float*)d_image, (const float*)d_background,
-                                                              (const float*)d_inv_var, d_stab, kh, smode, boxmax, diag);
+            if (smode == 3) go(k_diag<float, true>, 0.0f);
+            else go(k_diag<float, false>, 0.0f);
         }
         check(cudaGetLastError(), "k_diag");
     }

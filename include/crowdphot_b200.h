@@ -520,8 +520,8 @@ CPB_API int cpb_fit_lm_batch_device(cpb_ctx* ctx, const cpb_psf* psf, const cpb_
  * CPB_TUNE_CACHE environment variable, else no file) and, when absent, times
  * every candidate shape on the bound batch itself (each candidate runs the
  * real fits once; outputs are overwritten), keeps the fastest and records it;
- * 2 re-tunes even when cached.  The shapes are: persistent blocks per SM (1
- * or 2) and whether the ePSF node is staged in shared memory for the fit_star
+ * 2 re-tunes even when cached.  The shapes are: 256-thread
+ * shares of an SM (1 or 2) and whether the ePSF node is staged in shared memory for the fit_star
  * kernel; threads per block (64, 128 or 256) for each launch of the group
  * kernel (groups are launched in buckets of similar star count, each with a
  * shared-memory layout sized for its largest group).  `info` (nullable)

@@ -45,6 +45,7 @@ namespace {
 constexpr double kEpsG = 2.220446049250313e-16;
 constexpr int kMaxGroupStars = 64;
 constexpr int kNoU = 0x7fffffff;
+constexpr uint16_t kNoU16 = 0xffff;  // unusable stamp entry
 
 struct GroupConst {
     int p;
@@ -56,6 +57,8 @@ struct GroupConst {
     int nmax;      // star capacity of the shared-memory layout
     int umax;      // union-pixel capacity
     int keyn;      // power-of-two key buffer for the union sort (>= nmax * S2)
+    int same;      // model radius = fit half-width: one star mask a pixel
+    unsigned Smag; // quot_magic(S)
     int max_iter, max_trials, itmax;
     double linear_tol, max_step, x_tol, f_tol, g_tol;
     double lambda_init, lambda_up, lambda_down, lambda_min, lambda_max;
@@ -93,19 +96,36 @@ struct GroupOut {
     const double* sp_rule;  // kSpreadRuleLen doubles (spread_rule)
 };
 
+// q / d for q < 2^31 without a division: quot_magic(d) = min(floor(2^32 / d), 2^32 - 1),
+// whose product with q is short of 2^32 q / d by less than 2^32, so the high word is the
+// quotient or one below it.
+__host__ __device__ inline unsigned quot_magic(unsigned d) {
+    return d <= 1 ? 0xffffffffu : (unsigned)(0x100000000ull / d);
+}
+__device__ __forceinline__ int quot(int q, int d, unsigned magic, int& rem) {
+    int k = (int)__umulhi((unsigned)q, magic);
+    rem = q - k * d;
+    if (rem >= d) {
+        rem -= d;
+        ++k;
+    }
+    return k;
+}
+
 // Byte offsets of the shared-memory layout (same computation on host and device).
+// node: single-node image PSF (a NodeStar a star).
 struct Layout {
-    size_t coef, coefc, theta, delta, dsc, cn, D, bsc, xl, vt, wl;
+    size_t coef, ns, theta, delta, dsc, cn, D, bsc, xl, vt, wl;
     size_t ay, ax, act, frozen, live, conv, newf;
     size_t V, uidx;
-    size_t dw, w, wr, u, upix, fmask, mmask;
+    size_t dw, sw, wr, u, upix, fmask, mmask;
     size_t total;
 };
 
 __host__ __device__ inline size_t align16(size_t v) { return (v + 15) & ~(size_t)15; }
 
 template <typename MaskT>
-__host__ __device__ inline Layout make_layout(int nmax, int S2, int umax, int keyn) {
+__host__ __device__ inline Layout make_layout(int nmax, int S2, int umax, int keyn, bool node, bool same) {
     Layout L;
     size_t o = 0;
     auto take = [&](size_t bytes) {
@@ -115,7 +135,7 @@ __host__ __device__ inline Layout make_layout(int nmax, int S2, int umax, int ke
     };
     const size_t np = (size_t)3 * nmax;
     L.coef = take(sizeof(StarCoef) * nmax);
-    L.coefc = take(sizeof(StarCoef) * nmax);
+    L.ns = take(node ? sizeof(NodeStar<false>) * nmax : 0);
     L.theta = take(8 * np);
     L.delta = take(8 * np);
     L.dsc = take(8 * np);
@@ -132,18 +152,18 @@ __host__ __device__ inline Layout make_layout(int nmax, int S2, int umax, int ke
     L.live = take(nmax);
     L.conv = take(nmax);
     L.newf = take(nmax);
-    // V doubles as the key buffer of the union sort (keyn int32 <= 3 * 8 * nmax * S2 bytes)
+    // V doubles as the bit map (or key buffer) of the union (keyn int32 <= 3 * 8 * nmax * S2 bytes)
     size_t vbytes = (size_t)24 * nmax * S2;
     if (vbytes < (size_t)4 * keyn) vbytes = (size_t)4 * keyn;
     L.V = take(vbytes);
-    L.uidx = take((size_t)4 * nmax * S2);
+    L.uidx = take((size_t)2 * nmax * S2);
     L.dw = take((size_t)8 * umax);
-    L.w = take((size_t)8 * umax);
+    L.sw = take((size_t)8 * umax);
     L.wr = take((size_t)8 * umax);
     L.u = take((size_t)8 * umax);
     L.upix = take((size_t)4 * umax);
     L.fmask = take(sizeof(MaskT) * umax);
-    L.mmask = take(sizeof(MaskT) * umax);
+    L.mmask = same ? L.fmask : take(sizeof(MaskT) * umax);
     L.total = o;
     return L;
 }
@@ -226,22 +246,39 @@ __device__ __forceinline__ void psf_grad(const DevPsf& P, const StarCoef& c, int
     model_grad<double, double>(P, P.data64, c, (double)gy, (double)gx, g);
 }
 
-template <int NT, typename MaskT>
+// One group's fit by one block.  What bounds it: latency -- a group is a few hundred to
+// two thousand pixels, so every step is a short dependent chain between block barriers.
+// Hence two resident 256-thread blocks an SM (see plan_tiers); per-star cubic weights
+// (NodeStar) instead of a stencil worked out at every pixel; the accepted candidate's
+// residual kept as the next iteration's; and in LSQR the scalar recurrences, stopping
+// tests and the update of x and w on warp 0 while the other warps already gather the next
+// J v.  4,000 groups of 2-12 stars measured on the
+// B200: 13.6 ms with one block an SM, generic stencils and three barriers an iteration,
+// 9.6 ms now; 60 Gaussian groups 421 and 349 us.
+template <int NT, typename MaskT, bool NODE>
 struct GroupFit {
+    static constexpr int NW = NT / 32;
+    // warps that leave the next J v to the others while warp 0 works the scalars: with two
+    // warps that would be half the block, so there both gather
+    static constexpr bool kSplit = NW >= 4;
     const GroupConst& C;
     const DevPsf& P;
+    const PPNode& N;
     const GroupOut& O;
     GView G;
     char* smem;
     Layout L;
     double* sh;       // 64 doubles of reduction scratch
+    int* s_stop;      // 2 flags, used in turn
     int flip = 0;
     int n_act = 0, nU = 0;
+    unsigned nymag = 0;
 
     __device__ StarCoef* coef() const { return (StarCoef*)(smem + L.coef); }
-    __device__ StarCoef* coefc() const { return (StarCoef*)(smem + L.coefc); }
+    __device__ NodeStar<false>* ns() const { return (NodeStar<false>*)(smem + L.ns); }
     __device__ double* dp(size_t o) const { return (double*)(smem + o); }
     __device__ int32_t* ip(size_t o) const { return (int32_t*)(smem + o); }
+    __device__ uint16_t* hp(size_t o) const { return (uint16_t*)(smem + o); }
     __device__ uint8_t* bp(size_t o) const { return (uint8_t*)(smem + o); }
     __device__ MaskT* mp(size_t o) const { return (MaskT*)(smem + o); }
 
@@ -258,54 +295,122 @@ struct GroupFit {
             else if (C.gc[k] == 2) c.x = v;
             else c.flux = v;
         }
-        grid_corners_dw(P, c.y, c.x, c);
+        if (!NODE) grid_corners_dw(P, c.y, c.x, c);
     }
-    __device__ double mval(const StarCoef& c, int gy, int gx) const { return psf_value(P, c, gy, gx); }
+    // Star a's model at pixel (gy, gx) of its model box.
+    __device__ double mval(int a, int gy, int gx) const {
+        if (NODE) {
+            const StarCoef& c = coef()[a];
+            return c.flux * ns()[a].value(N, N.pp, gy - ip(L.ay)[a] + C.mR, gx - ip(L.ax)[a] + C.mR) + c.bkg;
+        }
+        return psf_value(P, coef()[a], gy, gx);
+    }
     __device__ void uxy(int u, int& gy, int& gx) const {
-        const int q = ip(L.upix)[u];
-        gy = q % G.ny + 1;
-        gx = q / G.ny + 1;
+        int r;
+        gx = quot(ip(L.upix)[u], G.ny, nymag, r) + 1;
+        gy = r + 1;
+    }
+    // stamp entry m = row + col S
+    __device__ int srow(int m, int& col) const {
+        int r;
+        col = quot(m, C.S, C.Smag, r);
+        return r;
     }
 
-    // coef[a] for every active slot at theta (+ delta into coefc).
+    // Block-wide sum of the warps' lane-0 values, in warp order; one barrier.
+    __device__ double warps_sum(double lane0) {
+        double* b = sh + 32 * (flip & 1);
+        ++flip;
+        if ((threadIdx.x & 31) == 0) b[threadIdx.x >> 5] = lane0;
+        __syncthreads();
+        double r = 0.0;
+#pragma unroll
+        for (int k = 0; k < NW; ++k) r += b[k];
+        return r;
+    }
+
+    // coef[a] (and the star's weights over its model box) for every active slot at theta
+    // (+ delta), a warp a star.
     __device__ void coefs(bool cand) {
         const double* th = dp(L.theta);
-        for (int a = threadIdx.x; a < n_act; a += NT) {
+        for (int a = threadIdx.x >> 5; a < n_act; a += NW) {
             StarCoef c;
             make_coef(a, th, cand ? dp(L.delta) : nullptr, c);
-            (cand ? coefc() : coef())[a] = c;
+            if (NODE) {
+                NodeStar<false> S;
+                const int n = 2 * C.mR + 1;
+                S.set(N, c.y, c.x, ip(L.ay)[a] - C.mR, ip(L.ax)[a] - C.mR, n, n);
+                if ((threadIdx.x & 31) == 0) {
+                    ns()[a] = S;
+                    StarCoef& t = coef()[a];
+                    t.y = c.y;
+                    t.x = c.x;
+                    t.flux = c.flux;
+                    t.bkg = c.bkg;
+                }
+            } else if ((threadIdx.x & 31) == 0) {
+                coef()[a] = c;
+            }
         }
         __syncthreads();
     }
 
     // _fill_stamps! (:342-543) for the live stars (all when `all`); with `gram`
     // the per-star p x p Gram block of the raw columns is written instead of V
-    // (errors pass, :1302-1329).  One warp per star.
+    // (errors pass, :1302-1329).  One warp per star.  V is zero at unusable entries.
     __device__ void fill(bool all, double* gram) {
         const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-        const int p = C.p, S = C.S, S2 = C.S2, R = C.R;
+        const int p = C.p, S2 = C.S2, R = C.R;
         double* V = dp(L.V);
-        const int32_t* ui = ip(L.uidx);
-        const double* w = dp(L.w);
+        const uint16_t* ui = hp(L.uidx);
+        const double* sw = dp(L.sw);
         double* cn = dp(L.cn);
         const uint8_t* live = bp(L.live);
-        const StarCoef* cf = coef();
-        for (int a = wid; a < n_act; a += NT / 32) {
+        for (int a = wid; a < n_act; a += NW) {
             if (!all && !live[a]) continue;
-            const StarCoef c = cf[a];
+            StarCoef c;
+            NodeStar<false> T;
+            if (NODE) {
+                T = ns()[a];
+                c.flux = coef()[a].flux;
+            } else {
+                c = coef()[a];
+            }
             const int ay = ip(L.ay)[a], ax = ip(L.ax)[a];
             double s0 = 0, s1 = 0, s2 = 0, g01 = 0, g02 = 0, g12 = 0;
             for (int m = lane; m < S2; m += 32) {
                 const int u = ui[a * S2 + m];
-                if (u == kNoU) continue;
-                const int gy = ay + (m % S) - R, gx = ax + (m / S) - R;
-                double g[3];
-                psf_grad(P, c, gy, gx, g);
-                const double swv = sqrt(w[u]);
                 double r[3] = {0, 0, 0};
-                for (int k = 0; k < p; ++k) r[k] = swv * g[C.gc[k] - 1];
-                if (!gram)
-                    for (int k = 0; k < p; ++k) V[(a * S2 + m) * p + k] = r[k];
+                if (u != kNoU16) {
+                    int col;
+                    const int row = srow(m, col);
+                    double g[3];
+                    if (NODE) {
+                        const int i = row - R + C.mR, j = col - R + C.mR;
+                        g[0] = g[1] = c.flux * 0.0;
+                        g[2] = N.nd.fill;
+                        if (i >= T.sy.lo && i <= T.sy.hi && j >= T.sx.lo && j <= T.sx.hi) {
+                            double rv[4], rd[4];
+                            T.template rows<true>(N.pp, i, j, rv, rd);
+                            const double dv = T.dy[0] * rv[0] + T.dy[1] * rv[1] + T.dy[2] * rv[2] + T.dy[3] * rv[3];
+                            const double du = T.wy[0] * rd[0] + T.wy[1] * rd[1] + T.wy[2] * rd[2] + T.wy[3] * rd[3];
+                            g[0] = c.flux * -(N.nd.sy * dv);
+                            g[1] = c.flux * -(N.nd.sx * du);
+                            g[2] = T.wy[0] * rv[0] + T.wy[1] * rv[1] + T.wy[2] * rv[2] + T.wy[3] * rv[3];
+                        }
+                    } else {
+                        psf_grad(P, c, ay + row - R, ax + col - R, g);
+                    }
+                    const double swv = sw[u];
+#pragma unroll
+                    for (int k = 0; k < 3; ++k)
+                        if (k < p) r[k] = swv * (C.gc[k] == 1 ? g[0] : (C.gc[k] == 2 ? g[1] : g[2]));
+                }
+                if (!gram) {
+#pragma unroll
+                    for (int k = 0; k < 3; ++k)
+                        if (k < p) V[(a * S2 + m) * p + k] = r[k];
+                }
                 s0 += r[0] * r[0];
                 s1 += r[1] * r[1];
                 s2 += r[2] * r[2];
@@ -331,55 +436,50 @@ struct GroupFit {
                 }
                 continue;
             }
-            const double ss[3] = {s0, s1, s2};
-            double inv[3];
-            for (int k = 0; k < p; ++k) {
-                double cv = sqrt(ss[k]);
-                cv = cv < kEpsG ? kEpsG : cv;
-                inv[k] = 1.0 / cv;
-                if (lane == 0) cn[a * p + k] = cv;
-            }
+            const double ss[3] = {__shfl_sync(0xffffffffu, s0, 0), __shfl_sync(0xffffffffu, s1, 0),
+                                  __shfl_sync(0xffffffffu, s2, 0)};
+            double inv[3] = {0, 0, 0};
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                if (k < p) {
+                    double cv = sqrt(ss[k]);
+                    cv = cv < kEpsG ? kEpsG : cv;
+                    inv[k] = 1.0 / cv;
+                    if (lane == 0) cn[a * p + k] = cv;
+                }
             for (int m = lane; m < S2; m += 32) {
-                if (ui[a * S2 + m] == kNoU) continue;
-                for (int k = 0; k < p; ++k) V[(a * S2 + m) * p + k] *= inv[k];
+#pragma unroll
+                for (int k = 0; k < 3; ++k)
+                    if (k < p) V[(a * S2 + m) * p + k] *= inv[k];
             }
         }
         __syncthreads();
     }
 
-    // Model render on U for the stars in `sel` (bit a = active slot a):
-    // mode 0: weighted residual wr = sqrt(w) (model - data_work) and its cost;
-    // mode 1: candidate cost sum w (model - data_work)^2 at coefc;
-    // mode 2: data_work -= model (frozen-star subtraction).
-    __device__ double render(int mode, MaskT sel) {
-        const StarCoef* cf = mode == 1 ? coefc() : coef();
+    // sqrt(w) (model - data_work) on U into `to` and its cost, for the stars in `sel` (bit
+    // a = active slot a); `freeze`: data_work -= model (frozen-star subtraction) instead.
+    __device__ double render(bool freeze, MaskT sel, double* to) {
         const MaskT* mm = mp(L.mmask);
         double* dw = dp(L.dw);
-        const double* w = dp(L.w);
-        double* wr = dp(L.wr);
+        const double* sw = dp(L.sw);
         double part = 0.0;
         for (int u = threadIdx.x; u < nU; u += NT) {
             int gy, gx;
             uxy(u, gy, gx);
             MaskT m = mm[u] & sel;
-            if (mode == 2) {
+            if (freeze) {
                 double d = dw[u];
-                while (m) d -= mval(cf[next_bit(m)], gy, gx);
+                while (m) d -= mval(next_bit(m), gy, gx);
                 dw[u] = d;
                 continue;
             }
             double acc = 0.0;
-            while (m) acc += mval(cf[next_bit(m)], gy, gx);
-            const double r = acc - dw[u];
-            if (mode == 0) {
-                const double v = sqrt(w[u]) * r;
-                wr[u] = v;
-                part += v * v;
-            } else {
-                part += w[u] * r * r;
-            }
+            while (m) acc += mval(next_bit(m), gy, gx);
+            const double v = sw[u] * (acc - dw[u]);
+            to[u] = v;
+            part += v * v;
         }
-        if (mode == 2) {
+        if (freeze) {
             __syncthreads();
             return 0.0;
         }
@@ -392,24 +492,25 @@ struct GroupFit {
         const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
         const int p = C.p, S2 = C.S2;
         const double* V = dp(L.V);
-        const int32_t* ui = ip(L.uidx);
+        const uint16_t* ui = hp(L.uidx);
         const uint8_t* live = bp(L.live);
         double part = 0.0;
-        for (int a = wid; a < n_act; a += NT / 32) {
+        for (int a = wid; a < n_act; a += NW) {
             if (!live[a]) continue;
             double z0 = 0, z1 = 0, z2 = 0;
+#pragma unroll 2
             for (int m = lane; m < S2; m += 32) {
                 const int u = ui[a * S2 + m];
-                if (u == kNoU) continue;
-                const double uv = lsqr ? src[u] * scale : src[u];
+                double uv = u == kNoU16 ? 0.0 : src[u];
+                if (lsqr) uv *= scale;
                 const double* v = V + (a * S2 + m) * p;
                 z0 += v[0] * uv;
                 if (p > 1) z1 += v[1] * uv;
                 if (p > 2) z2 += v[2] * uv;
             }
             z0 = warp_sum(z0);
-            z1 = warp_sum(z1);
-            z2 = warp_sum(z2);
+            if (p > 1) z1 = warp_sum(z1);
+            if (p > 2) z2 = warp_sum(z2);
             if (lane == 0) {
                 for (int k = 0; k < p; ++k) {
                     double val = k == 0 ? z0 : (k == 1 ? z1 : z2);
@@ -425,12 +526,14 @@ struct GroupFit {
             __syncthreads();
             return 0.0;
         }
-        return block_allsum<NT>(part, sh, flip);
+        return warps_sum(part);
     }
 
     // u_new = J v / alpha - alpha u_old (apply_J!, :95-137, gathered per pixel of
-    // U in Morton order); u_old = src * uscale.  Returns ||u_new||^2.
-    __device__ double jv(const double* src, double uscale, double alpha, double inv_alpha, MaskT live_bits) {
+    // U in Morton order); u_old = src * uscale.  Returns the calling thread's part of
+    // ||u_new||^2 over the pixels t0, t0 + tn, ...
+    __device__ double jv(const double* src, double uscale, double alpha, double inv_alpha, MaskT live_bits, int t0,
+                         int tn) {
         const int p = C.p, S = C.S, S2 = C.S2, R = C.R;
         const double* V = dp(L.V);
         const double* vt = dp(L.vt);
@@ -439,7 +542,7 @@ struct GroupFit {
         const int32_t* ax = ip(L.ax);
         double* uu = dp(L.u);
         double part = 0.0;
-        for (int u = threadIdx.x; u < nU; u += NT) {
+        for (int u = t0; u < nU; u += tn) {
             int gy, gx;
             uxy(u, gy, gx);
             MaskT m = fm[u] & live_bits;
@@ -457,133 +560,156 @@ struct GroupFit {
             uu[u] = un;
             part += un * un;
         }
-        return block_allsum<NT>(part, sh, flip);
+        return part;
     }
 
     // Damped LSQR (Paige & Saunders 1982, Krylov.jl 0.10 stopping rules) on
     // min ||J d + r||^2 + lambda ||d||^2, right-hand side -wr, zero start.
-    // Returns the iterations run.
+    // Returns the iterations run.  Two barriers an iteration: after J' u, and after the
+    // step in which warp 0 works the scalars, x, w and the stopping tests while the others
+    // gather the next iteration's J v (whose u is simply not used after a stop).
     __device__ int lsqr(double cost, double lam, MaskT live_bits) {
-        const int n = n_act * C.p;
+        const int n = n_act * C.p, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
         double* xl = dp(L.xl);
         double* vt = dp(L.vt);
         double* wl = dp(L.wl);
         const double* bsc = dp(L.bsc);
         const double beta1 = sqrt(cost);
-        for (int i = threadIdx.x; i < n; i += NT) xl[i] = 0.0;
+        if (wid == 0)
+            for (int i = lane; i < n; i += 32) xl[i] = 0.0;
         if (beta1 == 0.0) {
             __syncthreads();
             return 0;
         }
         const double inv_b1 = 1.0 / beta1;
-        // v1 = A'u1 = -b / beta1 (the gradient pass already holds A'r)
+        // v1 = A'u1 = -b / beta1 (the gradient pass already holds A'r); every warp sums its norm
         double part = 0.0;
-        for (int i = threadIdx.x; i < n; i += NT) {
+        for (int i = lane; i < n; i += 32) {
             const double v = -(bsc[i] * inv_b1);
-            vt[i] = v;
+            if (wid == 0) vt[i] = v;
             part += v * v;
         }
-        const double a2 = block_allsum<NT>(part, sh, flip);
+        const double a2 = __shfl_sync(0xffffffffu, warp_sum(part), 0);
         double alpha = sqrt(a2);
-        if (alpha == 0.0) return 0;
+        const double t0 = (alpha * beta1) / (alpha * beta1);
+        if (alpha == 0.0 || t0 <= 1.4901161193847656e-08 || 1.0 + t0 <= 1.0) {
+            __syncthreads();
+            return 0;
+        }
         double inv_alpha = 1.0 / alpha;
-        {
-            const double t = (alpha * beta1) / (alpha * beta1);
-            if (t <= 1.4901161193847656e-08 || 1.0 + t <= 1.0) return 0;
+        double wnorm2 = 0.0;
+        if (wid == 0) {
+            part = 0.0;
+            for (int i = lane; i < n; i += 32) {
+                const double v = vt[i] * inv_alpha;
+                wl[i] = v;
+                part += v * v;
+            }
+            wnorm2 = warp_sum(part);
         }
-        part = 0.0;
-        for (int i = threadIdx.x; i < n; i += NT) {
-            const double v = vt[i] * inv_alpha;
-            wl[i] = v;
-            part += v * v;
-        }
-        double wnorm2 = block_allsum<NT>(part, sh, flip);
+        __syncthreads();
         const double lambda = sqrt(lam);
         double Anorm2 = a2, dNorm2 = 0, xNorm2 = 0, c2 = -1, s2 = 0, z = 0, xENorm2 = 0, res2 = 0;
-        double rhobar = alpha, phibar = beta1, inv_beta = inv_b1, beta = beta1;
+        double rhobar = alpha, phibar = beta1, inv_beta = inv_b1;
         double err_vec[5] = {0, 0, 0, 0, 0};
         const double atol = C.linear_tol, btol = C.linear_tol;
         const double axtol = 1.4901161193847656e-08, etol = axtol, ctol = axtol;
-        int iter = 0;
-        for (int it = 0; it < C.itmax; ++it) {
-            // beta u = A v - alpha u
-            const double b2 = jv(it == 0 ? dp(L.wr) : dp(L.u), (it == 0 ? -1.0 : 1.0) * inv_beta, alpha, inv_alpha,
-                                 live_bits);
-            beta = sqrt(b2);
+        // beta u = A v - alpha u
+        double b2 = block_allsum<NT>(jv(dp(L.wr), -inv_beta, alpha, inv_alpha, live_bits, threadIdx.x, NT), sh, flip);
+        for (int it = 0;; ++it) {
+            const double beta = sqrt(b2);
+            const double alpha_old = alpha;
             if (beta != 0.0) {
                 inv_beta = 1.0 / beta;
-                Anorm2 = Anorm2 + alpha * alpha + beta * beta;
-                if (lambda > 0) Anorm2 += lambda * lambda;
                 // alpha v = A'u - beta v
                 const double an2 = jt(dp(L.u), inv_beta, true, beta, inv_alpha, vt);
                 alpha = sqrt(an2);
                 inv_alpha = alpha != 0.0 ? 1.0 / alpha : 0.0;
             }
-            double c1, s1, rhobar1;
-            sym_givens(rhobar, lambda, c1, s1, rhobar1);
-            const double psi = s1 * phibar;
-            phibar = c1 * phibar;
-            double c, s, rho;
-            sym_givens(rhobar1, beta, c, s, rho);
-            const double phi = c * phibar;
-            phibar = s * phibar;
-            const double theta = s * alpha;
-            const double sigma = phi / rho, tr = -theta / rho;
-            part = 0.0;
-            for (int i = threadIdx.x; i < n; i += NT) {
-                const double wi = wl[i];
-                xl[i] = xl[i] + sigma * wi;
-                const double wn = vt[i] * inv_alpha + tr * wi;
-                wl[i] = wn;
-                part += wn * wn;
-            }
-            const double wn2 = block_allsum<NT>(part, sh, flip);
-            iter += 1;
-            xENorm2 = xENorm2 + phi * phi;
-            err_vec[iter % 5] = phi;
-            double err_lbnd = 0;
-            if (iter >= 5) {
+            const bool last = it + 1 >= C.itmax;
+            if (wid == 0) {
+                const int iter = it + 1;
+                if (beta != 0.0) {
+                    Anorm2 = Anorm2 + alpha_old * alpha_old + beta * beta;
+                    if (lambda > 0) Anorm2 += lambda * lambda;
+                }
+                double c1, s1, rhobar1;
+                sym_givens(rhobar, lambda, c1, s1, rhobar1);
+                const double psi = s1 * phibar;
+                phibar = c1 * phibar;
+                double c, s, rho;
+                sym_givens(rhobar1, beta, c, s, rho);
+                const double phi = c * phibar;
+                phibar = s * phibar;
+                const double theta = s * alpha;
+                const double sigma = phi / rho, tr = -theta / rho;
+                part = 0.0;
+                for (int i = lane; i < n; i += 32) {
+                    const double wi = wl[i];
+                    xl[i] = xl[i] + sigma * wi;
+                    const double wn = vt[i] * inv_alpha + tr * wi;
+                    wl[i] = wn;
+                    part += wn * wn;
+                }
+                const double wn2 = warp_sum(part);
+                xENorm2 = xENorm2 + phi * phi;
                 double e2 = 0;
-                for (int k = 0; k < 5; ++k) e2 += err_vec[k] * err_vec[k];
-                err_lbnd = sqrt(e2);
+#pragma unroll
+                for (int k = 0; k < 5; ++k) {
+                    if (k == iter % 5) err_vec[k] = phi;
+                    e2 += err_vec[k] * err_vec[k];
+                }
+                const double err_lbnd = iter >= 5 ? sqrt(e2) : 0.0;
+                const double tau = s * phi;
+                dNorm2 = dNorm2 + wnorm2 / (rho * rho);
+                const double delta = s2 * rho;
+                const double gambar = -c2 * rho;
+                const double rhs = phi - delta * z;
+                const double zbar = rhs / gambar;
+                const double xNorm = sqrt(xNorm2 + zbar * zbar);
+                double gamma;
+                sym_givens(gambar, theta, c2, s2, gamma);
+                z = rhs / gamma;
+                xNorm2 = xNorm2 + z * z;
+                const double Anorm = sqrt(Anorm2);
+                const double Acond = Anorm * sqrt(dNorm2);
+                const double res1 = phibar * phibar;
+                res2 = res2 + psi * psi;
+                const double rNorm = sqrt(res1 + res2);
+                const double ArNorm = alpha * fabs(tau);
+                const double test1 = rNorm / beta1;
+                const double test2 = ArNorm / (Anorm * rNorm);
+                const double test3 = 1.0 / Acond;
+                const double t1 = test1 / (1.0 + Anorm * xNorm / beta1);
+                const double rNormtol = btol + axtol * Anorm * xNorm / beta1;
+                const bool ill = (1.0 + test3 <= 1.0) || (test3 <= ctol);
+                const bool zr = (1.0 + t1 <= 1.0) || (test1 <= rNormtol);
+                const bool fwd = iter >= 5 && err_lbnd <= etol * sqrt(xENorm2);
+                const bool solved = (1.0 + test2 <= 1.0) || (test2 <= axtol) || (ArNorm <= atol) || zr || fwd;
+                rhobar = -c * alpha;
+                wnorm2 = wn2;
+                // lane 0's: wnorm2 above is complete there only
+                if (lane == 0) s_stop[it & 1] = solved || ill;
             }
-            const double tau = s * phi;
-            dNorm2 = dNorm2 + wnorm2 / (rho * rho);
-            const double delta = s2 * rho;
-            const double gambar = -c2 * rho;
-            const double rhs = phi - delta * z;
-            const double zbar = rhs / gambar;
-            const double xNorm = sqrt(xNorm2 + zbar * zbar);
-            double gamma;
-            sym_givens(gambar, theta, c2, s2, gamma);
-            z = rhs / gamma;
-            xNorm2 = xNorm2 + z * z;
-            const double Anorm = sqrt(Anorm2);
-            const double Acond = Anorm * sqrt(dNorm2);
-            const double res1 = phibar * phibar;
-            res2 = res2 + psi * psi;
-            const double rNorm = sqrt(res1 + res2);
-            const double ArNorm = alpha * fabs(tau);
-            const double test1 = rNorm / beta1;
-            const double test2 = ArNorm / (Anorm * rNorm);
-            const double test3 = 1.0 / Acond;
-            const double t1 = test1 / (1.0 + Anorm * xNorm / beta1);
-            const double rNormtol = btol + axtol * Anorm * xNorm / beta1;
-            const bool ill = (1.0 + test3 <= 1.0) || (test3 <= ctol);
-            const bool zr = (1.0 + t1 <= 1.0) || (test1 <= rNormtol);
-            const bool fwd = iter >= 5 && err_lbnd <= etol * sqrt(xENorm2);
-            const bool solved = (1.0 + test2 <= 1.0) || (test2 <= axtol) || (ArNorm <= atol) || zr || fwd;
-            rhobar = -c * alpha;
-            wnorm2 = wn2;
-            if (solved || ill || iter >= C.itmax) break;
+            part = 0.0;
+            if (!last && (!kSplit || wid != 0))
+                part = jv(dp(L.u), inv_beta, alpha, inv_alpha, live_bits, kSplit ? threadIdx.x - 32 : threadIdx.x,
+                          kSplit ? NT - 32 : NT);
+            b2 = block_allsum<NT>(part, sh, flip);
+            if (last || s_stop[it & 1]) return it + 1;
         }
-        return iter;
     }
 };
 
-template <int NT, typename MaskT>
-__global__ void __launch_bounds__(NT) k_groups(GroupConst C, DevPsf P, GroupIn in, GroupOut O,
-                                               const int32_t* __restrict__ glist, int nlist, int* queue) {
+// Groups come from glist[0 .. nlist) through the queue counter, then from ovf_in (nullable;
+// its count *ovf_n_in, complete before the launch).  A group whose union exceeds the
+// layout's umax is appended to ovf_out and left to the next launch (without ovf_out the
+// layout holds any union of its groups).
+template <int NT, typename MaskT, bool NODE>
+__global__ void __launch_bounds__(NT, 512 / NT) k_groups(GroupConst C, DevPsf P, GroupIn in, GroupOut O,
+                                                         const int32_t* __restrict__ glist, int nlist, int* queue,
+                                                         const int32_t* __restrict__ ovf_in, const int* ovf_n_in,
+                                                         int32_t* ovf_out, int* ovf_n_out) {
     extern __shared__ __align__(16) char smem[];
     __shared__ double sh[64];
     __shared__ int s_g;
@@ -593,10 +719,15 @@ __global__ void __launch_bounds__(NT) k_groups(GroupConst C, DevPsf P, GroupIn i
     __shared__ uint8_t s_ok[kMaxGroupStars];
     const double NaN = __longlong_as_double(0x7ff8000000000000LL);
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    GroupFit<NT, MaskT> F{C, P, O};
+    __shared__ PPNode s_node;
+    __shared__ int s_stop[2];
+    if (NODE && tid == 0) node_of(P, s_node);
+    const int n_ovf = ovf_in ? *ovf_n_in : 0;
+    GroupFit<NT, MaskT, NODE> F{C, P, s_node, O};
     F.smem = smem;
-    F.L = make_layout<MaskT>(C.nmax, C.S2, C.umax, C.keyn);
+    F.L = make_layout<MaskT>(C.nmax, C.S2, C.umax, C.keyn, NODE, C.same);
     F.sh = sh;
+    F.s_stop = s_stop;
     F.G.in = in;
     F.G.eltype = C.eltype;
     const int p = C.p, S = C.S, S2 = C.S2, R = C.R;
@@ -605,14 +736,15 @@ __global__ void __launch_bounds__(NT) k_groups(GroupConst C, DevPsf P, GroupIn i
         __syncthreads();
         const int li = s_g;
         __syncthreads();
-        if (li >= nlist) break;
-        const int g = glist[li];
+        if (li >= nlist + n_ovf) break;
+        const int g = li < nlist ? glist[li] : ovf_in[li - nlist];
         const int64_t soff = in.star_off[g];
         const int ng = (int)(in.star_off[g + 1] - soff);
         F.G.off = in.pix_off[g];
         F.G.ny = in.ny[g];
         F.G.nx = in.nx[g];
         const int ny = F.G.ny, nx = F.G.nx;
+        F.nymag = quot_magic((unsigned)ny);
         const int64_t npix = (int64_t)ny * nx;
         const double* y0 = in.y0 + soff;
         const double* x0 = in.x0 + soff;
@@ -712,7 +844,9 @@ __global__ void __launch_bounds__(NT) k_groups(GroupConst C, DevPsf P, GroupIn i
             int any = 0;
             if (fin)
                 for (int m = lane; m < S2; m += 32) {
-                    const int gy = ay + (m % S) - R, gx = ax + (m / S) - R;
+                    int col;
+                    const int row = F.srow(m, col);
+                    const int gy = ay + row - R, gx = ax + col - R;
                     if (gy >= 1 && gy <= ny && gx >= 1 && gx <= nx) {
                         double d, w;
                         F.G.data_w((gy - 1) + (int64_t)(gx - 1) * ny, d, w);
@@ -785,56 +919,22 @@ __global__ void __launch_bounds__(NT) k_groups(GroupConst C, DevPsf P, GroupIn i
             frozen[a] = 0;
             for (int k = 0; k < p; ++k) cn[a * p + k] = 0.0;
         }
-        // ---- union of usable stamp pixels (_touched_pixels, :329-335): sort the
-        // entries' pixel indices (bitonic, in the V region) and drop duplicates
-        int32_t* keys = F.ip(F.L.V);
-        const int ne = n_act * S2;
-        int kn = 2;
-        while (kn < ne) kn <<= 1;
-        for (int e = tid; e < kn; e += NT) {
-            int key = kNoU;
-            if (e < ne) {
-                const int a = e / S2, m = e % S2;
-                const int gy = s_ay0[act[a]] + (m % S) - R, gx = s_ax0[act[a]] + (m / S) - R;
-                if (gy >= 1 && gy <= ny && gx >= 1 && gx <= nx) {
-                    const int q = (gy - 1) + (gx - 1) * ny;
-                    double d, w;
-                    F.G.data_w(q, d, w);
-                    if (w > 0) key = q;
-                }
-            }
-            keys[e] = key;
-        }
-        __syncthreads();
-        for (int k = 2; k <= kn; k <<= 1)
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                for (int i = tid; i < kn; i += NT) {
-                    const int l = i ^ j;
-                    if (l > i) {
-                        const int ki = keys[i], kl = keys[l];
-                        const bool up = (i & k) == 0;
-                        if ((ki > kl) == up) {
-                            keys[i] = kl;
-                            keys[l] = ki;
-                        }
-                    }
-                }
-                __syncthreads();
-            }
-        // compaction of the distinct keys (chunked block scan)
+        // ---- union of usable stamp pixels (_touched_pixels, :329-335), in column-major
+        // order: a bit map of the boxes' bounding box, where it fits the V region, gives
+        // each pixel's place by counting bits (66 sorting steps with a barrier each for a
+        // full 12-star group otherwise: 10 % of the fit); stars far apart sort the entries'
+        // pixel indices (bitonic) and drop duplicates
         int32_t* upix = F.ip(F.L.upix);
-        {
-            const int per = (kn + NT - 1) / NT;
-            const int b0 = min(tid * per, kn), b1 = min(b0 + per, kn);
-            int cnt = 0;
-            for (int e = b0; e < b1; ++e) cnt += keys[e] != kNoU && (e == 0 || keys[e] != keys[e - 1]);
-            // exclusive scan of cnt over the block
+        uint16_t* uidx = F.hp(F.L.uidx);
+        const int ne = n_act * S2;
+        __shared__ int s_wsum[32];
+        // places by a chunked block scan of each thread's count; returns the thread's first
+        auto scan = [&](int cnt) {
             int incl = cnt;
             for (int o = 1; o < 32; o <<= 1) {
                 const int t = __shfl_up_sync(0xffffffffu, incl, o);
                 if (lane >= o) incl += t;
             }
-            __shared__ int s_wsum[32];
             if (lane == 31) s_wsum[wid] = incl;
             __syncthreads();
             int wbase = 0, tot = 0;
@@ -842,20 +942,128 @@ __global__ void __launch_bounds__(NT) k_groups(GroupConst C, DevPsf P, GroupIn i
                 if (k < wid) wbase += s_wsum[k];
                 tot += s_wsum[k];
             }
-            int pos = wbase + incl - cnt;
+            F.nU = tot;
+            return wbase + incl - cnt;
+        };
+        int by0 = ny, by1 = 1, bx0 = nx, bx1 = 1;  // the boxes' bounding box, clipped to the image
+        for (int j = 0; j < ng; ++j)
+            if (s_ok[j]) {
+                by0 = min(by0, max(s_ay0[j] - R, 1));
+                by1 = max(by1, min(s_ay0[j] + R, ny));
+                bx0 = min(bx0, max(s_ax0[j] - R, 1));
+                bx1 = max(bx1, min(s_ax0[j] + R, nx));
+            }
+        const int bh = by1 - by0 + 1, bw = bx1 - bx0 + 1;
+        const size_t vbytes = F.L.uidx - F.L.V;
+        const int64_t area = (int64_t)bh * bw;
+        const bool by_map = ((area + 31) / 32) * 8 <= (int64_t)vbytes;
+        if (by_map) {
+            const int nwords = (int)((area + 31) / 32);
+            unsigned* map = (unsigned*)F.ip(F.L.V);
+            int* place = (int*)(map + nwords);
+            for (int i = tid; i < nwords; i += NT) map[i] = 0;
+            __syncthreads();
+            for (int e = tid; e < ne; e += NT) {
+                const int a = e / S2;
+                int col;
+                const int row = F.srow(e - a * S2, col);
+                const int gy = ay[a] + row - R, gx = ax[a] + col - R;
+                if (gy >= 1 && gy <= ny && gx >= 1 && gx <= nx) {
+                    double d, w;
+                    F.G.data_w((gy - 1) + (int64_t)(gx - 1) * ny, d, w);
+                    const int b = (gy - by0) + (gx - bx0) * bh;
+                    if (w > 0) atomicOr(&map[b >> 5], 1u << (b & 31));
+                }
+            }
+            __syncthreads();
+            const int per = (nwords + NT - 1) / NT;
+            const int b0 = min(tid * per, nwords), b1 = min(b0 + per, nwords);
+            int cnt = 0;
+            for (int i = b0; i < b1; ++i) cnt += __popc(map[i]);
+            int pos = scan(cnt);
+            const unsigned bmag = quot_magic((unsigned)bh);
+            for (int i = b0; i < b1; ++i) {
+                unsigned m = map[i];
+                place[i] = pos;
+                while (m) {
+                    const int b = 32 * i + __ffs((int)m) - 1;
+                    m &= m - 1;
+                    int r;
+                    const int c = quot(b, bh, bmag, r);
+                    if (pos < C.umax) upix[pos] = (by0 - 1 + r) + (bx0 - 1 + c) * ny;
+                    ++pos;
+                }
+            }
+        } else {
+            int32_t* keys = F.ip(F.L.V);
+            int kn = 2;
+            while (kn < ne) kn <<= 1;
+            for (int e = tid; e < kn; e += NT) {
+                int key = kNoU;
+                if (e < ne) {
+                    const int a = e / S2, m = e % S2;
+                    const int gy = ay[a] + (m % S) - R, gx = ax[a] + (m / S) - R;
+                    if (gy >= 1 && gy <= ny && gx >= 1 && gx <= nx) {
+                        const int q = (gy - 1) + (gx - 1) * ny;
+                        double d, w;
+                        F.G.data_w(q, d, w);
+                        if (w > 0) key = q;
+                    }
+                }
+                keys[e] = key;
+            }
+            __syncthreads();
+            for (int k = 2; k <= kn; k <<= 1)
+                for (int j = k >> 1; j > 0; j >>= 1) {
+                    for (int i = tid; i < kn; i += NT) {
+                        const int l = i ^ j;
+                        if (l > i) {
+                            const int ki = keys[i], kl = keys[l];
+                            const bool up = (i & k) == 0;
+                            if ((ki > kl) == up) {
+                                keys[i] = kl;
+                                keys[l] = ki;
+                            }
+                        }
+                    }
+                    __syncthreads();
+                }
+            // compaction of the distinct keys
+            const int per = (kn + NT - 1) / NT;
+            const int b0 = min(tid * per, kn), b1 = min(b0 + per, kn);
+            int cnt = 0;
+            for (int e = b0; e < b1; ++e) cnt += keys[e] != kNoU && (e == 0 || keys[e] != keys[e - 1]);
+            int pos = scan(cnt);
             for (int e = b0; e < b1; ++e)
-                if (keys[e] != kNoU && (e == 0 || keys[e] != keys[e - 1]) && pos < C.umax) upix[pos++] = keys[e];
-            F.nU = min(tot, C.umax);
+                if (keys[e] != kNoU && (e == 0 || keys[e] != keys[e - 1])) {
+                    if (pos < C.umax) upix[pos] = keys[e];
+                    ++pos;
+                }
+        }
+        if (F.nU > C.umax) {  // block-uniform: left to the launch with the full layout
+            if (tid == 0) {
+                if (ovf_out) ovf_out[atomicAdd(ovf_n_out, 1)] = g;
+                else group_stats(0, ng, CPB_ERR_INTERNAL, 0, 0, 0, 0, 0);
+            }
+            __syncthreads();
+            continue;
         }
         __syncthreads();
         const int nU = F.nU;
-        // per stamp entry: its position in U (binary search), kNoU when unusable
-        int32_t* uidx = F.ip(F.L.uidx);
+        // per stamp entry: its position in U, kNoU16 when unusable
         for (int e = tid; e < ne; e += NT) {
-            const int a = e / S2, m = e % S2;
-            const int gy = ay[a] + (m % S) - R, gx = ax[a] + (m / S) - R;
-            int r = kNoU;
-            if (gy >= 1 && gy <= ny && gx >= 1 && gx <= nx) {
+            const int a = e / S2;
+            int col;
+            const int row = F.srow(e - a * S2, col);
+            const int gy = ay[a] + row - R, gx = ax[a] + col - R;
+            int r = kNoU16;
+            if (gy >= 1 && gy <= ny && gx >= 1 && gx <= nx && by_map) {
+                const int b = (gy - by0) + (gx - bx0) * bh;
+                const unsigned* map = (const unsigned*)F.ip(F.L.V);
+                const unsigned m = map[b >> 5];
+                const int* place = (const int*)(map + (area + 31) / 32);
+                if (m >> (b & 31) & 1) r = place[b >> 5] + __popc(m & ((1u << (b & 31)) - 1));
+            } else if (gy >= 1 && gy <= ny && gx >= 1 && gx <= nx) {
                 const int q = (gy - 1) + (gx - 1) * ny;
                 int lo = 0, hi = nU;
                 while (lo < hi) {
@@ -865,12 +1073,12 @@ __global__ void __launch_bounds__(NT) k_groups(GroupConst C, DevPsf P, GroupIn i
                 }
                 if (lo < nU && upix[lo] == q) r = lo;
             }
-            uidx[e] = r;
+            uidx[e] = (uint16_t)r;
         }
         // per pixel of U: data_work, w and the star masks
         {
             double* dw = F.dp(F.L.dw);
-            double* wv = F.dp(F.L.w);
+            double* swv = F.dp(F.L.sw);
             MaskT* fm = F.mp(F.L.fmask);
             MaskT* mm = F.mp(F.L.mmask);
             for (int u = tid; u < nU; u += NT) {
@@ -878,8 +1086,9 @@ __global__ void __launch_bounds__(NT) k_groups(GroupConst C, DevPsf P, GroupIn i
                 double d, w;
                 F.G.data_w(q, d, w);
                 dw[u] = d;
-                wv[u] = w;
-                const int gy = q % ny + 1, gx = q / ny + 1;
+                swv[u] = sqrt(w);
+                int gy, gx;
+                F.uxy(u, gy, gx);
                 MaskT f = 0, mo = 0;
                 for (int a = 0; a < n_act; ++a) {
                     const int dy = abs(gy - ay[a]), dx = abs(gx - ax[a]);
@@ -887,7 +1096,7 @@ __global__ void __launch_bounds__(NT) k_groups(GroupConst C, DevPsf P, GroupIn i
                     if (dy <= C.mR && dx <= C.mR) mo |= (MaskT)1 << a;
                 }
                 fm[u] = f;
-                mm[u] = mo;
+                if (!C.same) mm[u] = mo;
             }
         }
         const MaskT all_bits = n_act >= (int)(8 * sizeof(MaskT)) ? ~(MaskT)0 : (((MaskT)1 << n_act) - 1);
@@ -899,19 +1108,21 @@ __global__ void __launch_bounds__(NT) k_groups(GroupConst C, DevPsf P, GroupIn i
         // ---- initial fill and cost (:1171-1178)
         F.coefs(false);
         F.fill(false, nullptr);
-        double cost = F.render(0, live_bits);
+        double cost = F.render(false, live_bits, F.dp(F.L.wr));
         for (int i = tid; i < n; i += NT) D[i] = cn[i];
-        bool fresh = true;
+        // the last iteration's step was accepted: coef is at theta and wr, cost are the
+        // candidate's (rendered again when stars were frozen, their models gone from
+        // data_work); after a rejected one nothing has changed but lambda
+        bool moved = false, froze = false;
         double lam = C.lambda_init;
         int n_run = 0, n_trials = 0, n_lsqr = 0;
         // ---- outer loop (:1186-1284)
         for (int iter = 1; iter <= C.max_iter; ++iter) {
-            if (!fresh) {
-                F.coefs(false);
+            if (moved) {
                 F.fill(false, nullptr);
-                cost = F.render(0, live_bits);
+                if (froze) cost = F.render(false, live_bits, F.dp(F.L.wr));
             }
-            fresh = false;
+            moved = froze = false;
             for (int i = tid; i < n; i += NT) bsc[i] = 0.0;
             __syncthreads();
             F.jt(F.dp(F.L.wr), 1.0, false, 0.0, 0.0, bsc);
@@ -961,7 +1172,7 @@ __global__ void __launch_bounds__(NT) k_groups(GroupConst C, DevPsf P, GroupIn i
                 }
                 __syncthreads();
                 F.coefs(true);
-                const double cost_cand = F.render(1, live_bits);
+                const double cost_cand = F.render(false, live_bits, F.dp(F.L.u));
                 f_conv = (cost_cand < cost) && ((cost - cost_cand) / cost <= C.f_tol);
                 if (cost_cand < cost) {
                     accepted = true;
@@ -997,13 +1208,17 @@ __global__ void __launch_bounds__(NT) k_groups(GroupConst C, DevPsf P, GroupIn i
                         }
                     }
                     cost = cost_cand;
+                    moved = true;
+                    const size_t t = F.L.wr;
+                    F.L.wr = F.L.u;
+                    F.L.u = t;
                     if (__syncthreads_or(nf)) {
+                        froze = true;
                         MaskT nb = 0;
                         for (int a = 0; a < n_act; ++a)
                             if (newf[a]) nb |= (MaskT)1 << a;
                         live_bits &= ~nb;
-                        F.coefs(false);
-                        F.render(2, nb);  // _freeze_star! in Morton order
+                        F.render(true, nb, nullptr);  // _freeze_star! in Morton order
                     }
                     break;
                 }
@@ -1072,10 +1287,12 @@ __global__ void __launch_bounds__(NT) k_groups(GroupConst C, DevPsf P, GroupIn i
         // ---- final residual against the original data (:1344-1356), every active star
         if (O.residual) {
             for (int64_t q = tid; q < npix; q += NT) {
-                const int gy = (int)(q % ny) + 1, gx = (int)(q / ny) + 1;
+                int gy;
+                const int gx = quot((int)q, ny, F.nymag, gy) + 1;
+                ++gy;
                 double acc = 0.0;
                 for (int a = 0; a < n_act; ++a)
-                    if (abs(gy - ay[a]) <= C.mR && abs(gx - ax[a]) <= C.mR) acc += F.mval(cf[a], gy, gx);
+                    if (abs(gy - ay[a]) <= C.mR && abs(gx - ax[a]) <= C.mR) acc += F.mval(a, gy, gx);
                 double d, w;
                 F.G.data_w(q, d, w);
                 O.residual[F.G.off + q] = d - acc;
@@ -1096,13 +1313,18 @@ __global__ void __launch_bounds__(NT) k_groups(GroupConst C, DevPsf P, GroupIn i
             const int h = yhi - ylo + 1, wd = xhi - xlo + 1;
             const double inv_flux = 1.0 / c.flux;
             double* rw = C.sp_on ? O.sp_rw + (size_t)o * 2 * C.sp_box : nullptr;
+            NodeStar<false> T;  // the star's own weights: its box may have moved off the anchor's
+            if (NODE) T.set(s_node, c.y, c.x, ylo, xlo, max(h, 0), max(wd, 0));
+            const unsigned hmag = quot_magic((unsigned)max(h, 1));
             if (h > 0 && wd > 0)
                 for (int e = lane; e < h * wd; e += 32) {
-                    const int gy = ylo + e % h, gx = xlo + e / h;
+                    int er;
+                    const int ec = quot(e, h, hmag, er);
+                    const int gy = ylo + er, gx = xlo + ec;
                     const int64_t q = (gy - 1) + (int64_t)(gx - 1) * ny;
                     double acc = 0.0;
                     for (int b = 0; b < n_act; ++b)
-                        if (abs(gy - ay[b]) <= C.mR && abs(gx - ax[b]) <= C.mR) acc += F.mval(cf[b], gy, gx);
+                        if (abs(gy - ay[b]) <= C.mR && abs(gx - ax[b]) <= C.mR) acc += F.mval(b, gy, gx);
                     double d, wsan;
                     F.G.data_w(q, d, wsan);
                     const double r = d - acc;
@@ -1114,7 +1336,8 @@ __global__ void __launch_bounds__(NT) k_groups(GroupConst C, DevPsf P, GroupIn i
                     if (isfinite(wp) && wp > 0) {
                         num += wp * (r * r);
                         ng_ += 1;
-                        const double mv = F.mval(c, gy, gx);
+                        const double mv = NODE ? c.flux * T.value(s_node, s_node.pp, er, ec) + c.bkg
+                                               : psf_value(P, c, gy, gx);
                         qv += fabs(r);
                         const double Pp = (mv - c.bkg) * inv_flux;
                         const double wP = wp * Pp;
@@ -1287,14 +1510,22 @@ inline int next_pow2(int v) {
 constexpr int kBucketEdges[] = {32, 64};
 constexpr int kNumBuckets = sizeof(kBucketEdges) / sizeof(int);
 
-struct Bucket {
-    std::vector<int32_t> groups;
-    int nmax = 1, umax = 1, keyn = 2;
-    bool wide = false;
+// One launch over a bucket's groups or part of them.
+struct Tier {
+    int64_t first = 0, n = 0;  // its groups within the bucket's list
     size_t smem = 0;
     GroupConst C{};
+};
+
+struct Bucket {
+    std::vector<int32_t> groups;  // most stars first
+    int nmax = 1, umax = 1, keyn = 2;
+    bool wide = false;
+    Tier full, half;    // half.n > 0: two launches, half then full (plan_tiers)
     int threads = 256;  // default block size
 };
+constexpr int kQueueInts = 3;  // a bucket's counters: the two launches' queues, deferred groups
+
 
 struct GroupPlan {
     std::vector<Bucket> buckets;  // non-empty buckets only
@@ -1318,11 +1549,72 @@ struct GroupSetup {
     int64_t n_stars = 0;  // catalogue length (sizes the residual / weight planes)
 };
 
-constexpr size_t kStaticSmem = 8 * 1024;  // the kernel's static shared arrays, rounded up
+constexpr size_t kStaticSmem = 6 * 1024;  // the kernel's static shared arrays, rounded up
 
-template <typename MaskT>
-size_t layout_bytes(int nmax, int S2, int umax, int keyn) {
-    return make_layout<MaskT>(nmax, S2, umax, keyn).total;
+// Single-node image PSFs take the per-star weights (NODE).
+inline bool group_node(const DevPsf& P) { return P.kind != CPB_PSF_CIRCULAR_GAUSSIAN && P.n_nodes == 1; }
+
+// The size rule of a group that the kernel takes (others go to the full-field fit): two
+// coefficient sets, 32-bit stamp indices and separate masks, within the block's shared
+// memory less 8 KB.  The layout proper needs less at every size near that limit.
+size_t group_rule_bytes(int nmax, int S2, int umax, int keyn) {
+    const size_t n = (size_t)nmax, mask = nmax > 32 ? 8 : 4;
+    return 2 * align16(sizeof(StarCoef) * n) + 9 * align16(24 * n) + 4 * align16(4 * n) + 3 * align16(n) +
+           align16(std::max((size_t)24 * n * S2, (size_t)4 * keyn)) + align16(4 * n * S2) +
+           4 * align16((size_t)8 * umax) + align16((size_t)4 * umax) + 2 * align16(mask * umax);
+}
+
+size_t layout_bytes(const GroupConst& C, int nmax, int umax, int keyn, bool node) {
+    return nmax > 32 ? make_layout<uint64_t>(nmax, C.S2, umax, keyn, node, C.same).total
+                     : make_layout<uint32_t>(nmax, C.S2, umax, keyn, node, C.same).total;
+}
+
+// The bucket's launches.  One block of the layout for the largest group an SM leaves its
+// schedulers 80 % idle (4,000 groups of 2-12 stars, 152 KB: 12.3 ms, 20 % of issue slots).
+// The union of a blend's boxes is usually well below the bound its layout allows for, so
+// where two such blocks do not fit an SM, the groups of up to `nA` stars run first with a
+// layout of half an SM: its union capacity is what is left beside the stars' arrays, at
+// least half the bound.  A group whose union is larger appends itself to a list, and a
+// second launch with the full layout takes those and the groups of more stars.
+void plan_tiers(Bucket& B, const GroupConst& C, bool node, size_t smem_sm, const std::vector<int64_t>& soff,
+                const std::vector<int32_t>& ny, const std::vector<int32_t>& nx) {
+    auto stars = [&](int32_t g) { return (int)(soff[g + 1] - soff[g]); };
+    std::stable_sort(B.groups.begin(), B.groups.end(), [&](int32_t a, int32_t b) { return stars(a) > stars(b); });
+    auto tier = [&](Tier& t, int nmax, int umax, int keyn) {
+        t.C = C;
+        t.C.nmax = nmax;
+        t.C.umax = umax;
+        t.C.keyn = keyn;
+        t.smem = layout_bytes(C, nmax, umax, keyn, node);
+    };
+    tier(B.full, B.nmax, B.umax, B.keyn);
+    B.full.first = 0;
+    B.full.n = (int64_t)B.groups.size();
+    B.half.n = 0;
+    const size_t half = smem_sm / 2 - 1024 - kStaticSmem;
+    if (B.full.smem <= half || B.wide) return;
+    for (size_t i = 0; i < B.groups.size(); ++i) {  // B.groups[i ..) in the half launch
+        const int nA = stars(B.groups[i]);
+        if (i && nA == stars(B.groups[i - 1])) continue;
+        int um = 1;
+        for (size_t k = i; k < B.groups.size(); ++k)
+            um = std::max(um, (int)std::min<int64_t>((int64_t)stars(B.groups[k]) * C.S2,
+                                                     (int64_t)ny[B.groups[k]] * nx[B.groups[k]]));
+        const int keyn = next_pow2(std::max(nA * C.S2, 2));
+        auto fits = [&](int u) { return layout_bytes(C, std::max(nA, 1), u, keyn, node) <= half; };
+        if (!fits((um + 1) / 2)) continue;
+        int lo = (um + 1) / 2, hi = um;  // the largest capacity that fits
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) / 2;
+            if (fits(mid)) lo = mid;
+            else hi = mid - 1;
+        }
+        tier(B.half, std::max(nA, 1), lo, keyn);
+        B.half.first = (int64_t)i;
+        B.half.n = (int64_t)(B.groups.size() - i);
+        B.full.n = (int64_t)i;
+        return;
+    }
 }
 
 // Argument checks (the reference's, :984-1051), constants, group metadata on
@@ -1396,6 +1688,8 @@ void setup_groups(cpb_ctx* ctx, const cpb_psf* psf, const cpb_sim_params* P, int
     C.lambda_down = P->lambda_down;
     C.lambda_min = P->lambda_min;
     C.lambda_max = P->lambda_max;
+    C.same = C.mR == C.R;
+    C.Smag = quot_magic((unsigned)C.S);
     C.eltype = eltype;
     C.reweighted = (P->covariance == CPB_COV_REWEIGHTED || (P->covariance == CPB_COV_AUTO && d_iv == nullptr)) ? 1 : 0;
     C.fit_rad = P->fit_rad;
@@ -1450,7 +1744,7 @@ void setup_groups(cpb_ctx* ctx, const cpb_psf* psf, const cpb_sim_params* P, int
     int smem_optin = 0, smem_sm = 0;
     check(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device), "attr");
     check(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx->device), "attr");
-    const size_t cap = (size_t)smem_optin - kStaticSmem;
+    const size_t cap = (size_t)smem_optin - 8 * 1024;  // of the size rule
     su.n_stars = h_soff[G];
     if (C.sp_on) {
         // k_group_spread: the disk table and one panel of the quadrature, then
@@ -1465,9 +1759,9 @@ void setup_groups(cpb_ctx* ctx, const cpb_psf* psf, const cpb_sim_params* P, int
         su.sp_smem = fixed + nw * per_warp;
     }
     GroupPlan& plan = su.plan;
+    const bool node = group_node(su.dp);
     auto need_of = [&](int ng, int um, int kn) {
-        return ng > 32 ? layout_bytes<uint64_t>(std::max(ng, 1), C.S2, std::max(um, 1), kn)
-                       : layout_bytes<uint32_t>(std::max(ng, 1), C.S2, std::max(um, 1), kn);
+        return group_rule_bytes(std::max(ng, 1), C.S2, std::max(um, 1), kn);
     };
     // a group runs in the kernel when it has <= 64 stars and its own layout fits;
     // the kernel computes in FP64 with LSQR and one scalar model radius, so
@@ -1501,14 +1795,12 @@ void setup_groups(cpb_ctx* ctx, const cpb_psf* psf, const cpb_sim_params* P, int
     for (Bucket& B : bk) {
         if (B.groups.empty()) continue;
         B.wide = B.nmax > 32;
-        B.smem = need_of(B.nmax, B.umax, B.keyn);
-        B.C = C;
-        B.C.nmax = B.nmax;
-        B.C.umax = B.umax;
-        B.C.keyn = B.keyn;
+        if (layout_bytes(C, B.nmax, B.umax, B.keyn, node) > (size_t)smem_optin - kStaticSmem)
+            throw CudaError{cudaErrorInvalidConfiguration, "group layout"};  // the size rule excludes it
+        plan_tiers(B, C, node, (size_t)smem_sm, h_soff, h_ny, h_nx);
         // default block size: about 512 threads an SM (the kernel's register budget
         // allows 512 threads of 128 registers), in as many blocks as shared memory holds
-        const int by_smem = std::max(1, (int)((size_t)smem_sm / (B.smem + kStaticSmem + 1024)));
+        const int by_smem = std::max(1, (int)((size_t)smem_sm / ((B.half.n ? B.half.smem : B.full.smem) + kStaticSmem + 1024)));
         const int blocks = std::min(by_smem, 8);
         B.threads = blocks >= 8 ? 64 : (blocks >= 4 ? 128 : 256);
         plan.n_kernel += (int64_t)B.groups.size();
@@ -1516,60 +1808,60 @@ void setup_groups(cpb_ctx* ctx, const cpb_psf* psf, const cpb_sim_params* P, int
     }
 }
 
-template <int NT, typename MaskT>
-void* group_kernel() {
-    return (void*)k_groups<NT, MaskT>;
+using GroupKernel = void (*)(GroupConst, DevPsf, GroupIn, GroupOut, const int32_t*, int, int*, const int32_t*,
+                             const int*, int32_t*, int*);
+template <int NT>
+GroupKernel group_kernel(bool wide, bool node) {
+    return wide ? (node ? k_groups<NT, uint64_t, true> : k_groups<NT, uint64_t, false>)
+                : (node ? k_groups<NT, uint32_t, true> : k_groups<NT, uint32_t, false>);
 }
 
-void* group_kernel_for(int threads, bool wide) {
-    if (threads == 64) return wide ? group_kernel<64, uint64_t>() : group_kernel<64, uint32_t>();
-    if (threads == 128) return wide ? group_kernel<128, uint64_t>() : group_kernel<128, uint32_t>();
-    return wide ? group_kernel<256, uint64_t>() : group_kernel<256, uint32_t>();
+GroupKernel group_kernel_for(int threads, bool wide, bool node) {
+    return threads == 64 ? group_kernel<64>(wide, node)
+                         : (threads == 128 ? group_kernel<128>(wide, node) : group_kernel<256>(wide, node));
 }
 
 inline int valid_threads(int t) { return t == 64 ? 64 : (t == 128 ? 128 : 256); }
 
-// Resident blocks per SM of the group kernel for this bucket and block size.
-int group_occupancy(const Bucket& B, int threads) {
-    threads = valid_threads(threads);
-    void* kfn = group_kernel_for(threads, B.wide);
-    check(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)B.smem), "smem attr");
+// Resident blocks per SM of the group kernel with a launch's layout and this block size.
+int tier_occupancy(const Bucket& B, const Tier& T, int threads, bool node) {
+    GroupKernel kfn = group_kernel_for(threads, B.wide, node);
+    check(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T.smem), "smem attr");
     int per_sm = 0;
-    check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, threads, B.smem), "occupancy");
+    check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, threads, T.smem), "occupancy");
     return std::max(per_sm, 1);
 }
+int group_occupancy(const Bucket& B, int threads, bool node) {
+    return tier_occupancy(B, B.half.n ? B.half : B.full, valid_threads(threads), node);
+}
 
-// One launch of the group kernel over one bucket's groups: resets the work
-// queue and starts min(groups, SMs x blocks_per_sm) persistent blocks.
-// threads: 64, 128 or 256 (<= 0: the bucket's default); blocks_per_sm <= 0
-// means the occupancy limit.
+// The group kernel over one bucket's groups: resets its counters and starts, for each of
+// its launches, min(groups, SMs x blocks_per_sm) persistent blocks.  threads: 64, 128 or
+// 256 (<= 0: the bucket's default); blocks_per_sm <= 0 means the occupancy limit.  d_ovf:
+// room for the half launch's deferred groups; d_queue: kQueueInts counters.
 void launch_bucket(cpb_ctx* ctx, cudaStream_t st, const GroupSetup& su, const Bucket& B, const int32_t* d_list,
-                   int* d_queue, int threads, int blocks_per_sm) {
+                   int32_t* d_ovf, int* d_queue, int threads, int blocks_per_sm) {
     const int64_t nk = (int64_t)B.groups.size();
     if (nk <= 0) return;
     threads = valid_threads(threads <= 0 ? B.threads : threads);
-    const int occ = group_occupancy(B, threads);
-    const int per_sm = blocks_per_sm <= 0 ? occ : std::min(blocks_per_sm, occ);
-    const int64_t grid = std::min<int64_t>(nk, (int64_t)ctx->n_sm * per_sm);
-    check(cudaMemsetAsync(d_queue, 0, sizeof(int), st), "memset");
-    KernelScope ks_(ctx, "k_groups",
-                    (double)su.total_pixels * (su.eltype == CPB_F64 ? 8 : 4) * (su.gin.iv ? 2 : 1) * nk /
-                        std::max<int64_t>(su.plan.n_kernel, 1));
-    const size_t smem = B.smem;
-#define CPB_GROUPS_LAUNCH(NTV)                                                                                      \
-    do {                                                                                                            \
-        if (B.wide)                                                                                                 \
-            k_groups<NTV, uint64_t><<<(unsigned)grid, NTV, smem, st>>>(B.C, su.dp, su.gin, su.go, d_list, (int)nk, \
-                                                                       d_queue);                                   \
-        else                                                                                                        \
-            k_groups<NTV, uint32_t><<<(unsigned)grid, NTV, smem, st>>>(B.C, su.dp, su.gin, su.go, d_list, (int)nk, \
-                                                                       d_queue);                                   \
-    } while (0)
-    if (threads == 64) CPB_GROUPS_LAUNCH(64);
-    else if (threads == 128) CPB_GROUPS_LAUNCH(128);
-    else CPB_GROUPS_LAUNCH(256);
-#undef CPB_GROUPS_LAUNCH
-    check(cudaGetLastError(), "k_groups");
+    const bool node = group_node(su.dp);
+    GroupKernel kern = group_kernel_for(threads, B.wide, node);
+    check(cudaMemsetAsync(d_queue, 0, sizeof(int) * kQueueInts, st), "memset");
+    auto go = [&](const Tier& T, bool half) {
+        KernelScope ks_(ctx, "k_groups",
+                        (double)su.total_pixels * (su.eltype == CPB_F64 ? 8 : 4) * (su.gin.iv ? 2 : 1) * T.n /
+                            std::max<int64_t>(su.plan.n_kernel, 1));
+        const int occ = tier_occupancy(B, T, threads, node);
+        const int per_sm = blocks_per_sm <= 0 ? occ : std::min(blocks_per_sm, occ);
+        const int64_t grid = std::min<int64_t>(half ? T.n : nk, (int64_t)ctx->n_sm * per_sm);
+        const bool rest = !half && B.half.n;  // takes the half launch's deferred groups
+        kern<<<(unsigned)grid, threads, T.smem, st>>>(T.C, su.dp, su.gin, su.go, d_list + T.first, (int)T.n,
+                                                      d_queue + (half ? 0 : 1), rest ? d_ovf : nullptr, d_queue + 2,
+                                                      half ? d_ovf : nullptr, d_queue + 2);
+        check(cudaGetLastError(), "k_groups");
+    };
+    if (B.half.n) go(B.half, true);
+    go(B.full, false);
 }
 
 // k_group_spread over the kernel-fitted groups (after their bucket launches).
@@ -1621,12 +1913,12 @@ int fit_groups_dev(cpb_ctx* ctx, const cpb_psf* psf, const cpb_sim_params* P, in
             su.go.sp_rule = d_rule;
             su.go.sp_rw = (double*)scratch(ctx, "grp_sp_rw", sizeof(double) * 2 * su.C.sp_box * su.n_stars);
         }
-        int32_t* d_list = (int32_t*)scratch(ctx, "grp_list", sizeof(int32_t) * nk);
-        int* d_queue = (int*)scratch(ctx, "grp_queue", sizeof(int) * plan.buckets.size());
+        int32_t* d_list = (int32_t*)scratch(ctx, "grp_list", sizeof(int32_t) * 2 * nk);  // and the deferred groups
+        int* d_queue = (int*)scratch(ctx, "grp_queue", sizeof(int) * kQueueInts * plan.buckets.size());
         check(cudaMemcpyAsync(d_list, lists.data(), sizeof(int32_t) * nk, cudaMemcpyHostToDevice, st), "h2d");
         int64_t at = 0;
         for (size_t b = 0; b < plan.buckets.size(); ++b) {
-            launch_bucket(ctx, st, su, plan.buckets[b], d_list + at, d_queue + b, 0, 0);
+            launch_bucket(ctx, st, su, plan.buckets[b], d_list + at, d_list + nk + at, d_queue + kQueueInts * b, 0, 0);
             at += (int64_t)plan.buckets[b].groups.size();
         }
         launch_spread(ctx, st, su, d_list, nk);
@@ -1750,8 +2042,8 @@ int fit_groups_dev(cpb_ctx* ctx, const cpb_psf* psf, const cpb_sim_params* P, in
 // ---------------------------------------------------------------------------
 struct GroupBatch {
     GroupSetup su;
-    int32_t* d_list = nullptr;  // owned: every bucket's groups back to back
-    int* d_queue = nullptr;     // owned: one counter per bucket
+    int32_t* d_list = nullptr;  // owned: every bucket's groups back to back, then as much for deferred ones
+    int* d_queue = nullptr;     // owned: kQueueInts counters per bucket
     std::vector<int64_t> at;    // first list entry of each bucket
     std::vector<int> threads;   // chosen block size per bucket
     double* sp_buf = nullptr;   // owned: spread_model rule and the stars' residual / weight planes
@@ -1784,8 +2076,8 @@ GroupBatch* group_batch_create(cpb_ctx* ctx, const cpb_psf* psf, const cpb_sim_p
             b->threads.push_back(B.threads);
             lists.insert(lists.end(), B.groups.begin(), B.groups.end());
         }
-        if (cudaMalloc(&b->d_list, sizeof(int32_t) * std::max<size_t>(lists.size(), 1)) != cudaSuccess ||
-            cudaMalloc(&b->d_queue, sizeof(int) * std::max<size_t>(plan.buckets.size(), 1)) != cudaSuccess) {
+        if (cudaMalloc(&b->d_list, sizeof(int32_t) * std::max<size_t>(2 * lists.size(), 1)) != cudaSuccess ||
+            cudaMalloc(&b->d_queue, sizeof(int) * kQueueInts * std::max<size_t>(plan.buckets.size(), 1)) != cudaSuccess) {
             cudaGetLastError();
             throw OomError{"device memory exhausted allocating the group work queues"};
         }
@@ -1822,8 +2114,8 @@ void group_batch_enqueue(cpb_ctx* ctx, GroupBatch* b, cudaStream_t st, int bucke
     const auto& bks = b->su.plan.buckets;
     for (int k = 0; k < (int)bks.size(); ++k) {
         if (bucket >= 0 && k != bucket) continue;
-        launch_bucket(ctx, st, b->su, bks[k], b->d_list + b->at[k], b->d_queue + k,
-                      threads > 0 ? threads : b->threads[k], 0);
+        launch_bucket(ctx, st, b->su, bks[k], b->d_list + b->at[k], b->d_list + b->su.plan.n_kernel + b->at[k],
+                      b->d_queue + kQueueInts * k, threads > 0 ? threads : b->threads[k], 0);
     }
     if (bucket < 0) launch_spread(ctx, st, b->su, b->d_list, group_batch_size(b));
 }
@@ -1831,7 +2123,7 @@ void group_batch_enqueue(cpb_ctx* ctx, GroupBatch* b, cudaStream_t st, int bucke
 void group_batch_set_threads(GroupBatch* b, int bucket, int threads) { b->threads[bucket] = valid_threads(threads); }
 int group_batch_threads(const GroupBatch* b, int bucket) { return b->threads[bucket]; }
 int group_batch_occupancy(GroupBatch* b, int bucket, int threads) {
-    return group_occupancy(b->su.plan.buckets[bucket], threads);
+    return group_occupancy(b->su.plan.buckets[bucket], threads, group_node(b->su.dp));
 }
 int64_t group_batch_size(const GroupBatch* b) { return b->su.plan.n_kernel; }
 

@@ -7,9 +7,10 @@
 // in shared memory:
 //
 //   * the union U of the stars' fit-box pixels (_touched_pixels, :329-335),
-//     sorted in the group image's column-major order, with data_work, w, the
-//     weighted residual and the LSQR u vector per pixel of U -- the reference's
-//     npix-long vectors are zero outside U, so nothing else is kept;
+//     sorted in the group image's column-major order, with the weighted
+//     residual and the LSQR u vector per pixel of U (data_work and sqrt(w) in
+//     the block's slice of global memory) -- the reference's npix-long vectors
+//     are zero outside U, so nothing else is kept;
 //   * per pixel of U, bit masks of the (Morton-ordered) active stars whose fit
 //     box and model box contain it.  J v, the renders and the frozen-star
 //     subtraction are gathers over those bits in ascending (Morton) order,
@@ -92,6 +93,7 @@ struct GroupOut {
     double* residual;
     int32_t *n_passes, *n_failed, *status, *error_kind, *n_active, *n_union, *n_trials, *n_lsqr;
     double *spread, *spread_err;
+    double* px;             // a block: data_work and sqrt(w) of its group's union, 2 umax doubles
     double* sp_rw;          // per star: residual and weight over its box, 2 sp_box doubles (spread_model)
     const double* sp_rule;  // kSpreadRuleLen doubles (spread_rule)
 };
@@ -118,7 +120,7 @@ struct Layout {
     size_t coef, ns, theta, delta, dsc, cn, D, bsc, xl, vt, wl;
     size_t ay, ax, act, frozen, live, conv, newf;
     size_t V, uidx;
-    size_t dw, sw, wr, u, upix, fmask, mmask;
+    size_t wr, u, upix, fmask, mmask;
     size_t total;
 };
 
@@ -157,8 +159,6 @@ __host__ __device__ inline Layout make_layout(int nmax, int S2, int umax, int ke
     if (vbytes < (size_t)4 * keyn) vbytes = (size_t)4 * keyn;
     L.V = take(vbytes);
     L.uidx = take((size_t)2 * nmax * S2);
-    L.dw = take((size_t)8 * umax);
-    L.sw = take((size_t)8 * umax);
     L.wr = take((size_t)8 * umax);
     L.u = take((size_t)8 * umax);
     L.upix = take((size_t)4 * umax);
@@ -246,6 +246,33 @@ __device__ __forceinline__ void psf_grad(const DevPsf& P, const StarCoef& c, int
     model_grad<double, double>(P, P.data64, c, (double)gy, (double)gx, g);
 }
 
+// sym_givens in the steps that lanes can share: tangent lo / hi, sign() / sqrt(1 + t^2),
+// hi over that; the same operations on the same operands.
+struct Rotation {
+    double a, b, hi, lo;
+    __device__ __forceinline__ Rotation(double a_, double b_) : a(a_), b(b_) {
+        const bool swap = fabs(b) > fabs(a);
+        hi = swap ? b : a;
+        lo = swap ? a : b;
+    }
+    __device__ __forceinline__ double sign() const { return sgn(hi); }
+    __device__ __forceinline__ void finish(double t, double q, double r, double& c, double& s, double& rho) const {
+        const bool swap = fabs(b) > fabs(a);
+        c = swap ? q * t : q;
+        s = swap ? q : q * t;
+        rho = r;
+        if (b == 0) {
+            c = (a == 0) ? 1.0 : sgn(a);
+            s = 0;
+            rho = fabs(a);
+        } else if (a == 0) {
+            c = 0;
+            s = sgn(b);
+            rho = fabs(b);
+        }
+    }
+};
+
 // One group's fit by one block.  What bounds it: latency -- a group is a few hundred to
 // two thousand pixels, so every step is a short dependent chain between block barriers.
 // Hence two resident 256-thread blocks an SM (see plan_tiers); per-star cubic weights
@@ -254,7 +281,7 @@ __device__ __forceinline__ void psf_grad(const DevPsf& P, const StarCoef& c, int
 // tests and the update of x and w on warp 0 while the other warps already gather the next
 // J v.  4,000 groups of 2-12 stars measured on the
 // B200: 13.6 ms with one block an SM, generic stencils and three barriers an iteration,
-// 9.6 ms now; 60 Gaussian groups 421 and 349 us.
+// 7.2 ms now; 60 Gaussian groups 421 and 350 us.
 template <int NT, typename MaskT, bool NODE>
 struct GroupFit {
     static constexpr int NW = NT / 32;
@@ -268,6 +295,7 @@ struct GroupFit {
     GView G;
     char* smem;
     Layout L;
+    double *dw, *sw;  // data_work and sqrt(w) of the union, in global memory: read in order, once a render
     double* sh;       // 64 doubles of reduction scratch
     int* s_stop;      // 2 flags, used in turn
     int flip = 0;
@@ -363,7 +391,6 @@ struct GroupFit {
         const int p = C.p, S2 = C.S2, R = C.R;
         double* V = dp(L.V);
         const uint16_t* ui = hp(L.uidx);
-        const double* sw = dp(L.sw);
         double* cn = dp(L.cn);
         const uint8_t* live = bp(L.live);
         for (int a = wid; a < n_act; a += NW) {
@@ -460,8 +487,6 @@ struct GroupFit {
     // a = active slot a); `freeze`: data_work -= model (frozen-star subtraction) instead.
     __device__ double render(bool freeze, MaskT sel, double* to) {
         const MaskT* mm = mp(L.mmask);
-        double* dw = dp(L.dw);
-        const double* sw = dp(L.sw);
         double part = 0.0;
         for (int u = threadIdx.x; u < nU; u += NT) {
             int gy, gx;
@@ -597,7 +622,8 @@ struct GroupFit {
             return 0;
         }
         double inv_alpha = 1.0 / alpha;
-        double wnorm2 = 0.0;
+        double wnorm2 = 0.0, c1 = 0, s1 = 0, rhobar1 = 0;
+        const double lambda = sqrt(lam);
         if (wid == 0) {
             part = 0.0;
             for (int i = lane; i < n; i += 32) {
@@ -605,12 +631,12 @@ struct GroupFit {
                 wl[i] = v;
                 part += v * v;
             }
-            wnorm2 = warp_sum(part);
+            wnorm2 = __shfl_sync(0xffffffffu, warp_sum(part), 0);
+            sym_givens(alpha, lambda, c1, s1, rhobar1);
         }
         __syncthreads();
-        const double lambda = sqrt(lam);
-        double Anorm2 = a2, dNorm2 = 0, xNorm2 = 0, c2 = -1, s2 = 0, z = 0, xENorm2 = 0, res2 = 0;
-        double rhobar = alpha, phibar = beta1, inv_beta = inv_b1;
+        double Anorm2 = a2, dNorm2 = 0, xNorm2 = 0, c2 = -1, s2 = 0, xENorm2 = 0, res2 = 0, rhs = 0, gamma = 1;
+        double phibar = beta1, inv_beta = inv_b1;
         double err_vec[5] = {0, 0, 0, 0, 0};
         const double atol = C.linear_tol, btol = C.linear_tol;
         const double axtol = 1.4901161193847656e-08, etol = axtol, ctol = axtol;
@@ -633,16 +659,41 @@ struct GroupFit {
                     Anorm2 = Anorm2 + alpha_old * alpha_old + beta * beta;
                     if (lambda > 0) Anorm2 += lambda * lambda;
                 }
-                double c1, s1, rhobar1;
-                sym_givens(rhobar, lambda, c1, s1, rhobar1);
+                // An FP64 division or root is a chain of 150-250 cycles, and an iteration has 28
+                // of them.  The independent ones go to different lanes of one instruction,
+                // which leaves 8 in a row (6,000 -> 4,900 cycles an iteration beside the
+                // other warps of two blocks an SM): lane k's operands below, results by shuffle.
                 const double psi = s1 * phibar;
                 phibar = c1 * phibar;
+                Rotation g2(rhobar1, beta);
+                // z of the iteration before (lane 1) beside this rotation's tangent (the rest)
+                double d = (lane == 1 ? rhs : g2.lo) / (lane == 1 ? gamma : g2.hi);
+                const double z = __shfl_sync(0xffffffffu, d, 1);
+                xNorm2 = xNorm2 + z * z;
                 double c, s, rho;
-                sym_givens(rhobar1, beta, c, s, rho);
+                {
+                    const double t = __shfl_sync(0xffffffffu, d, 0);
+                    const double q = g2.sign() / sqrt(1.0 + t * t);
+                    g2.finish(t, q, g2.hi / q, c, s, rho);
+                }
                 const double phi = c * phibar;
                 phibar = s * phibar;
-                const double theta = s * alpha;
-                const double sigma = phi / rho, tr = -theta / rho;
+                const double theta = s * alpha, tau = s * phi;
+                const double delta = s2 * rho, gambar = -c2 * rho;
+                rhs = phi - delta * z;
+                // lane 4: the rotation of (gambar, theta); lane 5: the next iteration's of
+                // (rhobar, lambda); lanes 0-3: sigma, the w factor, |w|^2 / rho^2, zbar
+                Rotation g3(lane == 4 ? gambar : -c * alpha, lane == 4 ? theta : lambda);
+                const bool rot = lane == 4 || lane == 5;
+                {
+                    const double num = rot ? g3.lo : (lane == 1 ? -theta : (lane == 2 ? wnorm2 : (lane == 3 ? rhs : phi)));
+                    const double den = rot ? g3.hi : (lane == 2 ? rho * rho : (lane == 3 ? gambar : rho));
+                    d = num / den;
+                }
+                const double tan3 = d;
+                const double sigma = __shfl_sync(0xffffffffu, d, 0), tr = __shfl_sync(0xffffffffu, d, 1);
+                dNorm2 = dNorm2 + __shfl_sync(0xffffffffu, d, 2);
+                const double zbar = __shfl_sync(0xffffffffu, d, 3);
                 part = 0.0;
                 for (int i = lane; i < n; i += 32) {
                     const double wi = wl[i];
@@ -651,7 +702,7 @@ struct GroupFit {
                     wl[i] = wn;
                     part += wn * wn;
                 }
-                const double wn2 = warp_sum(part);
+                wnorm2 = __shfl_sync(0xffffffffu, warp_sum(part), 0);
                 xENorm2 = xENorm2 + phi * phi;
                 double e2 = 0;
 #pragma unroll
@@ -659,36 +710,52 @@ struct GroupFit {
                     if (k == iter % 5) err_vec[k] = phi;
                     e2 += err_vec[k] * err_vec[k];
                 }
-                const double err_lbnd = iter >= 5 ? sqrt(e2) : 0.0;
-                const double tau = s * phi;
-                dNorm2 = dNorm2 + wnorm2 / (rho * rho);
-                const double delta = s2 * rho;
-                const double gambar = -c2 * rho;
-                const double rhs = phi - delta * z;
-                const double zbar = rhs / gambar;
-                const double xNorm = sqrt(xNorm2 + zbar * zbar);
-                double gamma;
-                sym_givens(gambar, theta, c2, s2, gamma);
-                z = rhs / gamma;
-                xNorm2 = xNorm2 + z * z;
-                const double Anorm = sqrt(Anorm2);
-                const double Acond = Anorm * sqrt(dNorm2);
                 const double res1 = phibar * phibar;
                 res2 = res2 + psi * psi;
-                const double rNorm = sqrt(res1 + res2);
+                d = sqrt(rot         ? 1.0 + tan3 * tan3
+                         : lane == 1 ? dNorm2
+                         : lane == 2 ? res1 + res2
+                         : lane == 3 ? e2
+                         : lane == 6 ? Anorm2
+                         : lane == 7 ? xENorm2
+                                     : xNorm2 + zbar * zbar);
+                const double xNorm = __shfl_sync(0xffffffffu, d, 0);
+                const double rNorm = __shfl_sync(0xffffffffu, d, 2);
+                const double err_lbnd = __shfl_sync(0xffffffffu, d, 3);
+                const double Anorm = __shfl_sync(0xffffffffu, d, 6);
+                const double Acond = Anorm * __shfl_sync(0xffffffffu, d, 1);
+                const double xENorm = __shfl_sync(0xffffffffu, d, 7);
                 const double ArNorm = alpha * fabs(tau);
-                const double test1 = rNorm / beta1;
-                const double test2 = ArNorm / (Anorm * rNorm);
-                const double test3 = 1.0 / Acond;
-                const double t1 = test1 / (1.0 + Anorm * xNorm / beta1);
-                const double rNormtol = btol + axtol * Anorm * xNorm / beta1;
+                {
+                    const double num = rot         ? g3.sign()
+                                       : lane == 1 ? ArNorm
+                                       : lane == 2 ? 1.0
+                                       : lane == 3 ? Anorm * xNorm
+                                       : lane == 6 ? axtol * Anorm * xNorm
+                                                   : rNorm;
+                    const double den = rot ? d : (lane == 1 ? Anorm * rNorm : (lane == 2 ? Acond : beta1));
+                    d = num / den;
+                }
+                const double q3 = d;
+                const double test1 = __shfl_sync(0xffffffffu, d, 0);
+                const double test2 = __shfl_sync(0xffffffffu, d, 1);
+                const double test3 = __shfl_sync(0xffffffffu, d, 2);
+                const double xrel = __shfl_sync(0xffffffffu, d, 3);
+                const double rNormtol = btol + __shfl_sync(0xffffffffu, d, 6);
+                d = (rot ? g3.hi : test1) / (rot ? q3 : 1.0 + xrel);
+                const double t1 = __shfl_sync(0xffffffffu, d, 0);
+                double cr, sr, rr;
+                g3.finish(tan3, q3, d, cr, sr, rr);
+                c2 = __shfl_sync(0xffffffffu, cr, 4);
+                s2 = __shfl_sync(0xffffffffu, sr, 4);
+                gamma = __shfl_sync(0xffffffffu, rr, 4);
+                c1 = __shfl_sync(0xffffffffu, cr, 5);
+                s1 = __shfl_sync(0xffffffffu, sr, 5);
+                rhobar1 = __shfl_sync(0xffffffffu, rr, 5);
                 const bool ill = (1.0 + test3 <= 1.0) || (test3 <= ctol);
                 const bool zr = (1.0 + t1 <= 1.0) || (test1 <= rNormtol);
-                const bool fwd = iter >= 5 && err_lbnd <= etol * sqrt(xENorm2);
+                const bool fwd = iter >= 5 && err_lbnd <= etol * xENorm;
                 const bool solved = (1.0 + test2 <= 1.0) || (test2 <= axtol) || (ArNorm <= atol) || zr || fwd;
-                rhobar = -c * alpha;
-                wnorm2 = wn2;
-                // lane 0's: wnorm2 above is complete there only
                 if (lane == 0) s_stop[it & 1] = solved || ill;
             }
             part = 0.0;
@@ -728,6 +795,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_groups(GroupConst C, DevPsf P,
     F.L = make_layout<MaskT>(C.nmax, C.S2, C.umax, C.keyn, NODE, C.same);
     F.sh = sh;
     F.s_stop = s_stop;
+    F.dw = O.px + (size_t)blockIdx.x * 2 * C.umax;
+    F.sw = F.dw + C.umax;
     F.G.in = in;
     F.G.eltype = C.eltype;
     const int p = C.p, S = C.S, S2 = C.S2, R = C.R;
@@ -1077,16 +1146,14 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_groups(GroupConst C, DevPsf P,
         }
         // per pixel of U: data_work, w and the star masks
         {
-            double* dw = F.dp(F.L.dw);
-            double* swv = F.dp(F.L.sw);
             MaskT* fm = F.mp(F.L.fmask);
             MaskT* mm = F.mp(F.L.mmask);
             for (int u = tid; u < nU; u += NT) {
                 const int q = upix[u];
                 double d, w;
                 F.G.data_w(q, d, w);
-                dw[u] = d;
-                swv[u] = sqrt(w);
+                F.dw[u] = d;
+                F.sw[u] = sqrt(w);
                 int gy, gx;
                 F.uxy(u, gy, gx);
                 MaskT f = 0, mo = 0;
@@ -1390,8 +1457,9 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_groups(GroupConst C, DevPsf P,
 // the group's disk into shared memory, its width from the first catalogue
 // star's final parameters; each warp renders its star's model stamp over the
 // fit box and correlates it with the disk one component at a time (x pass, then
-// the y pass added into the correlated stamp), all in its own 3 sp_box doubles
-// of shared memory, and sums against the residual and weight planes k_groups
+// the y pass added into the correlated stamp; boxes up to kLine px in register
+// lines, spread_lines_warp), all in its own stamp and two planes of shared
+// memory, and sums against the residual and weight planes k_groups
 // saved for the star.  Kept out of k_groups so that the fit's register
 // allocation does not carry it.
 __global__ void __launch_bounds__(128) k_group_spread(GroupConst C, DevPsf P, GroupIn in, GroupOut O,
@@ -1403,9 +1471,13 @@ __global__ void __launch_bounds__(128) k_group_spread(GroupConst C, DevPsf P, Gr
     const int nw = blockDim.x >> 5, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     double* tab = sm;
     double* pan = tab + ((C.sp_tab + 1) & ~1);
-    double* M = pan + (7 + kh) * kSpreadGL + (size_t)wid * 3 * box;  // the warp's model stamp
-    double* T = M + box;                                             // one component's x pass
-    double* Gs = T + box;                                            // the disk-correlated stamp
+    const bool lines = spread_lines_fit(kh);
+    const int ld = lines ? spread_plane(box, kh) : box;
+    double* M = pan + (7 + kh) * kSpreadGL + (size_t)wid * (box + 2 * ld);  // the warp's model stamp
+    double* T = M + box;                                                   // one component's x pass
+    double* Gs = T + ld;                                                   // the disk-correlated stamp
+    PPNode N;
+    const bool one_node = node_of(P, N);
     DevPsf Ps = P;
     Ps.fwhm = C.sp_psf_fwhm;  // _spread_fwhm renders the PSF object's own width
     for (int li = blockIdx.x; li < nlist; li += gridDim.x) {
@@ -1435,11 +1507,20 @@ __global__ void __launch_bounds__(128) k_group_spread(GroupConst C, DevPsf P, Gr
             const double* Rr = O.sp_rw + (size_t)o * 2 * box;
             const double* Wt = Rr + box;
             __syncwarp();  // the warp's previous stamp is no longer read
-            for (int e = lane; e < nb; e += 32) {
-                M[e] = psf_value(P, c, ylo + e % h, xlo + e / h);
-                Gs[e] = 0.0;
+            const unsigned hmag = quot_magic((unsigned)h);
+            if (one_node) {
+                NodeStar<false> S;
+                S.set(N, c.y, c.x, ylo, xlo, h, wd);
+                for (int e = lane; e < nb; e += 32) {
+                    int r;
+                    const int col = quot(e, h, hmag, r);
+                    M[e] = c.flux * S.value(N, N.pp, r, col) + c.bkg;
+                }
+            } else {
+                for (int e = lane; e < nb; e += 32) M[e] = psf_value(P, c, ylo + e % h, xlo + e / h);
             }
-            for (int cc = 0; cc < 6; ++cc) {
+            if (lines) spread_lines_warp(D, D.I, M, T, Gs, h | 1, h, wd);
+            for (int cc = 0; cc < 6 && !lines; ++cc) {
                 const int L = D.L[cc];
                 const double* I = D.I + cc * n + kh;
                 __syncwarp();
@@ -1456,10 +1537,11 @@ __global__ void __launch_bounds__(128) k_group_spread(GroupConst C, DevPsf P, Gr
                     const int p0 = max(-L, -r), p1 = min(L, h - 1 - r);
                     double t = 0.0;
                     for (int p = p0; p <= p1; ++p) t += I[p] * T[r + p + col * h];
-                    Gs[e] += D.alpha[cc] * t;
+                    Gs[e] = (cc ? Gs[e] : 0.0) + D.alpha[cc] * t;
                 }
             }
             __syncwarp();
+            const int pad = lines ? (h | 1) - h : 0;  // of a Gs column
             const double inv_flux = 1.0 / c.flux;
             double Sp = 0, Sq = 0, Sp0 = 0, Sq0 = 0, SqG = 0;
             for (int e = lane; e < nb; e += 32) {
@@ -1469,7 +1551,8 @@ __global__ void __launch_bounds__(128) k_group_spread(GroupConst C, DevPsf P, Gr
                     const double Pp = (mv - c.bkg) * inv_flux;
                     const double wP = wp * Pp;
                     const double p_i = Rr[e] + mv - c.bkg;
-                    const double g_i = (Gs[e] - c.bkg) * inv_flux;
+                    int r;
+                    const double g_i = (Gs[e + pad * quot(e, h, hmag, r)] - c.bkg) * inv_flux;
                     Sp += wP * p_i;
                     Sq += wp * g_i * p_i;
                     Sp0 += wP * Pp;
@@ -1571,6 +1654,9 @@ size_t layout_bytes(const GroupConst& C, int nmax, int umax, int keyn, bool node
 
 // The bucket's launches.  One block of the layout for the largest group an SM leaves its
 // schedulers 80 % idle (4,000 groups of 2-12 stars, 152 KB: 12.3 ms, 20 % of issue slots).
+// With data_work and sqrt(w) in global memory (read in order, once a render) two blocks of
+// 12-star groups of 13 px boxes fit; with both in shared memory 40 % of those groups were
+// deferred and the batch took 9.6 ms instead of 7.2.
 // The union of a blend's boxes is usually well below the bound its layout allows for, so
 // where two such blocks do not fit an SM, the groups of up to `nA` stars run first with a
 // layout of half an SM: its union capacity is what is left beside the stars' arrays, at
@@ -1711,7 +1797,7 @@ void setup_groups(cpb_ctx* ctx, const cpb_psf* psf, const cpb_sim_params* P, int
                      out->n_iter, out->chisq, out->qfit, out->qfit_expected, out->qfit_z, out->crowding,
                      out->residual, out->n_passes, out->n_failed, out->status, out->error_kind, out->n_active,
                      out->n_union, out->n_trials, out->n_lsqr_iters, out->spread_model, out->spread_model_err,
-                     nullptr, nullptr};
+                     nullptr, nullptr, nullptr};
     if (G == 0) return;
     // group sizes on the host (plan the shared-memory layout, route oversized groups)
     std::vector<int64_t>& h_off = su.h_off;
@@ -1748,10 +1834,11 @@ void setup_groups(cpb_ctx* ctx, const cpb_psf* psf, const cpb_sim_params* P, int
     su.n_stars = h_soff[G];
     if (C.sp_on) {
         // k_group_spread: the disk table and one panel of the quadrature, then
-        // 3 sp_box doubles a warp; up to 4 warps within 96 KB, else fewer; a fit
+        // the stamp and two planes a warp (3 sp_box doubles or a little more); up to 4 warps within 96 KB, else fewer; a fit
         // box beyond shared memory even for one warp leaves spread_model NaN
         const size_t fixed = ((size_t)((C.sp_tab + 1) & ~1) + (size_t)(7 + C.R) * kSpreadGL) * sizeof(double);
-        const size_t per_warp = (size_t)3 * C.sp_box * sizeof(double);
+        const size_t per_warp =
+            (C.sp_box + 2 * (size_t)(spread_lines_fit(C.R) ? spread_plane(C.sp_box, C.R) : C.sp_box)) * sizeof(double);
         int nw = 4;
         while (nw > 1 && fixed + nw * per_warp > 96 * 1024) --nw;
         if (fixed + nw * per_warp > cap) C.sp_on = 0;
@@ -1830,6 +1917,20 @@ int tier_occupancy(const Bucket& B, const Tier& T, int threads, bool node) {
     int per_sm = 0;
     check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, threads, T.smem), "occupancy");
     return std::max(per_sm, 1);
+}
+// Doubles of the blocks' union arrays (GroupOut::px) for any block size of any launch.
+size_t group_px_doubles(const cpb_ctx* ctx, const GroupSetup& su) {
+    size_t most = 0;
+    const bool node = group_node(su.dp);
+    for (const Bucket& B : su.plan.buckets)
+        for (const Tier* T : {&B.half, &B.full})
+            for (int t = 64; t <= 256; t *= 2)
+                if (T->C.umax) {
+                    const int64_t grid = std::min<int64_t>((int64_t)B.groups.size(),
+                                                           (int64_t)ctx->n_sm * tier_occupancy(B, *T, t, node));
+                    most = std::max(most, (size_t)2 * T->C.umax * (size_t)grid);
+                }
+    return most;
 }
 int group_occupancy(const Bucket& B, int threads, bool node) {
     return tier_occupancy(B, B.half.n ? B.half : B.full, valid_threads(threads), node);
@@ -1913,6 +2014,7 @@ int fit_groups_dev(cpb_ctx* ctx, const cpb_psf* psf, const cpb_sim_params* P, in
             su.go.sp_rule = d_rule;
             su.go.sp_rw = (double*)scratch(ctx, "grp_sp_rw", sizeof(double) * 2 * su.C.sp_box * su.n_stars);
         }
+        su.go.px = (double*)scratch(ctx, "grp_px", sizeof(double) * group_px_doubles(ctx, su));
         int32_t* d_list = (int32_t*)scratch(ctx, "grp_list", sizeof(int32_t) * 2 * nk);  // and the deferred groups
         int* d_queue = (int*)scratch(ctx, "grp_queue", sizeof(int) * kQueueInts * plan.buckets.size());
         check(cudaMemcpyAsync(d_list, lists.data(), sizeof(int32_t) * nk, cudaMemcpyHostToDevice, st), "h2d");
@@ -2046,6 +2148,7 @@ struct GroupBatch {
     int* d_queue = nullptr;     // owned: kQueueInts counters per bucket
     std::vector<int64_t> at;    // first list entry of each bucket
     std::vector<int> threads;   // chosen block size per bucket
+    double* px = nullptr;       // owned: the blocks' union arrays
     double* sp_buf = nullptr;   // owned: spread_model rule and the stars' residual / weight planes
 };
 
@@ -2085,6 +2188,12 @@ GroupBatch* group_batch_create(cpb_ctx* ctx, const cpb_psf* psf, const cpb_sim_p
             check(cudaMemcpy(b->d_list, lists.data(), sizeof(int32_t) * lists.size(), cudaMemcpyHostToDevice),
                   "h2d");
         GroupSetup& su = b->su;
+        if (cudaMalloc(&b->px, sizeof(double) * std::max<size_t>(plan.buckets.empty() ? 0 : group_px_doubles(ctx, su), 1)) !=
+            cudaSuccess) {
+            cudaGetLastError();
+            throw OomError{"device memory exhausted allocating the groups' pixel arrays"};
+        }
+        su.go.px = b->px;
         if (su.C.sp_on && !plan.buckets.empty()) {
             const size_t n_rule = kSpreadRuleLen, n_rw = (size_t)2 * su.C.sp_box * su.n_stars;
             if (cudaMalloc(&b->sp_buf, sizeof(double) * (n_rule + n_rw)) != cudaSuccess) {
@@ -2099,6 +2208,7 @@ GroupBatch* group_batch_create(cpb_ctx* ctx, const cpb_psf* psf, const cpb_sim_p
         }
     } catch (...) {
         cudaFree(b->sp_buf);
+        cudaFree(b->px);
         cudaFree(b->d_list);
         cudaFree(b->d_queue);
         delete b;
@@ -2141,6 +2251,7 @@ std::string group_batch_signature(const GroupBatch* b, int bucket) {
 void group_batch_destroy(GroupBatch* b) {
     if (!b) return;
     cudaFree(b->sp_buf);
+    cudaFree(b->px);
     cudaFree(b->d_list);
     cudaFree(b->d_queue);
     delete b;

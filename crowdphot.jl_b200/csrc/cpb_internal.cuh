@@ -672,8 +672,10 @@ inline size_t spread_smem_bytes(int mode, int boxmax, int kh) {
            : mode == 1 ? ((size_t)7 * boxmax + prof) * sizeof(double)
                        : (mode == 2 ? (size_t)3 * boxmax * sizeof(double) : 0);
 }
+// Boxes and supports of the line form (a warp a star).
+__host__ __device__ inline bool spread_lines_fit(int kh) { return 2 * kh + 2 <= kLine && kh <= kLineL; }
 inline int spread_mode(int boxmax, int kh, int64_t n_stars, int n_sm) {
-    if (2 * kh + 2 <= kLine && kh <= kLineL && n_stars > (int64_t)kDiagFew * n_sm) return 3;
+    if (spread_lines_fit(kh) && n_stars > (int64_t)kDiagFew * n_sm) return 3;
     if (spread_smem_bytes(1, boxmax, kh) <= 200 * 1024) return 1;
     if (spread_smem_bytes(2, boxmax, kh) <= 200 * 1024) return 2;
     return 0;

@@ -246,33 +246,6 @@ __device__ __forceinline__ void psf_grad(const DevPsf& P, const StarCoef& c, int
     model_grad<double, double>(P, P.data64, c, (double)gy, (double)gx, g);
 }
 
-// sym_givens in the steps that lanes can share: tangent lo / hi, sign() / sqrt(1 + t^2),
-// hi over that; the same operations on the same operands.
-struct Rotation {
-    double a, b, hi, lo;
-    __device__ __forceinline__ Rotation(double a_, double b_) : a(a_), b(b_) {
-        const bool swap = fabs(b) > fabs(a);
-        hi = swap ? b : a;
-        lo = swap ? a : b;
-    }
-    __device__ __forceinline__ double sign() const { return sgn(hi); }
-    __device__ __forceinline__ void finish(double t, double q, double r, double& c, double& s, double& rho) const {
-        const bool swap = fabs(b) > fabs(a);
-        c = swap ? q * t : q;
-        s = swap ? q : q * t;
-        rho = r;
-        if (b == 0) {
-            c = (a == 0) ? 1.0 : sgn(a);
-            s = 0;
-            rho = fabs(a);
-        } else if (a == 0) {
-            c = 0;
-            s = sgn(b);
-            rho = fabs(b);
-        }
-    }
-};
-
 // One group's fit by one block.  What bounds it: latency -- a group is a few hundred to
 // two thousand pixels, so every step is a short dependent chain between block barriers.
 // Hence two resident 256-thread blocks an SM (see plan_tiers); per-star cubic weights

@@ -34,6 +34,33 @@ __device__ __forceinline__ void sym_givens(double a, double b, double& c, double
     }
 }
 
+// sym_givens in the steps that lanes can share: tangent lo / hi, sign() / sqrt(1 + t^2),
+// hi over that; the same operations on the same operands.
+struct Rotation {
+    double a, b, hi, lo;
+    __device__ __forceinline__ Rotation(double a_, double b_) : a(a_), b(b_) {
+        const bool swap = fabs(b) > fabs(a);
+        hi = swap ? b : a;
+        lo = swap ? a : b;
+    }
+    __device__ __forceinline__ double sign() const { return sgn(hi); }
+    __device__ __forceinline__ void finish(double t, double q, double r, double& c, double& s, double& rho) const {
+        const bool swap = fabs(b) > fabs(a);
+        c = swap ? q * t : q;
+        s = swap ? q : q * t;
+        rho = r;
+        if (b == 0) {
+            c = (a == 0) ? 1.0 : sgn(a);
+            s = 0;
+            rho = fabs(a);
+        } else if (a == 0) {
+            c = 0;
+            s = sgn(b);
+            rho = fabs(b);
+        }
+    }
+};
+
 // Per-star p x p covariance from the Gram block (:1305-1329,
 // levenberg_marquardt.jl:366-388): ridge 1e-12 tr, Cholesky inverse,
 // Jacobi pseudo-inverse fallback, reweighted scaling by cost/dof.

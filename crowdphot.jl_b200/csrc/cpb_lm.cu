@@ -733,6 +733,42 @@ __device__ __forceinline__ bool chol_factor_t(const double* A, double* U, double
         }
     return true;
 }
+// A x = b with a division at every use, as psf_fitting.jl's solves divide: the chained
+// fits' form (CHAIN below).
+template <int NF>
+__device__ __forceinline__ bool chol_solve_t(const double* A, const double* b, double* x) {
+    double U[NF * NF];
+#pragma unroll
+    for (int j = 0; j < NF; ++j)
+#pragma unroll
+        for (int i = 0; i <= j; ++i) {
+            double s = A[i + j * NF];
+#pragma unroll
+            for (int k = 0; k < i; ++k) s -= U[k + i * NF] * U[k + j * NF];
+            if (i == j) {
+                if (!(s > 0)) return false;
+                U[j + j * NF] = sqrt(s);
+            } else {
+                U[i + j * NF] = s / U[i + i * NF];
+            }
+        }
+    double y[NF];
+#pragma unroll
+    for (int i = 0; i < NF; ++i) {
+        double s = b[i];
+#pragma unroll
+        for (int k = 0; k < i; ++k) s -= U[k + i * NF] * y[k];
+        y[i] = s / U[i + i * NF];
+    }
+#pragma unroll
+    for (int i = NF - 1; i >= 0; --i) {
+        double s = y[i];
+#pragma unroll
+        for (int k = i + 1; k < NF; ++k) s -= U[i + k * NF] * x[k];
+        x[i] = s / U[i + i * NF];
+    }
+    return true;
+}
 template <int NF>
 __device__ __forceinline__ void chol_back_t(const double* U, const double* Ri, const double* b, double* x) {
     double y[NF];
@@ -760,6 +796,98 @@ __device__ __forceinline__ double pick(const double* v, int idx) {
     for (int q = 0; q < N; ++q) r = (q == idx) ? v[q] : r;
     return r;
 }
+
+// The star model pixel by pixel, from the pixel's own grid coordinate and with the
+// interpolation polynomial in differences (corner_eval's operations): the chained fits'
+// form.  A cursor keeps the stencil's row offsets while the lane's next pixel moves by
+// whole oversampling periods, which is always but for a rounding at a sample.
+// SMEM: row-phase copy 2, else the polyphase copy (as in NodeStar).
+template <bool SMEM>
+struct TapCursor {
+    int ly = 0, lx = 0;  // stencil origin of the lane's previous pixel (0: none)
+    int ry[4], cx[4];
+
+    // offsets of the four taps from 0-based padded sample i0 on: sample i lies at
+    // (i % is) * pstride + (i / is) * qstride
+    static __device__ __forceinline__ void taps(int i0, int is, int pstride, int qstride, int* t) {
+        int q = i0 / is, r = i0 - q * is;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            t[k] = r * pstride + q * qstride;
+            if (++r == is) {
+                r = 0;
+                ++q;
+            }
+        }
+    }
+    // Profile s and, with GRAD, dsdY = -sy dp/dv and dsdX = -sx dp/du of pixel (py, px) for a
+    // star at (Y, X).  (di, dj): how far the cutout row / column moved since the last call.
+    template <bool GRAD>
+    __device__ __forceinline__ void profile(const PPNode& N, const double* pp, int di, int dj, double Y, double X,
+                                            double py, double px, double& s, double& dY, double& dX) {
+        const DevNode& nd = N.nd;
+        const double u = nd.sx * (px - X) + nd.ox;
+        const double v = nd.sy * (py - Y) + nd.oy;
+        const int nyd = nd.ny, nxd = nd.nx;
+        // NaN and infinite u, v fail these range tests, as isfinite would
+        const bool inb = u >= 1.0 && u <= (double)nxd && v >= 1.0 && v <= (double)nyd;
+        if (!inb) {
+            s = nd.fill;
+            dY = 0.0;
+            dX = 0.0;
+            ly = lx = 0;
+            return;
+        }
+        const int kx = clampi((int)floor(u), 1, nxd - 1);
+        const int ky = clampi((int)floor(v), 1, nyd - 1);
+        const double du = u - (double)kx, dv = v - (double)ky;
+        const int qy = SMEM ? nd.RPX : 1;
+        if (ly != 0 && ky == ly + nd.isy * di) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) ry[k] += di * qy;
+        } else {
+            taps(ky - 1, nd.isy, SMEM ? nd.RPY[2] * nd.RPX : N.plane, qy, ry);
+        }
+        if (!SMEM) {
+            if (lx != 0 && kx == lx + nd.isx * dj) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) cx[k] += dj * nd.LPY;
+            } else {
+                taps(kx - 1, nd.isx, nd.isy * N.plane, nd.LPY, cx);
+            }
+        }
+        ly = ky;
+        lx = kx;
+        double row[4], drow[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const double* q = pp + ry[r] + (SMEM ? kx - 1 : 0);
+            const double a = q[SMEM ? 0 : cx[0]], b = q[SMEM ? 1 : cx[1]], c = q[SMEM ? 2 : cx[2]],
+                         e = q[SMEM ? 3 : cx[3]];
+            const double k1 = (c - a) / 2;
+            const double k4 = c - b - k1;
+            const double k2 = 3 * k4 - (e - b) / 2 + k1;
+            const double k3 = k4 - k2;
+            row[r] = du * (du * (du * k3 + k2) + k1) + b;
+            if (GRAD) drow[r] = du * (3 * du * k3 + 2 * k2) + k1;
+        }
+        const double v1 = (row[2] - row[0]) / 2;
+        const double v4 = row[2] - row[1] - v1;
+        const double v2 = 3 * v4 - (row[3] - row[1]) / 2 + v1;
+        const double v3 = v4 - v2;
+        s = dv * (dv * (dv * v3 + v2) + v1) + row[1];
+        if (GRAD) {
+            const double pdv = dv * (3 * dv * v3 + 2 * v2) + v1;
+            const double u1 = (drow[2] - drow[0]) / 2;
+            const double u4 = drow[2] - drow[1] - u1;
+            const double u2 = 3 * u4 - (drow[3] - drow[1]) / 2 + u1;
+            const double u3 = u4 - u2;
+            const double pdu = dv * (dv * (dv * u3 + u2) + u1) + drow[1];
+            dY = -(nd.sy * pdv);
+            dX = -(nd.sx * pdu);
+        }
+    }
+};
 
 // A cutout is fitted by a team of WPC warps (1: one warp a cutout, the
 // throughput form for large batches; 4: a 128-thread team, the latency form for
@@ -810,7 +938,17 @@ __device__ __forceinline__ void stage_async(TI* dst, const TI* src) {
 
 // ID: the free parameters are the first NF (L.fidx[k] == k), so only their entries
 // are summed; otherwise all NP are and the free ones picked at the end.
-template <typename TI, int NP, int NF, bool SMEM, int WPC, bool ID>
+// CHAIN: the fits of fit_all_stars, where each star's data are what the fits before it
+// left of the image.  Every rounding of a bright star's model is in its neighbours' data,
+// and ill-conditioned fits and quotients by a flux that ends near zero (qfit,
+// spread_model_err) enlarge it by up to 1e8: with the constant weights, the scaled
+// derivatives and the reciprocal solve of the single fits those quotients moved by 2e-9 of
+// their norm on a three-pass 1024^2 field, more than the 1e-9 an FP64 result is held to.  So the chain keeps one order of
+// operations: the per-pixel profile (TapCursor), sums over the rectangle of pixels at most
+// one beyond the table, (w g_p) g_q products and divided solves.  Its sums say themselves
+// where a product is rounded before it is added (left to the compiler, that changed with
+// the code around them).
+template <typename TI, int NP, int NF, bool SMEM, int WPC, bool ID, bool CHAIN>
 __device__ double lm_accum_t(const PPNode& N, const double* pp, const LMConst& L, const TI* pix,
                              const TI* iv, int ny, int nx, int y1, int x1, int qs, int rs,
                              const double* fv, double* A, double* b, double* red) {
@@ -830,11 +968,22 @@ __device__ double lm_accum_t(const PPNode& N, const double* pp, const LMConst& L
         const double r = mval - d;
         double w = 1.0;
         if (iv) w = (isfinite(vv) && vv > 0) ? vv : 0.0;
-        const double wr = w * r;
-        cost = wr * r + cost;
+        const double wr = CHAIN ? __dmul_rn(w, r) : w * r;
+        cost = CHAIN ? __fma_rn(wr, r, cost) : wr * r + cost;
         int t = 0;
 #pragma unroll
         for (int q = 0; q < NA; ++q) {
+            if constexpr (CHAIN) {
+                const bool one = q == NP - 1;  // the background: gv = 1
+                bf[q] = one ? __dadd_rn(wr, bf[q]) : __fma_rn(wr, gv[q], bf[q]);
+#pragma unroll
+                for (int pq = 0; pq <= q; ++pq) {
+                    const double wg = __dmul_rn(w, gv[pq]);
+                    Af[t] = one ? __dadd_rn(wg, Af[t]) : __fma_rn(wg, gv[q], Af[t]);
+                    ++t;
+                }
+                continue;
+            }
             bf[q] = wr * gv[q] + bf[q];
             const double wg = w * gv[q];
 #pragma unroll
@@ -863,7 +1012,7 @@ __device__ double lm_accum_t(const PPNode& N, const double* pp, const LMConst& L
             gv[2] = -2 * Ag * (1 + gp * sq) / fwhm;
             gv[3] = g / norm;
             gv[NP - 1] = 1.0;
-            acc((double)pix[e], iv ? (double)iv[e] : 1.0, amp * g + bkg, gv);
+            acc((double)pix[e], iv ? (double)iv[e] : 1.0, CHAIN ? __dadd_rn(Ag, bkg) : amp * g + bkg, gv);
             i += r32;
             j += q32;
             if (i >= ny) {
@@ -874,51 +1023,91 @@ __device__ double lm_accum_t(const PPNode& N, const double* pp, const LMConst& L
     } else {
         const DevNode& nd = N.nd;
         const double Y = fv[0], X = fv[1], flux = fv[2], bkg = fv[3];
-        NodeStar<SMEM> T;
-        T.set(N, Y, X, y1, x1, ny, nx);
-        // the derivatives by Y and X carry -flux * oversampling: in the weights
-        {
-            const double fy = -(flux * nd.sy), fx = -(flux * nd.sx);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                T.dy[k] *= fy;
-                T.dx[k] *= fx;
-            }
-        }
         // pixels outside [ilo, ihi] x [jlo, jhi] are beyond the table: the fill value
         // with zero derivatives
-        const int ilo = T.sy.lo, ihi = T.sy.hi, jlo = T.sx.lo, jhi = T.sx.hi;
-        const int ni = ihi - ilo + 1, nj = jhi - jlo + 1;
-        if (ni > 0 && nj > 0) {
-            const int nr = ni * nj, rq = TS / ni, rr = TS % ni;
-            int i = ilo + lane % ni, j = jlo + lane / ni;
-            // the next pixel's data and weight load behind this one's arithmetic
-            double dn = 0.0, vn = 1.0;
-            if (lane < nr) {
-                dn = (double)pix[i + j * ny];
-                if (iv) vn = (double)iv[i + j * ny];
+        int ilo, ihi, jlo, jhi, ni, nj;
+        if constexpr (CHAIN) {
+            ilo = 0, ihi = ny - 1, jlo = 0, jhi = nx - 1;
+            if (isfinite(Y) && isfinite(X)) {
+                const double ya = Y - (double)y1 + (1.0 - nd.oy) / nd.sy;
+                const double yb = Y - (double)y1 + ((double)nd.ny - nd.oy) / nd.sy;
+                const double xa = X - (double)x1 + (1.0 - nd.ox) / nd.sx;
+                const double xb = X - (double)x1 + ((double)nd.nx - nd.ox) / nd.sx;
+                ilo = (int)fmin(fmax(0.0, floor(ya) - 1.0), (double)ny);
+                ihi = (int)fmax(fmin((double)(ny - 1), ceil(yb) + 1.0), -1.0);
+                jlo = (int)fmin(fmax(0.0, floor(xa) - 1.0), (double)nx);
+                jhi = (int)fmax(fmin((double)(nx - 1), ceil(xb) + 1.0), -1.0);
             }
-            for (int k = lane; k < nr; k += TS) {
-                const double d = dn, vv = vn;
-                const int ic = i, jc = j;
-                i += rr;
-                j += rq;
-                if (i > ihi) {
-                    i -= ni;
-                    ++j;
+            ni = ihi - ilo + 1;
+            nj = jhi - jlo + 1;
+            if (ni > 0 && nj > 0) {
+                const int nr = ni * nj, rq = TS / ni, rr = TS % ni;
+                int ii = lane % ni, jj = lane / ni, di = 0, dj = 0;
+                TapCursor<SMEM> T;
+                for (int k = lane; k < nr; k += TS) {
+                    const int i = ilo + ii, j = jlo + jj, e = i + j * ny;
+                    double s, dY, dX;
+                    T.template profile<true>(N, pp, di, dj, Y, X, (double)(y1 + i), (double)(x1 + j), s, dY, dX);
+                    const double gv[4] = {flux * dY, flux * dX, s, 1.0};
+                    acc((double)pix[e], iv ? (double)iv[e] : 1.0, __fma_rn(flux, s, bkg), gv);
+                    ii += rr;
+                    jj += rq;
+                    di = rr;
+                    dj = rq;
+                    if (ii >= ni) {
+                        ii -= ni;
+                        ++jj;
+                        di -= ni;
+                        ++dj;
+                    }
                 }
-                if (k + TS < nr) {
+            }
+        } else {
+            NodeStar<SMEM> T;
+            T.set(N, Y, X, y1, x1, ny, nx);
+            // the derivatives by Y and X carry -flux * oversampling: in the weights
+            {
+                const double fy = -(flux * nd.sy), fx = -(flux * nd.sx);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    T.dy[k] *= fy;
+                    T.dx[k] *= fx;
+                }
+            }
+            ilo = T.sy.lo, ihi = T.sy.hi, jlo = T.sx.lo, jhi = T.sx.hi;
+            ni = ihi - ilo + 1;
+            nj = jhi - jlo + 1;
+            if (ni > 0 && nj > 0) {
+                const int nr = ni * nj, rq = TS / ni, rr = TS % ni;
+                int i = ilo + lane % ni, j = jlo + lane / ni;
+                // the next pixel's data and weight load behind this one's arithmetic
+                double dn = 0.0, vn = 1.0;
+                if (lane < nr) {
                     dn = (double)pix[i + j * ny];
                     if (iv) vn = (double)iv[i + j * ny];
                 }
-                double rv[4], rd[4], gv[4];
-                T.template rows<true>(pp, ic, jc, rv, rd);
-                const double s = T.wy[0] * rv[0] + T.wy[1] * rv[1] + T.wy[2] * rv[2] + T.wy[3] * rv[3];
-                gv[0] = T.dy[0] * rv[0] + T.dy[1] * rv[1] + T.dy[2] * rv[2] + T.dy[3] * rv[3];
-                gv[1] = T.wy[0] * rd[0] + T.wy[1] * rd[1] + T.wy[2] * rd[2] + T.wy[3] * rd[3];
-                gv[2] = s;
-                gv[3] = 1.0;
-                acc(d, vv, flux * s + bkg, gv);
+                for (int k = lane; k < nr; k += TS) {
+                    const double d = dn, vv = vn;
+                    const int ic = i, jc = j;
+                    i += rr;
+                    j += rq;
+                    if (i > ihi) {
+                        i -= ni;
+                        ++j;
+                    }
+                    if (k + TS < nr) {
+                        dn = (double)pix[i + j * ny];
+                        if (iv) vn = (double)iv[i + j * ny];
+                    }
+                    double rv[4], rd[4], gv[4];
+                    T.template rows<true>(pp, ic, jc, rv, rd);
+                    const double s = T.wy[0] * rv[0] + T.wy[1] * rv[1] + T.wy[2] * rv[2] + T.wy[3] * rv[3];
+                    gv[0] = T.dy[0] * rv[0] + T.dy[1] * rv[1] + T.dy[2] * rv[2] + T.dy[3] * rv[3];
+                    gv[1] = T.wy[0] * rd[0] + T.wy[1] * rd[1] + T.wy[2] * rd[2] + T.wy[3] * rd[3];
+                    gv[2] = s;
+                    gv[3] = 1.0;
+                    acc(d, vv, flux * s + bkg, gv);
+                }
             }
         }
         if (ni < ny || nj < nx) {
@@ -987,10 +1176,10 @@ __device__ double lm_accum_t(const PPNode& N, const double* pp, const LMConst& L
 
 // covariance! (levenberg_marquardt.jl:366-388) for compile-time NF; the pinv
 // fallback is the general one.
-template <int NF>
+template <int NF, bool CHAIN>
 __device__ void lm_cov_t(const double* A, double* cov) {
     double U[NF * NF], Ri[NF], e[NF], x[NF];
-    if (!chol_factor_t<NF>(A, U, Ri)) {
+    if (!CHAIN && !chol_factor_t<NF>(A, U, Ri)) {
         lm_cov(A, NF, cov);
         return;
     }
@@ -998,7 +1187,14 @@ __device__ void lm_cov_t(const double* A, double* cov) {
     for (int c = 0; c < NF; ++c) {
 #pragma unroll
         for (int i = 0; i < NF; ++i) e[i] = (i == c) ? 1.0 : 0.0;
-        chol_back_t<NF>(U, Ri, e, x);
+        if constexpr (CHAIN) {
+            if (!chol_solve_t<NF>(A, e, x)) {
+                lm_cov(A, NF, cov);
+                return;
+            }
+        } else {
+            chol_back_t<NF>(U, Ri, e, x);
+        }
 #pragma unroll
         for (int i = 0; i < NF; ++i) cov[i + c * NF] = x[i];
     }
@@ -1019,7 +1215,7 @@ struct LMState {
 // next candidate; returns true when the fit is over.  Every thread of the team
 // computes the same values; its first thread (lane 0) stores them.  lm_irls,
 // levenberg_marquardt.jl:478-680.
-template <int NP, int NF, int WPC>
+template <int NP, int NF, int WPC, bool CHAIN>
 __device__ __forceinline__ bool lm_step(LMState<NP, NF>& S, const LMConst& L, double cost_c, const double* Ac,
                                         const double* bc, int lane) {
     double fv[NP], x[NF], A[NF * NF], b[NF], D[NF];
@@ -1098,7 +1294,9 @@ __device__ __forceinline__ bool lm_step(LMState<NP, NF>& S, const LMConst& L, do
         bool gsmall = true;  // the largest gradient cosine is within g_tol (false with a NaN)
 #pragma unroll
         for (int k = 0; k < NF; ++k)
-            gsmall = gsmall && fabs(b[k]) <= L.g_tol * (sqrt(A[k + k * NF] * cost) + 2.220446049250313e-16);
+            gsmall = gsmall &&
+                     (CHAIN ? fabs(b[k]) / (sqrt(A[k + k * NF] * cost) + 2.220446049250313e-16) <= L.g_tol
+                            : fabs(b[k]) <= L.g_tol * (sqrt(A[k + k * NF] * cost) + 2.220446049250313e-16));
         if (gsmall) {
             gconv = conv = 1;
             done = true;
@@ -1115,11 +1313,14 @@ __device__ __forceinline__ bool lm_step(LMState<NP, NF>& S, const LMConst& L, do
             for (int k = 0; k < NF; ++k) Ad[k + k * NF] += lam;
         }
         double U[NF * NF], Ri[NF];
-        if (!chol_factor_t<NF>(Ad, U, Ri)) {
+        bool solved;
+        if constexpr (CHAIN) solved = chol_solve_t<NF>(Ad, b, d);
+        else solved = chol_factor_t<NF>(Ad, U, Ri);
+        if (!solved) {
             lam = fmin(lam * L.lambda_up, L.lambda_max);
             continue;
         }
-        chol_back_t<NF>(U, Ri, b, d);
+        if constexpr (!CHAIN) chol_back_t<NF>(U, Ri, b, d);
 #pragma unroll
         for (int k = 0; k < NF; ++k) d[k] = -d[k];
         double db = 0, dAd = 0;
@@ -1186,7 +1387,7 @@ static_assert(kLMThreads % 256 == 0, "half a block must still hold whole 128-thr
 // parameters, fixed ones replaced by L.fixv).  Returns 0 with the result in S,
 // or CPB_ERR_ARGUMENT when the inputs fail _prepare_fit_star_inputs's checks
 // (psf_fitting.jl:61-90) or lm_irls's dof test (:461-467).
-template <typename TI, int NP, int NF, bool SMEM, int WPC, bool ID>
+template <typename TI, int NP, int NF, bool SMEM, int WPC, bool ID, bool CHAIN>
 __device__ int lm_team_fit(const PPNode& N, const double* pp, const LMConst& L, const TI* pix,
                            const TI* iv, int ny, int nx, int y1, int x1, const double* init,
                            LMState<NP, NF>& S, double* red, int lane, unsigned char* stage, int stage_bytes) {
@@ -1240,8 +1441,9 @@ __device__ int lm_team_fit(const PPNode& N, const double* pp, const LMConst& L, 
         double fc[NP], Ac[NF * NF], bc[NF];
 #pragma unroll
         for (int q = 0; q < NP; ++q) fc[q] = S.fc[q];
-        const double cost_c = lm_accum_t<TI, NP, NF, SMEM, WPC, ID>(N, pp, L, pix, iv, ny, nx, y1, x1, qs, rs, fc, Ac, bc, red);
-        if (lm_step<NP, NF, WPC>(S, L, cost_c, Ac, bc, lane)) break;
+        const double cost_c =
+            lm_accum_t<TI, NP, NF, SMEM, WPC, ID, CHAIN>(N, pp, L, pix, iv, ny, nx, y1, x1, qs, rs, fc, Ac, bc, red);
+        if (lm_step<NP, NF, WPC, CHAIN>(S, L, cost_c, Ac, bc, lane)) break;
     }
     return 0;
 }
@@ -1286,9 +1488,9 @@ __global__ void __launch_bounds__(kLMThreads, 1) k_lm_t(int64_t n_cut, LMConst L
         const int64_t c = (int64_t)cc;
         const int ny = cny[c], nx = cnx[c];
         const int64_t o = (ny > 0 && nx > 0) ? offs[c] : 0;
-        const int st = lm_team_fit<TI, NP, NF, SMEM, WPC, ID>(N, pp, L, pixels + o, ivs ? ivs + o : nullptr, ny, nx, cy1[c],
-                                                    cx1[c], init + c * NP, S, red, lane,
-                                                    (unsigned char*)(node_smem + N.nel) + team * stage_bytes, stage_bytes);
+        const int st = lm_team_fit<TI, NP, NF, SMEM, WPC, ID, false>(
+            N, pp, L, pixels + o, ivs ? ivs + o : nullptr, ny, nx, cy1[c], cx1[c], init + c * NP, S, red, lane,
+            (unsigned char*)(node_smem + N.nel) + team * stage_bytes, stage_bytes);
         if (st != 0) {
             if (lane == 0) out.status[c] = st;
             team_sync<WPC>();
@@ -1299,7 +1501,7 @@ __global__ void __launch_bounds__(kLMThreads, 1) k_lm_t(int64_t n_cut, LMConst L
             const double cost = S.cost;
             if (out.cov) {
                 double cov[NF * NF];
-                lm_cov_t<NF>(S.A, cov);
+                lm_cov_t<NF, false>(S.A, cov);
                 const double f = L.reweighted ? cost / dof : 1.0;
 #pragma unroll
                 for (int k = 0; k < NF * NF; ++k) out.cov[c * NF * NF + k] = cov[k] * f;
@@ -1340,9 +1542,10 @@ __global__ void __launch_bounds__(kLMThreads, 1) k_lm_t(int64_t n_cut, LMConst L
 constexpr long long kDagSpinLimit = 1ll << 26;  // default: ~64 M polls of >= 64 ns before a team gives up
 // Warps of one team: 4 measured fastest on a 2048^2 field when each pixel worked its own
 // weights out (34.6 ms for three passes, against 58.2 ms with 1 and 41.0 ms with 8).
-// With the star's weights, staged cutouts and fewer divisions in the serial steps, three
-// passes over 12,500 stars of a 1024^2 field take 8.4 ms, from 12.9 (bound by the chain
-// of overlapping stars, one fit's latency a link).
+// With the cutouts staged in shared memory and the staged node's row-phase copy, three
+// passes over 12,500 stars of a 1024^2 field take 10.3 ms, from 12.9 (bound by the chain
+// of overlapping stars, one fit's latency a link; 8.4 ms with the single fits' constant
+// weights, whose roundings the chain cannot take: CHAIN above).
 constexpr int kDagWarps = 4;
 
 template <typename TIV, int NP, int NF, bool SMEM, bool ID>
@@ -1402,34 +1605,46 @@ __global__ void __launch_bounds__(kLMThreads, 1) k_mp_dag(LMConst L, PPNode N, D
         const int4 b = A.box[k];
         const int nb = b.z * b.w;
         const double* pin = A.pin + (int64_t)k * np;
-        // a star's model over its box: the staged node's weights once a star
-        NodeStar<SMEM> T;
-        double mflux = 0.0, mbkg = 0.0;
-        auto model_of = [&](const double* pr) {
-            if (NP != 4) return;
-            T.set(N, pr[0], pr[1], b.x, b.y, b.z, b.w);
-            mflux = pr[2];
-            mbkg = pr[3];
+        // a star's model at pixel (i, j) of the image; (di, dj) as in TapCursor
+        TapCursor<SMEM> T;
+        auto model_at = [&](const double* pr, int i, int j, int di, int dj) {
+            if (NP != 4) return mp_model(P, A.M, pr, i, j);
+            double s, dY, dX;
+            T.template profile<false>(N, pp, di, dj, pr[0], pr[1], (double)i, (double)j, s, dY, dX);
+            return __dadd_rn(__dmul_rn(pr[2], s), pr[3]);
         };
-        auto model_at = [&](const double* pr, int i, int j) {
-            return NP == 4 ? mflux * T.value(N, pp, i, j) + mbkg : mp_model(P, A.M, pr, b.x + i, b.y + j);
+        // the lane's pixels e = lane, lane + TS, ... of the box: f(e, image row, column, di, dj)
+        auto box_walk = [&](auto f) {
+            const int rq = TS / b.z, rr = TS % b.z;
+            int i = lane % b.z, j = lane / b.z, di = 0, dj = 0;
+            for (int e = lane; e < nb; e += TS) {
+                f(e, b.x + i, b.y + j, di, dj);
+                i += rr;
+                j += rq;
+                di = rr;
+                dj = rq;
+                if (i >= b.z) {
+                    i -= b.z;
+                    ++j;
+                    di -= b.z;
+                    ++dj;
+                }
+            }
         };
         // passes 2+: the previous model back in (:360-365), and the cutout
-        if (A.pass > 1) model_of(pin);
-        for (int e = lane; e < nb; e += TS) {
-            const int i = b.x + e % b.z, j = b.y + e / b.z;
+        box_walk([&](int e, int i, int j, int di, int dj) {
             const int64_t q = (i - 1) + (int64_t)(j - 1) * A.ny;
             double r = __ldcg(A.resid + q);
             if (A.pass > 1) {
-                r = r + model_at(pin, i - b.x, j - b.y);
+                r = r + model_at(pin, i, j, di, dj);
                 __stcg(A.resid + q, r);
             }
             cpix[e] = r;
             if (civ) civ[e] = (double)ivimg[q];
-        }
+        });
         team_sync<WPC>();
-        const int st = lm_team_fit<double, NP, NF, SMEM, WPC, ID>(N, pp, L, cpix, civ, b.z, b.w, b.x, b.y, pin, S, red, lane,
-                                                                     nullptr, 0);
+        const int st = lm_team_fit<double, NP, NF, SMEM, WPC, ID, true>(N, pp, L, cpix, civ, b.z, b.w, b.x, b.y, pin, S,
+                                                                        red, lane, nullptr, 0);
         // bookkeeping (:373-401)
         const int64_t s = A.idx[k];
         double* ps = A.psub + (int64_t)k * np;
@@ -1442,7 +1657,7 @@ __global__ void __launch_bounds__(kLMThreads, 1) k_mp_dag(LMConst L, PPNode N, D
             } else {
                 const double dof = (double)((int64_t)nb - NF);
                 double cov[NF * NF];
-                lm_cov_t<NF>(S.A, cov);
+                lm_cov_t<NF, true>(S.A, cov);
                 const double f = L.reweighted ? S.cost / dof : 1.0;
                 for (int q = 0; q < np; ++q) {
                     A.prm[s * np + q] = S.fv[q];
@@ -1461,14 +1676,13 @@ __global__ void __launch_bounds__(kLMThreads, 1) k_mp_dag(LMConst L, PPNode N, D
             double pr[NP];
 #pragma unroll
             for (int q = 0; q < NP; ++q) pr[q] = ps[q];
-            model_of(pr);
-            for (int e = lane; e < nb; e += TS) {
-                const int i = b.x + e % b.z, j = b.y + e / b.z;
+            T.ly = T.lx = 0;
+            box_walk([&](int e, int i, int j, int di, int dj) {
                 const int64_t q = (i - 1) + (int64_t)(j - 1) * A.ny;
-                const double r = __ldcg(A.resid + q) - model_at(pr, i - b.x, j - b.y);
+                const double r = __ldcg(A.resid + q) - model_at(pr, i, j, di, dj);
                 __stcg(A.resid + q, r);
                 if (A.snap) A.snap[A.snap_off[k] + e] = r;
-            }
+            });
         } else if (A.snap) {
             for (int e = lane; e < nb; e += TS) {
                 const int i = b.x + e % b.z, j = b.y + e / b.z;

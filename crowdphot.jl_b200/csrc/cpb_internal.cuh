@@ -1009,6 +1009,13 @@ inline void check(cudaError_t e, const char* what) {
     if (e != cudaSuccess) throw CudaError{e, what};
 }
 
+// Lets `kern` ask for `bytes` of dynamic shared memory.  Without it a block may have 48 KB
+// with the kernel's static arrays included, so the limit is set at every size.
+template <typename K>
+void allow_smem(K kern, size_t bytes) {
+    check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), "smem attr");
+}
+
 struct ArgError {
     std::string msg;
 };

@@ -653,8 +653,7 @@ int fit_all_stars_dev(cpb_ctx* ctx, const cpb_psf* psf, const cpb_lm_params* P, 
     }
     const size_t diag_smem = spread_smem_bytes(smode, boxmax, sd.kh);
     auto diag_attr = [&](auto kern) {
-        if (diag_smem > 48 * 1024)
-            check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)diag_smem), "smem attr");
+        allow_smem(kern, diag_smem);
     };
     if (smode == 3) diag_attr(k_mp_diag<double, true>), diag_attr(k_mp_diag<float, true>);
     else diag_attr(k_mp_diag<double, false>), diag_attr(k_mp_diag<float, false>);

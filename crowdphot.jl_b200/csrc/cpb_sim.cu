@@ -2348,8 +2348,7 @@ void launch_overlapped(void (*kern)(KA...), unsigned grid, int threads, size_t s
 template <bool GRAD, typename TS, bool GRAM = false, typename... A>
 void launch_eval_warp(bool plan, unsigned grid, unsigned thr, size_t smem, cudaStream_t st, A... args) {
     auto go = [&](auto kern) {
-        if (smem > 48 * 1024)
-            check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attr");
+        allow_smem(kern, smem);
         kern<<<grid, thr, smem, st>>>(args...);
     };
     if (plan) go(k_eval_warp<GRAD, TS, true, GRAM>);
@@ -2370,7 +2369,7 @@ void launch_eval_node(const DevPsf& dp, const DevNode& nd, int n_sm, cudaStream_
     constexpr int GH = Gran<T>::H, CP = GH == 2 ? 0 : 1;
     const size_t smem = sizeof(T) * (size_t)((GH * nd.isy * nd.RPY[CP] * nd.RPX + 3) / 4 * 4);
     auto go = [&](auto kern) {
-        check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attr");
+        allow_smem(kern, smem);
         const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(nlist, n_sm));
         kern<<<grid, NodeThreads<T, GRAD>::N, smem, st>>>(list, nlist, fc, nd, rpp_host<T>(dp) + nd.rpoff[CP], args...);
     };
@@ -2381,8 +2380,7 @@ void launch_eval_node(const DevPsf& dp, const DevNode& nd, int n_sm, cudaStream_
 template <bool GRAD, typename T, typename... A>
 void launch_k_eval(int64_t S2, unsigned grid, size_t smem, cudaStream_t st, A... args) {
     auto go = [&](auto kern, int threads) {
-        if (smem > 48 * 1024)
-            check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attr");
+        allow_smem(kern, smem);
         kern<<<grid, threads, smem, st>>>(args...);
     };
     if (S2 <= 256)
@@ -3546,9 +3544,7 @@ void SimFit::finish() {
                         (double)n_act * boxmax * (8.0 + (d_inv_var ? 2.0 : 1.0) * (eltype == CPB_F64 ? 8 : 4)));
         auto go = [&](auto kern, auto ti) {
             using TI = decltype(ti);
-            if (diag_smem > 48 * 1024)
-                check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)diag_smem),
-                      "smem attr");
+            allow_smem(kern, diag_smem);
             kern<<<dgrid, spread_threads(smode), diag_smem, st>>>(n_act, fc, dp, P->fit_rad, coef, resid,
                                                                   (const TI*)d_image, (const TI*)d_background,
                                                                   (const TI*)d_inv_var, d_stab, kh, smode, boxmax,

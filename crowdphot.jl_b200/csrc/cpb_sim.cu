@@ -2504,6 +2504,18 @@ namespace {
 // is not used before the final pass.
 bool radii_in_spread_tab(int R_cap, int R) { return R_cap + 2 <= spread_tab_len(R); }
 
+// Blocks of the J^T u kernel: eight stars each (a warp a star), at most 8 an SM.
+constexpr int64_t kJtMaxBlocks = 2048;
+int64_t jt_grid(int64_t n, int n_sm) {
+    return std::max<int64_t>(1, std::min({(n + 7) / 8, (int64_t)n_sm * 8, kJtMaxBlocks}));
+}
+// Blocks of the largest kernel that reduces over its grid: a gather's regions, the
+// per-parameter kernels or J^T u, whose grid is the largest of them where more than one
+// star falls on 32 pixels.
+int64_t reduce_blocks(int64_t n, int64_t npix, int64_t ntiles) {
+    return std::max({ntiles, (int64_t)nblk(std::max<int64_t>(n * 3, npix)) + 1, jt_grid(n, (int)kJtMaxBlocks)});
+}
+
 // Bytes arena_carve reserves for one named buffer of `bytes`.
 size_t carve_size(size_t bytes) { return (std::max<size_t>(bytes, 256) + 255) & ~size_t(255); }
 
@@ -2575,7 +2587,7 @@ size_t sim_scratch_bound(const cpb_sim_params* P, int64_t ny, int64_t nx, int64_
     const int64_t ntiles = ((ny + TY - 1) / TY) * ((nx + TX - 1) / TX);
     const int64_t np = (int64_t)p * n;
     size_t b = 2 * carve_size(sizeof(Scalars));                                    // scalars, scalars_freeze
-    b += carve_size(8 * std::max<int64_t>(ntiles, nblk(std::max<int64_t>(n * 3, npix)) + 1)) + carve_size(4);
+    b += carve_size(8 * reduce_blocks(n, npix, ntiles)) + carve_size(4);            // red_partials, red_counter
     b += 4 * carve_size(8 * npix) + carve_size(16);                                // data, data_work, w, sw, flags
     b += 2 * carve_size(4 * n) + carve_size(n) + carve_size(8 * n);                // ay_c, ax_c, ok, key
     b += 2 * carve_size(4 * n) + 2 * carve_size(8 * n) + carve_size(4 * n) + carve_size(4);  // iota .. nsel
@@ -3000,8 +3012,7 @@ bool SimFit::setup() {
     // device-resident scalars and reducers
     sc = S_<Scalars>("scalars", 1);
     check(cudaMemsetAsync(sc, 0, sizeof(Scalars), st), "memset");
-    const int64_t max_blocks = std::max<int64_t>(ntiles, nblk(std::max<int64_t>(n_stars * 3, npix)) + 1);
-    red = Reducer{S_<double>("red_partials", max_blocks), S_<unsigned>("red_counter", 1)};
+    red = Reducer{S_<double>("red_partials", reduce_blocks(n_stars, npix, ntiles)), S_<unsigned>("red_counter", 1)};
     check(cudaMemsetAsync(red.counter, 0, sizeof(unsigned), st), "memset");
     h_sc = (Scalars*)ctx->pinned;
 
@@ -3196,7 +3207,7 @@ bool SimFit::setup() {
     warp_eval = dp.kind == CPB_PSF_CIRCULAR_GAUSSIAN || dp.n_nodes == 1;
     if (dp.kind != CPB_PSF_CIRCULAR_GAUSSIAN) node0 = psf->h_nodes[0];
     check(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device), "attr");
-    jt_blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>((n_act + 7) / 8, (int64_t)ctx->n_sm * 8));
+    jt_blocks = (unsigned)jt_grid(n_act, ctx->n_sm);
     lam = P->lambda_init;
     if (ctx->arena) arena_precheck();
     return true;

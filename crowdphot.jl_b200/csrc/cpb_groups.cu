@@ -1886,7 +1886,7 @@ inline int valid_threads(int t) { return t == 64 ? 64 : (t == 128 ? 128 : 256); 
 // Resident blocks per SM of the group kernel with a launch's layout and this block size.
 int tier_occupancy(const Bucket& B, const Tier& T, int threads, bool node) {
     GroupKernel kfn = group_kernel_for(threads, B.wide, node);
-    check(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T.smem), "smem attr");
+    allow_smem(kfn, T.smem);
     int per_sm = 0;
     check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, threads, T.smem), "occupancy");
     return std::max(per_sm, 1);
@@ -1942,8 +1942,7 @@ void launch_bucket(cpb_ctx* ctx, cudaStream_t st, const GroupSetup& su, const Bu
 void launch_spread(cpb_ctx* ctx, cudaStream_t st, const GroupSetup& su, const int32_t* d_list, int64_t nk) {
     if (!su.C.sp_on || nk <= 0) return;
     const int threads = 32 * su.sp_nw;
-    check(cudaFuncSetAttribute(k_group_spread, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)su.sp_smem),
-          "smem attr");
+    allow_smem(k_group_spread, su.sp_smem);
     int per_sm = 0;
     check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_group_spread, threads, su.sp_smem), "occupancy");
     const int64_t grid = std::min<int64_t>(nk, (int64_t)ctx->n_sm * std::max(per_sm, 1));

@@ -1010,10 +1010,24 @@ inline void check(cudaError_t e, const char* what) {
 }
 
 // Lets `kern` ask for `bytes` of dynamic shared memory.  Without it a block may have 48 KB
-// with the kernel's static arrays included, so the limit is set at every size.
-template <typename K>
-void allow_smem(K kern, size_t bytes) {
+// with the kernel's static arrays included, so the limit is set at every size.  The limit
+// belongs to the kernel on its device, whatever context launches it, so it is only ever
+// raised: another thread's context may be about to launch the same kernel with a larger
+// table.
+inline void raise_smem_limit(const void* kern, size_t bytes) {
+    static std::mutex mu;
+    static std::map<std::pair<const void*, int>, size_t> limit;
+    int device = 0;
+    check(cudaGetDevice(&device), "device");
+    std::lock_guard<std::mutex> lk(mu);
+    size_t& top = limit[{kern, device}];
+    if (bytes <= top) return;
     check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), "smem attr");
+    top = bytes;
+}
+template <typename K>
+void allow_smem(K* kern, size_t bytes) {
+    raise_smem_limit((const void*)kern, bytes);
 }
 
 struct ArgError {

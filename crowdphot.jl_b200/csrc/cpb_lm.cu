@@ -1858,8 +1858,7 @@ void launch_lm(cpb_ctx* ctx, const cpb_psf* psf, const LMConst& L, int64_t n_cut
         KernelScope ks_(ctx, "k_lm", bytes);
         auto go = [&](auto ti, auto kern) {
             using TI = decltype(ti);
-            check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes),
-                  "smem attribute");
+            allow_smem(kern, smem_bytes);
             kern<<<blocks, threads, smem_bytes, st>>>(n_cut, L, N, d_off, d_ny, d_nx, d_y1, d_x1, (const TI*)d_pix,
                                                       (const TI*)d_iv, d_init, o, queue, stage_bytes);
         };
@@ -2176,8 +2175,7 @@ void mp_dag_launch(cpb_ctx* ctx, const cpb_psf* psf, const cpb_lm_params* P, int
     const unsigned blocks = (unsigned)ctx->n_sm;  // persistent: every team resident
     KernelScope ks_(ctx, "k_mp_dag", 0.0);
     auto go = [&](auto kern) {
-        check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes),
-              "smem attribute");
+        allow_smem(kern, smem_bytes);
         kern<<<blocks, kLMThreads, smem_bytes, st>>>(L, N, psf->dev, A, stage_bytes);
     };
 #define CPB_DAG_S(TIV, NF, ID)                          \

@@ -340,16 +340,17 @@ __device__ __forceinline__ void ld_gran(const double* p, double (&o)[2]) {
     o[0] = t.x;
     o[1] = t.y;
 }
-// one 16-byte run of a per-pixel vector (reused, read-only for the launch)
+// one 16-byte run of a per-pixel vector (a plain load: the kernel before may still be
+// writing it when this one starts, see overlap_launch)
 __device__ __forceinline__ void ld_px16(const float* p, float (&o)[4]) {
-    const float4 t = __ldg((const float4*)p);
+    const float4 t = *(const float4*)p;
     o[0] = t.x;
     o[1] = t.y;
     o[2] = t.z;
     o[3] = t.w;
 }
 __device__ __forceinline__ void ld_px16(const double* p, double (&o)[2]) {
-    const double2 t = __ldg((const double2*)p);
+    const double2 t = *(const double2*)p;
     o[0] = t.x;
     o[1] = t.y;
 }
@@ -1344,9 +1345,12 @@ constexpr size_t kGatherSmem = (size_t)(NT / 32) * TX * TY * sizeof(double);
 // The kernels of an LSQR iteration depend on one another in turn, and on a small field each
 // is a few microseconds of work behind its launch.  They are launched so that a kernel's
 // blocks may take their places while the one before still runs (launch_overlapped): each
-// first waits here for that one's completion, so nothing is read early.  Whole calls, measured on the
-// B200: 200 Gaussian stars on 256^2 (60 iterations) 3.00 -> 2.73 ms, 1,500 gridded-PSF
-// stars on 500^2 6.00 -> 5.72 ms; fields of 50,000 stars unchanged.
+// first waits here for that one's completion, so nothing is read early.  What such a kernel
+// reads of the kernel before (u, vt, the scalars) is not `const __restrict__` and not read by
+// __ldg: both promise that it is constant from the kernel's start, and allow loads ahead of
+// the wait and from a cache that is not coherent.  Whole calls, measured on the B200: 200
+// Gaussian stars on 256^2 (60 iterations) 3.00 -> 2.73 ms, 1,500 gridded-PSF stars on 500^2
+// 6.00 -> 5.72 ms; fields of 50,000 stars unchanged.
 __device__ __forceinline__ void overlap_launch() {
     cudaGridDependencySynchronize();
     cudaTriggerProgrammaticLaunchCompletion();
@@ -1358,7 +1362,7 @@ __global__ void __launch_bounds__(NT) k_gather(FitConst fc, const int32_t* __res
                                                const int32_t* __restrict__ tord,
                                                const uint8_t* __restrict__ incl, const TS* __restrict__ src,
                                                int Rbox, const int64_t* __restrict__ roff, int64_t src_len,
-                                               const double* __restrict__ vt, const double* __restrict__ cn,
+                                               const double* vt, const double* __restrict__ cn,
                                                const TU* u_src, double u_sign,
                                                TU* outu, double* outd, const uint8_t* __restrict__ umask,
                                                const double* __restrict__ w, const double* __restrict__ sw,
@@ -1592,7 +1596,7 @@ template <bool LSQR, typename TS, typename TU>
 __global__ void __launch_bounds__(256, 4) k_JT(const int32_t* __restrict__ list, int64_t nlist, FitConst fc,
                                             const int32_t* __restrict__ ay, const int32_t* __restrict__ ax,
                                             const TS* __restrict__ V, RectMap vmap, const double* __restrict__ cn,
-                                            const TU* __restrict__ u, double* __restrict__ z, Scalars* sc,
+                                            const TU* u, double* z, Scalars* sc,
                                             Reducer red) {
     static_assert(sizeof(TS) == sizeof(TU), "u granules match stamp granules");
     constexpr int GH = Gran<TS>::H;
@@ -1673,7 +1677,7 @@ __global__ void __launch_bounds__(256, 4) k_JT(const int32_t* __restrict__ list,
                             ld_px16(u + pq, uu[q]);
                         } else {
 #pragma unroll
-                            for (int rr = 0; rr < GH; ++rr) uu[q][rr] = gy + rr < ny ? __ldg(u + pq + rr) : (TU)0;
+                            for (int rr = 0; rr < GH; ++rr) uu[q][rr] = gy + rr < ny ? u[pq + rr] : (TU)0;
                         }
                     }
                     t += 32;

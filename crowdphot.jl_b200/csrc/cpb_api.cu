@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <type_traits>
 #include <set>
 #include <string>
@@ -288,12 +289,57 @@ int cpb_psf_upload(cpb_ctx* ctx, const cpb_psf_desc* d, cpb_psf** out) {
                     slot = k;
                 }
             }
-            std::vector<float> h32(h64.size());
-            for (size_t q = 0; q < h64.size(); ++q) h32[q] = (float)h64[q];
+            // geometry of the copies (DevNode) and their places in one device block (256-byte
+            // aligned pieces).  The edge-padded and row-phase copies are read for single-node
+            // PSFs only, the row-phase ones where they fit the kernels' shared memory.
+            int optin = 0;
+            check(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device), "attr");
+            size_t n_pp = 0, n_lpp = 0, n_row[3] = {0, 0, 0};
+            for (int k = 0; k < nn; ++k) {
+                DevNode& nd = nodes[k];
+                nd.isy = (int32_t)d->node_os[2 * k + 1];
+                nd.isx = (int32_t)d->node_os[2 * k];
+                nd.PY = (nd.ny + nd.isy - 1) / nd.isy;
+                nd.PX = (nd.nx + nd.isx - 1) / nd.isx;
+                nd.LPY = (nd.ny + 3 + nd.isy - 1) / nd.isy;
+                nd.LPX = (nd.nx + 3 + nd.isx - 1) / nd.isx;
+                nd.RPX = (nd.nx + 3) | 1;
+                nd.poff = (int64_t)n_pp;
+                n_pp += ((size_t)nd.PY * nd.PX * nd.isy * nd.isx + 3) / 4 * 4;
+                for (int c = 0; c < 3; ++c) {
+                    const int ph = kRowPhase[c] * nd.isy;
+                    nd.RPY[c] = (nd.ny + 3 + ph - 1) / ph;
+                    if (nn == 1 && row_phase_staged(nd, c, optin)) n_row[c] = row_phase_len(nd, c);
+                }
+                if (nn == 1) n_lpp = ((size_t)nd.LPY * nd.LPX * nd.isy * nd.isx + 3) / 4 * 4;
+            }
+            nodes[0].rpoff[2] = (int64_t)n_row[0];  // copies 0 and 2 share rpp64
+            size_t bytes = 0;
+            auto place = [&](size_t n, size_t size) {
+                const size_t at = bytes;
+                bytes = (at + n * size + 255) & ~size_t(255);
+                return at;
+            };
+            const size_t n64 = h64.size();
+            const size_t o_d64 = place(n64, 8), o_d32 = place(n64, 4), o_pp64 = place(n_pp, 8),
+                         o_pp32 = place(n_pp, 4), o_lpp = place(n_lpp, 8), o_r64 = place(n_row[0] + n_row[2], 8),
+                         o_r32 = place(n_row[1], 4), o_nd = place(nn, sizeof(DevNode)), o_yg = place(yg.size(), 8),
+                         o_xg = place(xg.size(), 8), o_ig = place(ig.size(), 4);
+            std::unique_ptr<char[]> block(new char[bytes]);
+            char* host = block.get();
+            std::memset(host, 0, bytes);
+            std::memcpy(host + o_d64, h64.data(), 8 * n64);
+            std::memcpy(host + o_nd, nodes.data(), sizeof(DevNode) * nn);
+            std::memcpy(host + o_yg, yg.data(), 8 * yg.size());
+            std::memcpy(host + o_xg, xg.data(), 8 * xg.size());
+            std::memcpy(host + o_ig, ig.data(), 4 * ig.size());
+            auto round_all = [](float* to, const double* from, size_t n) {
+                for (size_t q = 0; q < n; ++q) to[q] = (float)from[q];
+            };
+            round_all((float*)(host + o_d32), h64.data(), n64);
             // Offsets of an axis' n entries in a copy that regroups them by their index modulo
             // `ph`, and the samples they come from (before: replicates in front).  Tabulated: a
-            // few divisions an axis instead of four a sample of each copy (preparing a fit with a
-            // 101 x 101-sample image PSF: 2.4 ms with those, 1.8 ms with these).
+            // few divisions an axis instead of four a sample of each copy.
             struct AxisMap {
                 std::vector<int64_t> at, src;
             };
@@ -308,77 +354,43 @@ int cpb_psf_upload(cpb_ctx* ctx, const cpb_psf_desc* d, cpb_psf** out) {
                 return m;
             };
             auto regroup = [&](auto* to, const AxisMap& y, const AxisMap& x, const DevNode& nd) {
-                for (size_t k = 0; k < x.at.size(); ++k)
+                for (size_t k = 0; k < x.at.size(); ++k) {
+                    const double* from = h64.data() + nd.off + x.src[k] * nd.ny;
+                    auto* col = to + x.at[k];
                     for (size_t i = 0; i < y.at.size(); ++i)
-                        to[y.at[i] + x.at[k]] = (std::decay_t<decltype(*to)>)h64[nd.off + y.src[i] + x.src[k] * nd.ny];
+                        col[y.at[i]] = (std::decay_t<decltype(*to)>)from[y.src[i]];
+                }
             };
-            // polyphase copies (DevNode): samples regrouped by oversampling phase
-            std::vector<double> pp;
-            for (int k = 0; k < nn; ++k) {
-                DevNode& nd = nodes[k];
-                nd.isy = (int32_t)d->node_os[2 * k + 1];
-                nd.isx = (int32_t)d->node_os[2 * k];
-                nd.PY = (nd.ny + nd.isy - 1) / nd.isy;
-                nd.PX = (nd.nx + nd.isx - 1) / nd.isx;
-                nd.poff = (int64_t)pp.size();
+            for (const DevNode& nd : nodes) {
                 const int64_t plane = (int64_t)nd.PY * nd.PX;
-                pp.resize(pp.size() + (size_t)(plane * nd.isy * nd.isx + 3) / 4 * 4, 0.0);
-                regroup(pp.data() + nd.poff, axis_map(nd.ny, nd.ny, 0, nd.isy, plane, 1),
+                regroup((double*)(host + o_pp64) + nd.poff, axis_map(nd.ny, nd.ny, 0, nd.isy, plane, 1),
                         axis_map(nd.nx, nd.nx, 0, nd.isx, plane * nd.isy, nd.PY), nd);
             }
-            std::vector<double> lpp;
-            for (int k = 0; k < nn; ++k) {
-                DevNode& nd = nodes[k];
-                nd.LPY = (nd.ny + 3 + nd.isy - 1) / nd.isy;
-                nd.LPX = (nd.nx + 3 + nd.isx - 1) / nd.isx;
-                nd.lpoff = (int64_t)lpp.size();
+            round_all((float*)(host + o_pp32), (const double*)(host + o_pp64), n_pp);
+            if (nn == 1) {
+                const DevNode& nd = nodes[0];
                 const int64_t plane = (int64_t)nd.LPY * nd.LPX;
-                lpp.resize(lpp.size() + (size_t)(plane * nd.isy * nd.isx + 3) / 4 * 4, 0.0);
-                regroup(lpp.data() + nd.lpoff, axis_map(nd.ny + 3, nd.ny, 1, nd.isy, plane, 1),
+                regroup((double*)(host + o_lpp), axis_map(nd.ny + 3, nd.ny, 1, nd.isy, plane, 1),
                         axis_map(nd.nx + 3, nd.nx, 1, nd.isx, plane * nd.isy, nd.LPY), nd);
+                const AxisMap cols = axis_map(nd.nx + 3, nd.nx, 1, nd.nx + 3, 1, 1);
+                for (int c = 0; c < 3; ++c) {
+                    if (!n_row[c]) continue;
+                    const AxisMap rows = axis_map(nd.ny + 3, nd.ny, 1, kRowPhase[c] * nd.isy,
+                                                  (int64_t)nd.RPY[c] * nd.RPX, nd.RPX);
+                    if (c == 1) regroup((float*)(host + o_r32), rows, cols, nd);
+                    else regroup((double*)(host + o_r64) + nd.rpoff[c], rows, cols, nd);
+                }
             }
-            // row-phase copies (DevNode), each node on a 16-byte boundary
-            std::vector<double> rpp;
-            std::vector<float> rpp32, pp32(pp.size());
-            for (int k = 0; k < nn; ++k) {
-                DevNode& nd = nodes[k];
-                nd.RPX = (nd.nx + 3) | 1;
-                auto fill = [&](auto& v, int c, int gh) {
-                    const int ph = gh * nd.isy;
-                    nd.RPY[c] = (nd.ny + 3 + ph - 1) / ph;
-                    nd.rpoff[c] = (int64_t)v.size();
-                    v.resize(v.size() + ((size_t)ph * nd.RPY[c] * nd.RPX + 3) / 4 * 4);
-                    regroup(v.data() + nd.rpoff[c],
-                            axis_map(nd.ny + 3, nd.ny, 1, ph, (int64_t)nd.RPY[c] * nd.RPX, nd.RPX),
-                            axis_map(nd.nx + 3, nd.nx, 1, nd.nx + 3, 1, 1), nd);
-                };
-                fill(rpp, 0, 2);
-                fill(rpp32, 1, 4);
-                fill(rpp, 2, 1);
-            }
-            for (size_t q = 0; q < pp.size(); ++q) pp32[q] = (float)pp[q];
-            // one device block and one copy for every table (256-byte aligned pieces)
-            std::vector<char> blob;
-            auto add = [&](const void* src, size_t bytes) {
-                const size_t at = (blob.size() + 255) & ~size_t(255);
-                blob.resize(at + bytes);
-                std::memcpy(blob.data() + at, src, bytes);
-                return at;
-            };
-            auto addv = [&](const auto& v) { return add(v.data(), sizeof(v[0]) * v.size()); };
-            const size_t o_d64 = addv(h64), o_d32 = addv(h32), o_pp64 = addv(pp), o_pp32 = addv(pp32),
-                         o_lpp = addv(lpp), o_r64 = addv(rpp), o_r32 = addv(rpp32), o_nd = addv(nodes),
-                         o_yg = addv(yg), o_xg = addv(xg), o_ig = addv(ig);
-            check(cudaMalloc(&ps->d_blob, blob.size()), "cudaMalloc");
-            check(cudaMemcpy(ps->d_blob, blob.data(), blob.size(), cudaMemcpyHostToDevice), "h2d");
+            check(cudaMalloc(&ps->d_blob, bytes), "cudaMalloc");
+            check(cudaMemcpy(ps->d_blob, host, bytes, cudaMemcpyHostToDevice), "h2d");
             const char* base = (const char*)ps->d_blob;
             dp.data64 = (const double*)(base + o_d64);
             dp.data32 = (const float*)(base + o_d32);
             dp.pp64 = (const double*)(base + o_pp64);
             dp.pp32 = (const float*)(base + o_pp32);
-            dp.lpp64 = (const double*)(base + o_lpp);
-            dp.rpp64 = (const double*)(base + o_r64);
-            dp.rpp32 = (const float*)(base + o_r32);
+            dp.lpp64 = n_lpp ? (const double*)(base + o_lpp) : nullptr;
+            dp.rpp64 = n_row[0] + n_row[2] ? (const double*)(base + o_r64) : nullptr;
+            dp.rpp32 = n_row[1] ? (const float*)(base + o_r32) : nullptr;
             dp.nodes = (const DevNode*)(base + o_nd);
             dp.ygrid = (const double*)(base + o_yg);
             dp.xgrid = (const double*)(base + o_xg);
@@ -386,14 +398,14 @@ int cpb_psf_upload(cpb_ctx* ctx, const cpb_psf_desc* d, cpb_psf** out) {
             dp.n_nodes = nn;
             dp.gny = (int32_t)yg.size();
             dp.gnx = (int32_t)xg.size();
-            dp.total_elems = (int64_t)h64.size();
+            dp.total_elems = (int64_t)n64;
             ps->h_nodes = nodes;
-            ps->h_data64 = h64;
+            ps->h_data64 = std::move(h64);
             ps->h_ygrid = yg;
             ps->h_xgrid = xg;
             ps->h_index_grid = ig;
-            ps->smem_bytes64 = (int64_t)h64.size() * 8;
-            ps->smem_bytes32 = (int64_t)h64.size() * 4;
+            ps->smem_bytes64 = (int64_t)n64 * 8;
+            ps->smem_bytes32 = (int64_t)n64 * 4;
         } catch (...) {
             cudaFree(ps->d_blob);
             delete ps;

@@ -62,6 +62,18 @@ struct DevNode {
 
 constexpr int kMaxNodes = 64;
 
+// Row-phase copies: pixel rows GH of each, its elements (a multiple of four), and whether
+// the kernels stage it in shared memory -- the stamp kernel beside 8 KB of static tables,
+// fit_star's up to 100 KB (the rest holds the teams' cutouts).  Others are not made.
+constexpr int kRowPhase[3] = {2, 4, 1};
+inline size_t row_phase_len(const DevNode& nd, int c) {
+    return ((size_t)kRowPhase[c] * nd.isy * nd.RPY[c] * nd.RPX + 3) / 4 * 4;
+}
+inline bool row_phase_staged(const DevNode& nd, int c, int smem_optin) {
+    const size_t bytes = row_phase_len(nd, c) * (c == 1 ? sizeof(float) : sizeof(double));
+    return c == 2 ? bytes <= 100 * 1024 : bytes + 8192 <= (size_t)smem_optin;
+}
+
 struct DevPsf {
     int32_t kind;       // CPB_PSF_*
     int32_t n_nodes;

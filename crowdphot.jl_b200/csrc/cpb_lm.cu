@@ -1761,19 +1761,17 @@ LMConst lm_const(const cpb_psf* psf, const cpb_lm_params* P, bool have_iv) {
 }
 
 // The node as the fast forms read it: the row-phase copy for staging in shared memory
-// up to 100 KB (the rest holds the teams' cutouts), else the polyphase copy in global
-// memory.
+// (row_phase_staged), else the polyphase copy in global memory.
 PPNode pp_node(const cpb_psf* psf, bool staged_wanted, size_t& smem_bytes) {
     PPNode N{};
     smem_bytes = 0;
     if (psf->dev.kind == CPB_PSF_CIRCULAR_GAUSSIAN) return N;
     N.nd = psf->h_nodes[0];
     N.plane = N.nd.LPY * N.nd.LPX;
-    const int nel = (N.nd.isy * N.nd.RPY[2] * N.nd.RPX + 3) / 4 * 4;
-    if (staged_wanted && sizeof(double) * (size_t)nel <= 100 * 1024) {
-        N.nel = nel;
+    if (staged_wanted && row_phase_staged(N.nd, 2, 0)) {
+        N.nel = (int)row_phase_len(N.nd, 2);
         N.pp = psf->dev.rpp64 + N.nd.rpoff[2];
-        smem_bytes = sizeof(double) * (size_t)nel;
+        smem_bytes = sizeof(double) * (size_t)N.nel;
     } else {
         N.pp = psf->dev.lpp64 + N.nd.lpoff;
     }

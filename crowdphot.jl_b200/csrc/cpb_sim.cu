@@ -2371,7 +2371,7 @@ template <bool GRAD, typename T, bool GRAM, typename... A>
 void launch_eval_node(const DevPsf& dp, const DevNode& nd, int n_sm, cudaStream_t st, const int32_t* list, int64_t nlist,
                       const FitConst& fc, A... args) {
     constexpr int GH = Gran<T>::H, CP = GH == 2 ? 0 : 1;
-    const size_t smem = sizeof(T) * (size_t)((GH * nd.isy * nd.RPY[CP] * nd.RPX + 3) / 4 * 4);
+    const size_t smem = sizeof(T) * row_phase_len(nd, CP);
     auto go = [&](auto kern) {
         allow_smem(kern, smem);
         const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(nlist, n_sm));
@@ -2695,8 +2695,7 @@ class SimFit {
     // `item` bytes) fits the block's shared memory beside its static tables
     bool node_eval(size_t item) const {
         return dp.kind != CPB_PSF_CIRCULAR_GAUSSIAN && dp.n_nodes == 1 &&
-               (int64_t)item * (item == 8 ? 2 : 4) * node0.isy * node0.RPY[item == 8 ? 0 : 1] * node0.RPX + 8192 <=
-                   smem_optin;
+               row_phase_staged(node0, item == 8 ? 0 : 1, smem_optin);
     }
     void warp_shape(int Sx, size_t tab_size, unsigned& threads, size_t& smem) const;
     void arena_precheck();

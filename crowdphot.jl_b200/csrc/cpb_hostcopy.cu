@@ -3,14 +3,19 @@
 // A pageable cudaMemcpyAsync is staged by one driver thread: it moved the three
 // 16.8 MB images of a 2048^2 field and the 33.5 MB residual (into memory the caller
 // has not touched yet, so every page faults) at a few GB/s while the GPU waited.
-// Here a few worker threads each own a stream and two pinned chunks and copy every
-// kThreads-th chunk of the job: the host copies, the page faults and the DMA
+// Here a few worker threads each own a stream and two pinned chunks and take the chunks of
+// the job in turn: the host copies, the page faults and the DMA
 // transfers run side by side (2048^2 field with residual, whole call: 44.4 -> 35.5 ms),
 // and the residual leaves while the diagnostics run.  Memory the caller has pinned goes to the driver as
 // before.  One copier per context, made at its first large pageable copy and given
-// back with the context; kThreads * 2 chunks of pinned memory.
+// back with the context; kThreads * 2 chunks of pinned memory.  A process' copiers together
+// have a worker a processor it may run on, each copier at least one.
+#include <sched.h>
+#include <stdlib.h>
 #include <string.h>
+#include <sys/mman.h>
 
+#include <atomic>
 #include <condition_variable>
 #include <mutex>
 #include <thread>
@@ -22,11 +27,25 @@ namespace cpb {
 
 namespace {
 
-constexpr int kThreads = 4;
-constexpr size_t kChunk = size_t(1) << 18;  // 2 MB of pinned memory in all: quick to make
+constexpr int kThreads = 4;                 // at most
+constexpr size_t kChunk = size_t(1) << 18;
+// The pinned memory: one huge page, registered.  Making a copier falls into a context's first
+// large request, and cudaMallocHost of 2 MB took 1.2-3.9 ms of it, registering a huge page
+// 0.35 (2.2 where the host has none to give); the first pass of a new server of four slots
+// 30.6 -> 26.5 ms (22.0 from then on).
+constexpr size_t kPage = size_t(2) << 20;
+static_assert(kThreads * 2 * kChunk <= kPage, "the workers' chunks");
 // Below this the workers' wake-up and scheduling costs more than they save: a 613 x 421
 // field (3 MB in, 2 MB out) took 5.7 ms a call with them and 5.1 ms without.
 constexpr size_t kMinBytes = size_t(8) << 20;
+
+std::atomic<int> n_workers{0};  // of every copier
+
+int processors() {
+    cpu_set_t set;
+    CPU_ZERO(&set);
+    return sched_getaffinity(0, sizeof(set), &set) == 0 ? CPU_COUNT(&set) : 1;
+}
 
 bool pinned_host(const void* p) {
     cudaPointerAttributes a{};
@@ -48,8 +67,23 @@ class HostCopier {
     };
 
     explicit HostCopier(int device) : device_(device) {
-        if (cudaMallocHost((void**)&pin_, kThreads * 2 * kChunk) != cudaSuccess) ok_ = false;
-        for (int k = 0; k < kThreads; ++k) {
+        int others = n_workers.load();
+        do {
+            n_ = std::min(std::max(processors() - others, 1), kThreads);
+        } while (!n_workers.compare_exchange_weak(others, others + n_));
+        pin_ = (char*)aligned_alloc(kPage, kPage);
+        if (pin_) {
+            madvise(pin_, kPage, MADV_HUGEPAGE);
+            memset(pin_, 0, (size_t)n_ * 2 * kChunk);
+            registered_ = cudaHostRegister(pin_, (size_t)n_ * 2 * kChunk, cudaHostRegisterDefault) == cudaSuccess;
+        }
+        if (!registered_) {  // no room to lock it
+            cudaGetLastError();
+            free(pin_);
+            pin_ = nullptr;
+            if (cudaMallocHost((void**)&pin_, (size_t)n_ * 2 * kChunk) != cudaSuccess) ok_ = false;
+        }
+        for (int k = 0; k < n_; ++k) {
             Worker& w = w_[k];
             w.pin = pin_ + k * 2 * kChunk;
             if (cudaStreamCreateWithFlags(&w.stream, cudaStreamNonBlocking) != cudaSuccess) ok_ = false;
@@ -62,7 +96,7 @@ class HostCopier {
             return;
         }
         try {
-            for (int k = 0; k < kThreads; ++k) w_[k].th = std::thread([this, k] { loop(k); });
+            for (int k = 0; k < n_; ++k) w_[k].th = std::thread([this, k] { loop(k); });
         } catch (...) {  // no threads to be had: the caller copies through the driver
             ok_ = false;
         }
@@ -80,8 +114,14 @@ class HostCopier {
                 if (e) cudaEventDestroy(e);
             if (w.stream) cudaStreamDestroy(w.stream);
         }
-        if (pin_) cudaFreeHost(pin_);
+        if (registered_) {
+            cudaHostUnregister(pin_);
+            free(pin_);
+        } else if (pin_) {
+            cudaFreeHost(pin_);
+        }
         if (start_) cudaEventDestroy(start_);
+        n_workers -= n_;
     }
 
     bool ok() const { return ok_; }
@@ -94,7 +134,7 @@ class HostCopier {
             parts_ = std::move(parts);
             to_device_ = to_device;
             err_ = cudaSuccess;
-            running_ = kThreads;
+            running_ = n_;
             ++job_;
         }
         cv_.notify_all();
@@ -107,8 +147,8 @@ class HostCopier {
         done_.wait(lk, [this] { return running_ == 0; });
         cudaError_t e = err_;
         if (to_device_)
-            for (auto& w : w_)
-                for (auto& ev : w.ev)
+            for (int k = 0; k < n_; ++k)
+                for (auto& ev : w_[k].ev)
                     if (e == cudaSuccess) e = cudaStreamWaitEvent(st, ev, 0);
         return e;
     }
@@ -162,7 +202,7 @@ class HostCopier {
         };
         for (const Part& p : parts_)
             for (size_t at = 0; at < p.bytes; at += kChunk, ++c) {
-                if (c % kThreads != (size_t)k) continue;
+                if (c % (size_t)n_ != (size_t)k) continue;
                 const size_t n = p.bytes - at < kChunk ? p.bytes - at : kChunk;
                 const int half = (int)(w.n++ & 1);
                 char* pin = w.pin + half * kChunk;
@@ -185,7 +225,8 @@ class HostCopier {
     }
 
     int device_;
-    bool ok_ = true;
+    bool ok_ = true, registered_ = false;
+    int n_ = 0;  // workers
     char* pin_ = nullptr;
     Worker w_[kThreads];
     cudaEvent_t start_ = nullptr;

@@ -53,13 +53,16 @@ class Context:
             raise CudaError(f"cpb_ctx_create(device={device}) failed with status {rc}")
         self.handle = h
         self.device = device
-        self._psfs: dict[int, tuple] = {}
+        self._psfs: dict[int, list] = {}  # id -> [handle, weak reference, handed out by psf_handle]
+        self._kept: list = []             # handed-out handles of PSFs that are gone
+        self._psf_lock = threading.Lock()
 
     def close(self):
         if self.handle:
-            for _, (hp, _ref) in list(self._psfs.items()):
+            for hp in self._kept + [e[0] for e in self._psfs.values()]:
                 self.lib.cpb_psf_free(self.handle, hp)
             self._psfs.clear()
+            self._kept.clear()
             self.lib.cpb_ctx_destroy(self.handle)
             self.handle = None
 
@@ -109,17 +112,37 @@ class Context:
         return stats, int(launches.value)
 
     def psf_handle(self, psf, fwhm_override=None):
-        key = id(psf)
-        hit = self._psfs.get(key)
-        if hit is not None and hit[1]() is psf:
-            return hit[0]
-        desc, keep = psf_descriptor(psf)
-        hp = C.c_void_p()
-        rc = self.lib.cpb_psf_upload(self.handle, C.byref(desc), C.byref(hp))
-        self.raise_for(rc, "cpb_psf_upload")
-        del keep
-        self._psfs[key] = (hp, weakref.ref(psf))
-        return hp
+        """Device tables of `psf`, uploaded at its first use; the handle is good until the context is closed."""
+        entry = self._psf_entry(psf)
+        entry[2] = True
+        return entry[0]
+
+    def _call_handle(self, psf):
+        """psf_handle for as long as the caller keeps `psf`: the tables of a PSF that is gone (a loop
+        over models made by replace_params) are given back at a later upload."""
+        return self._psf_entry(psf)[0]
+
+    def _psf_entry(self, psf):
+        entry = self._psfs.get(id(psf))
+        if entry is not None and entry[1]() is psf:
+            return entry
+        with self._psf_lock:
+            entry = self._psfs.get(id(psf))   # another thread's upload
+            if entry is not None and entry[1]() is psf:
+                return entry
+            for key in [k for k, e in self._psfs.items() if e[1]() is None]:
+                gone = self._psfs.pop(key)
+                if gone[2]:
+                    self._kept.append(gone[0])
+                else:
+                    self.lib.cpb_psf_free(self.handle, gone[0])
+            desc, keep = psf_descriptor(psf)
+            hp = C.c_void_p()
+            rc = self.lib.cpb_psf_upload(self.handle, C.byref(desc), C.byref(hp))
+            self.raise_for(rc, "cpb_psf_upload")
+            del keep
+            entry = self._psfs[id(psf)] = [hp, weakref.ref(psf), False]
+            return entry
 
 
 _default_ctx: Context | None = None
@@ -436,7 +459,7 @@ def fit_all_stars_simultaneous(image, psf, sources, fit_rad, *, fixed=None, inv_
     R = int(np.ceil(fit_rad)) if fit_rad > 0 else 0
     S2 = (2 * R + 1) ** 2
     outs = SimOutputs(y0.size, ny, nx, S2, residual=residual, debug=debug)
-    hp = ctx.psf_handle(psf)
+    hp = ctx._call_handle(psf)
     vp = lambda a: None if a is None else a.ctypes.data_as(C.c_void_p)
     rc = ctx.lib.cpb_fit_simultaneous(ctx.handle, hp, C.byref(P), vp(imgf), et, ny, nx, vp(ivf), vp(bkf),
                                       y0.size, y0.ctypes.data_as(_abi._dp), x0.ctypes.data_as(_abi._dp),
@@ -503,7 +526,7 @@ def fit_groups_packed(psf, pixels, offsets, ny, nx, star_offsets, y0, x0, flux0,
     P = sim_params(psf, fit_rad, fixed, inv_var_given=iv is not None, **kw)
     o = group_outputs(int(ys.size), G, int(pix.size), residual=residual)
     r = group_result_struct(o, lambda a: a.ctypes.data)
-    hp = ctx.psf_handle(psf)
+    hp = ctx._call_handle(psf)
     vp = lambda a: None if a is None else a.ctypes.data_as(C.c_void_p)
     rc = ctx.lib.cpb_fit_simultaneous_batch(ctx.handle, hp, C.byref(P), G, off.ctypes.data_as(_abi._i64p),
                                             nyv.ctypes.data_as(_abi._i32p), nxv.ctypes.data_as(_abi._i32p), vp(pix),
@@ -597,8 +620,8 @@ class BatchGraph:
     def __init__(self, psf, *, lm=None, lm_fixed=None, groups=None, fit_rad=None, group_kw=None,
                  autotune=1, cache_path=None, ctx: Context | None = None):
         self.ctx = ctx or get_context()
-        self._keep = []
-        hp = self.ctx.psf_handle(psf)
+        self._keep = [psf]   # its tables are good while it lives
+        hp = self.ctx._call_handle(psf)
         ptr = lambda t: None if t is None else C.c_void_p(t.data_ptr())
         lm_args = [None, 0] + [None] * 6 + [0, None, None, 0, None]
         if lm is not None:
@@ -835,7 +858,7 @@ def fit_star_batch(model, cutouts, *, inv_vars=None, origins, inits=None, fixed=
     nf = bin(P.free_mask).count("1")
     out = _lm_outputs(n, np_, nf)
     r = _lm_result_struct(out, lambda a: a.ctypes.data)
-    hp = ctx.psf_handle(model)
+    hp = ctx._call_handle(model)
     et = _abi.CPB_F32 if dt == np.float32 else _abi.CPB_F64
     rc = ctx.lib.cpb_fit_lm_batch(ctx.handle, hp, C.byref(P), n, offs.ctypes.data_as(_abi._i64p),
                                   nyv.ctypes.data_as(_abi._i32p), nxv.ctypes.data_as(_abi._i32p),
@@ -896,7 +919,7 @@ def fit_star_packed(model, pixels, offsets, ny, nx, y_origin, x_origin, init, *,
     out = _lm_outputs(n, np_, nf)
     r = _lm_result_struct(out, lambda a: a.ctypes.data)
     et = _abi.CPB_F32 if dt == np.float32 else _abi.CPB_F64
-    rc = ctx.lib.cpb_fit_lm_batch(ctx.handle, ctx.psf_handle(model), C.byref(P), n, offs.ctypes.data_as(_abi._i64p),
+    rc = ctx.lib.cpb_fit_lm_batch(ctx.handle, ctx._call_handle(model), C.byref(P), n, offs.ctypes.data_as(_abi._i64p),
                                   nyv.ctypes.data_as(_abi._i32p), nxv.ctypes.data_as(_abi._i32p),
                                   y1.ctypes.data_as(_abi._i32p), x1.ctypes.data_as(_abi._i32p),
                                   pix.ctypes.data_as(C.c_void_p), et,
@@ -989,7 +1012,7 @@ def fit_all_stars(image, psf, sources, fit_rad, *, n_passes=3, fixed=None, inv_v
     ny, nx = imgf.shape
     outs = MultipassOutputs(init.shape[0], init.shape[1], ny, nx, residual=residual)
     vp = lambda a: None if a is None else a.ctypes.data_as(C.c_void_p)
-    rc = ctx.lib.cpb_fit_all_stars(ctx.handle, ctx.psf_handle(psf), C.byref(P), float(fit_rad), int(n_passes),
+    rc = ctx.lib.cpb_fit_all_stars(ctx.handle, ctx._call_handle(psf), C.byref(P), float(fit_rad), int(n_passes),
                                    spread_fwhm_arg(spread_model_fwhm), vp(imgf), et, ny, nx, vp(ivf), init.shape[0],
                                    init.ctypes.data_as(_abi._dp), C.byref(outs.c))
     ctx.raise_for(rc, "cpb_fit_all_stars")

@@ -381,8 +381,11 @@ int cpb_psf_upload(cpb_ctx* ctx, const cpb_psf_desc* d, cpb_psf** out) {
                     else regroup((double*)(host + o_r64) + nd.rpoff[c], rows, cols, nd);
                 }
             }
-            check(cudaMalloc(&ps->d_blob, bytes), "cudaMalloc");
-            check(cudaMemcpy(ps->d_blob, host, bytes, cudaMemcpyHostToDevice), "h2d");
+            // from the device's pool, as the scratch: a loop over new models takes back what the
+            // last one gave
+            check(cudaMallocAsync(&ps->d_blob, bytes, ctx->stream), "cudaMallocAsync");
+            check(cudaMemcpyAsync(ps->d_blob, host, bytes, cudaMemcpyHostToDevice, ctx->stream), "h2d");
+            check(cudaStreamSynchronize(ctx->stream), "sync");
             const char* base = (const char*)ps->d_blob;
             dp.data64 = (const double*)(base + o_d64);
             dp.data32 = (const float*)(base + o_d32);
@@ -407,7 +410,7 @@ int cpb_psf_upload(cpb_ctx* ctx, const cpb_psf_desc* d, cpb_psf** out) {
             ps->smem_bytes64 = (int64_t)n64 * 8;
             ps->smem_bytes32 = (int64_t)n64 * 4;
         } catch (...) {
-            cudaFree(ps->d_blob);
+            if (ps->d_blob) cudaFreeAsync(ps->d_blob, ctx->stream);
             delete ps;
             throw;
         }
@@ -420,7 +423,7 @@ int cpb_psf_free(cpb_ctx* ctx, cpb_psf* ps) {
     if (!ps) return CPB_OK;
     return guarded(ctx, [&]() -> int {
         cudaStreamSynchronize(ctx->stream);
-        cudaFree(ps->d_blob);
+        if (ps->d_blob) cudaFreeAsync(ps->d_blob, ctx->stream);
         delete ps;
         return CPB_OK;
     });

@@ -35,8 +35,17 @@ constexpr size_t kChunk = size_t(1) << 18;
 // 30.6 -> 26.5 ms (22.0 from then on).
 constexpr size_t kPage = size_t(2) << 20;
 static_assert(kThreads * 2 * kChunk <= kPage, "the workers' chunks");
-// Below this the workers' wake-up and scheduling costs more than they save: a 613 x 421
-// field (3 MB in, 2 MB out) took 5.7 ms a call with them and 5.1 ms without.
+// Below this the workers' wake-up and scheduling costs more than they save.  Whole calls on
+// square fields, by workers and by the driver.  Up, three Float32 images read from memory (a
+// new field each call) and from the processor's cache (the same one again):
+//    3.2 MB 2.0 and 1.9 ms, 2.0 and 1.8;   8.4 MB 2.4 and 2.45, 2.4 and 2.1;
+//   17.3 MB 3.2 and 3.5,    3.2 and 2.9;  27.0 MB 4.0 and 4.9,  4.1 and 3.9;
+//   50.3 MB 5.0 and 6.7,    5.1 and 5.1.
+// Down, the residual to memory not touched before (results are kept) and used again:
+//    3.9 MB 2.3 and 3.7,    2.7 and 2.4;   8.4 MB 3.2 and 4.6,  3.6 and 3.3;
+//   18.0 MB 5.7 and 8.3,    5.7 and 5.8;  23.1 MB 6.3 and 9.7,  6.9 and 7.1.
+// Six served fields, two of them above the line: 21.9 ms, and 20.7 with every one below it,
+// from the cache; 22.6 and 22.9 from memory.
 constexpr size_t kMinBytes = size_t(8) << 20;
 
 std::atomic<int> n_workers{0};  // of every copier

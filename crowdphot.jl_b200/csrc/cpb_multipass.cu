@@ -67,16 +67,12 @@ __global__ void k_mp_addcut(int nL, const int4* __restrict__ boxes, const double
 // right after its subtraction (snap_off per position), used in place of the
 // residual image when the diagnostics run after the whole pass.
 template <typename TI, bool WARP>
-__global__ void __launch_bounds__(WARP ? 32 * kDiagWarps : kDiagThreads, WARP ? 4 : 2) 
-    k_mp_diag(int nL, const int4* __restrict__ boxes,    const double* __restrict__ params,
-                                                         const uint8_t* __restrict__ flags,
-                                                         const TI* __restrict__ img,
-                                                         const double* __restrict__ residual,
-                                                         const double* __restrict__ snap,
-                                                         const int64_t* __restrict__ snap_off,
-                                                         const TI* __restrict__ iv, DevPsf P, MPConst M, int n_free,
-                                                         int ny, SpreadDev D, int smode, int boxmax,
-                                                         const int32_t* __restrict__ idx, double* __restrict__ out) {
+__global__ void __launch_bounds__(WARP ? 32 * kDiagWarps : kDiagThreads, WARP ? 4 : 2)
+    k_mp_diag(int nL, const int4* __restrict__ boxes, const double* __restrict__ params,
+              const uint8_t* __restrict__ flags, const TI* __restrict__ img, const double* __restrict__ residual,
+              const double* __restrict__ snap, const int64_t* __restrict__ snap_off, const TI* __restrict__ iv, DevPsf P,
+              MPConst M, int n_free, int ny, SpreadDev D, int smode, int boxmax, const int32_t* __restrict__ idx,
+              double* __restrict__ out) {
     extern __shared__ double diag_smem[];
     __shared__ double red[12 * (kDiagThreads / 32)];
     const double NaN = __longlong_as_double(0x7ff8000000000000LL);

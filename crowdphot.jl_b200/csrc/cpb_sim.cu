@@ -2170,13 +2170,10 @@ __global__ void __launch_bounds__(256) k_spread_disk(DevPsf P, double param, int
 // (spread_disk_block; null or off: spread_model NaN), smode its layout.
 template <typename TI, bool WARP>
 __global__ void __launch_bounds__(WARP ? 32 * kDiagWarps : kDiagThreads, WARP ? 4 : 2)
-    k_diag(int64_t n_act, FitConst fc, DevPsf P, double fit_rad,                       const StarCoef* __restrict__ coef,
-                                                      const double* __restrict__ resid, const TI* __restrict__ img,
-                                                      const TI* __restrict__ bkgimg, const TI* __restrict__ iv,
-                                                      const double* __restrict__ stab, int kh, int smode,
-                                                      int boxmax,
-                                                      double* out /* n_act x 7: chisq qfit qfit_exp qfit_z crowding
-                                                                     spread spread_err */) {
+    k_diag(int64_t n_act, FitConst fc, DevPsf P, double fit_rad, const StarCoef* __restrict__ coef,
+           const double* __restrict__ resid, const TI* __restrict__ img, const TI* __restrict__ bkgimg,
+           const TI* __restrict__ iv, const double* __restrict__ stab, int kh, int smode, int boxmax,
+           double* out /* n_act x 7: chisq qfit qfit_exp qfit_z crowding spread spread_err */) {
     extern __shared__ double diag_smem[];
     __shared__ double red[14 * (kDiagThreads / 32)];
     __shared__ StarCoef cs[WARP ? kDiagWarps : 1];

@@ -2116,12 +2116,12 @@ int fit_groups_dev(cpb_ctx* ctx, const cpb_psf* psf, const cpb_sim_params* P, in
 // ---------------------------------------------------------------------------
 struct GroupBatch {
     GroupSetup su;
-    int32_t* d_list = nullptr;  // owned: every bucket's groups back to back, then as much for deferred ones
-    int* d_queue = nullptr;     // owned: kQueueInts counters per bucket
+    void* block = nullptr;      // owned: spread_model rule, the lists, the stars' residual / weight
+                                // planes, the blocks' union arrays (GroupOut::px) and the counters
+    int32_t* d_list = nullptr;  // every bucket's groups back to back, then as much for deferred ones
+    int* d_queue = nullptr;     // kQueueInts counters per bucket
     std::vector<int64_t> at;    // first list entry of each bucket
     std::vector<int> threads;   // chosen block size per bucket
-    double* px = nullptr;       // owned: the blocks' union arrays
-    double* sp_buf = nullptr;   // owned: spread_model rule and the stars' residual / weight planes
 };
 
 GroupBatch* group_batch_create(cpb_ctx* ctx, const cpb_psf* psf, const cpb_sim_params* P, int64_t G,
@@ -2151,38 +2151,41 @@ GroupBatch* group_batch_create(cpb_ctx* ctx, const cpb_psf* psf, const cpb_sim_p
             b->threads.push_back(B.threads);
             lists.insert(lists.end(), B.groups.begin(), B.groups.end());
         }
-        if (cudaMalloc(&b->d_list, sizeof(int32_t) * std::max<size_t>(2 * lists.size(), 1)) != cudaSuccess ||
-            cudaMalloc(&b->d_queue, sizeof(int) * kQueueInts * std::max<size_t>(plan.buckets.size(), 1)) != cudaSuccess) {
-            cudaGetLastError();
-            throw OomError{"device memory exhausted allocating the group work queues"};
-        }
-        if (!lists.empty())
-            check(cudaMemcpy(b->d_list, lists.data(), sizeof(int32_t) * lists.size(), cudaMemcpyHostToDevice),
-                  "h2d");
+        // one allocation and one copy: three or four of each took a tenth of binding a small batch
         GroupSetup& su = b->su;
-        if (cudaMalloc(&b->px, sizeof(double) * std::max<size_t>(plan.buckets.empty() ? 0 : group_px_doubles(ctx, su), 1)) !=
-            cudaSuccess) {
+        const bool sp = su.C.sp_on && !plan.buckets.empty();
+        size_t bytes = 0;
+        auto place = [&](size_t n) {
+            const size_t at = bytes;
+            bytes = (at + n + 255) & ~size_t(255);
+            return at;
+        };
+        const size_t o_rule = place(sp ? sizeof(double) * kSpreadRuleLen : 0);
+        const size_t o_list = place(sizeof(int32_t) * 2 * lists.size());
+        const size_t o_rw = place(sp ? sizeof(double) * 2 * su.C.sp_box * su.n_stars : 0);
+        const size_t o_px = place(plan.buckets.empty() ? 0 : sizeof(double) * group_px_doubles(ctx, su));
+        const size_t o_queue = place(sizeof(int) * kQueueInts * plan.buckets.size());
+        if (cudaMalloc(&b->block, std::max<size_t>(bytes, 256)) != cudaSuccess) {
             cudaGetLastError();
-            throw OomError{"device memory exhausted allocating the groups' pixel arrays"};
+            throw OomError{"device memory exhausted allocating the groups' work queues, pixel arrays and "
+                           "spread_model planes"};
         }
-        su.go.px = b->px;
-        if (su.C.sp_on && !plan.buckets.empty()) {
-            const size_t n_rule = kSpreadRuleLen, n_rw = (size_t)2 * su.C.sp_box * su.n_stars;
-            if (cudaMalloc(&b->sp_buf, sizeof(double) * (n_rule + n_rw)) != cudaSuccess) {
-                cudaGetLastError();
-                throw OomError{"device memory exhausted allocating the spread_model planes"};
-            }
-            double h_rule[kSpreadRuleLen];
-            spread_rule(h_rule);
-            check(cudaMemcpy(b->sp_buf, h_rule, sizeof(h_rule), cudaMemcpyHostToDevice), "h2d");
-            su.go.sp_rule = b->sp_buf;
-            su.go.sp_rw = b->sp_buf + n_rule;
+        char* base = (char*)b->block;
+        b->d_list = (int32_t*)(base + o_list);
+        b->d_queue = (int*)(base + o_queue);
+        su.go.px = (double*)(base + o_px);
+        std::vector<char> head(o_list + sizeof(int32_t) * lists.size());
+        if (sp) {
+            spread_rule((double*)head.data());
+            su.go.sp_rule = (const double*)(base + o_rule);
+            su.go.sp_rw = (double*)(base + o_rw);
+        }
+        if (!lists.empty()) {
+            std::copy(lists.begin(), lists.end(), (int32_t*)(head.data() + o_list));
+            check(cudaMemcpy(base, head.data(), head.size(), cudaMemcpyHostToDevice), "h2d");
         }
     } catch (...) {
-        cudaFree(b->sp_buf);
-        cudaFree(b->px);
-        cudaFree(b->d_list);
-        cudaFree(b->d_queue);
+        cudaFree(b->block);
         delete b;
         throw;
     }
@@ -2222,10 +2225,7 @@ std::string group_batch_signature(const GroupBatch* b, int bucket) {
 
 void group_batch_destroy(GroupBatch* b) {
     if (!b) return;
-    cudaFree(b->sp_buf);
-    cudaFree(b->px);
-    cudaFree(b->d_list);
-    cudaFree(b->d_queue);
+    cudaFree(b->block);
     delete b;
 }
 

@@ -254,7 +254,7 @@ int cpb_batch_graph_create(cpb_ctx* ctx, const cpb_psf* psf, const cpb_lm_params
                 if (e) cudaEventDestroy(e);
             if (g->side) cudaStreamDestroy(g->side);
             lm_batch_destroy(g->lm);
-            group_batch_destroy(g->grp);
+            group_batch_destroy(ctx, g->grp);
             delete g;
             throw;
         }
@@ -292,7 +292,7 @@ int cpb_batch_graph_destroy(cpb_ctx* ctx, cpb_batch_graph* g) {
             if (e) cudaEventDestroy(e);
         if (g->side) cudaStreamDestroy(g->side);
         lm_batch_destroy(g->lm);
-        group_batch_destroy(g->grp);
+        group_batch_destroy(ctx, g->grp);
         delete g;
         return CPB_OK;
     });

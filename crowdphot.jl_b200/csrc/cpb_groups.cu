@@ -2116,8 +2116,9 @@ int fit_groups_dev(cpb_ctx* ctx, const cpb_psf* psf, const cpb_sim_params* P, in
 // ---------------------------------------------------------------------------
 struct GroupBatch {
     GroupSetup su;
-    void* block = nullptr;      // owned: spread_model rule, the lists, the stars' residual / weight
-                                // planes, the blocks' union arrays (GroupOut::px) and the counters
+    void* block = nullptr;      // owned, from the device's pool: spread_model rule, the lists, the stars'
+                                // residual / weight planes, the blocks' union arrays (GroupOut::px) and
+                                // the counters
     int32_t* d_list = nullptr;  // every bucket's groups back to back, then as much for deferred ones
     int* d_queue = nullptr;     // kQueueInts counters per bucket
     std::vector<int64_t> at;    // first list entry of each bucket
@@ -2151,7 +2152,10 @@ GroupBatch* group_batch_create(cpb_ctx* ctx, const cpb_psf* psf, const cpb_sim_p
             b->threads.push_back(B.threads);
             lists.insert(lists.end(), B.groups.begin(), B.groups.end());
         }
-        // one allocation and one copy: three or four of each took a tenth of binding a small batch
+        // One block from the pool, whose first chunk a scratch buffer keeps, and one copy: three or
+        // four cudaMalloc, and the memory the driver maps for each above 1 MB, took a tenth of
+        // binding a small batch (milliseconds on some hosts).
+        scratch(ctx, "grp_keep", 256);
         GroupSetup& su = b->su;
         const bool sp = su.C.sp_on && !plan.buckets.empty();
         size_t bytes = 0;
@@ -2163,9 +2167,9 @@ GroupBatch* group_batch_create(cpb_ctx* ctx, const cpb_psf* psf, const cpb_sim_p
         const size_t o_rule = place(sp ? sizeof(double) * kSpreadRuleLen : 0);
         const size_t o_list = place(sizeof(int32_t) * 2 * lists.size());
         const size_t o_rw = place(sp ? sizeof(double) * 2 * su.C.sp_box * su.n_stars : 0);
-        const size_t o_px = place(plan.buckets.empty() ? 0 : sizeof(double) * group_px_doubles(ctx, su));
         const size_t o_queue = place(sizeof(int) * kQueueInts * plan.buckets.size());
-        if (cudaMalloc(&b->block, std::max<size_t>(bytes, 256)) != cudaSuccess) {
+        const size_t o_px = place(plan.buckets.empty() ? 0 : sizeof(double) * group_px_doubles(ctx, su));
+        if (cudaMallocAsync(&b->block, std::max<size_t>(bytes, 256), ctx->stream) != cudaSuccess) {
             cudaGetLastError();
             throw OomError{"device memory exhausted allocating the groups' work queues, pixel arrays and "
                            "spread_model planes"};
@@ -2182,11 +2186,11 @@ GroupBatch* group_batch_create(cpb_ctx* ctx, const cpb_psf* psf, const cpb_sim_p
         }
         if (!lists.empty()) {
             std::copy(lists.begin(), lists.end(), (int32_t*)(head.data() + o_list));
-            check(cudaMemcpy(base, head.data(), head.size(), cudaMemcpyHostToDevice), "h2d");
+            check(cudaMemcpyAsync(base, head.data(), head.size(), cudaMemcpyHostToDevice, ctx->stream), "h2d");
+            check(cudaStreamSynchronize(ctx->stream), "sync");
         }
     } catch (...) {
-        cudaFree(b->block);
-        delete b;
+        group_batch_destroy(ctx, b);
         throw;
     }
     return b;
@@ -2223,9 +2227,9 @@ std::string group_batch_signature(const GroupBatch* b, int bucket) {
     return buf;
 }
 
-void group_batch_destroy(GroupBatch* b) {
+void group_batch_destroy(cpb_ctx* ctx, GroupBatch* b) {
     if (!b) return;
-    cudaFree(b->block);
+    if (b->block) cudaFreeAsync(b->block, ctx->stream);
     delete b;
 }
 

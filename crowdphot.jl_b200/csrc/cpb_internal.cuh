@@ -1150,7 +1150,7 @@ int group_batch_threads(const GroupBatch* b, int bucket);
 int group_batch_occupancy(GroupBatch* b, int bucket, int threads);
 int64_t group_batch_size(const GroupBatch* b);
 std::string group_batch_signature(const GroupBatch* b, int bucket);
-void group_batch_destroy(GroupBatch* b);
+void group_batch_destroy(cpb_ctx* ctx, GroupBatch* b);  // no launch of it in flight
 
 // fit_all_stars (cpb_multipass.cu): device image / weights, host catalogue and outputs.
 int fit_all_stars_dev(cpb_ctx* ctx, const cpb_psf* psf, const cpb_lm_params* P, double fit_rad, int n_passes,
